@@ -39,7 +39,8 @@ def build(ref: bool = True) -> None:
     # the reference tree sits beside the repository checkout unless REF says
     # otherwise (the same rule as the Makefile's)
     ref_dir = os.environ.get("REF", os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference"))
-    if ref and os.path.isdir(ref_dir):
+    # (an empty folder in its place is no reference tree)
+    if ref and os.path.isfile(os.path.join(ref_dir, "OpenMPManager.cpp")):
         targets.append("ref")
     subprocess.run(["make", "-s", "-C", HERE, *targets], check=True)
 

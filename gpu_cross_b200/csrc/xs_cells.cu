@@ -1,0 +1,162 @@
+// Cell moments: the far wings of 2^cshift consecutive lines as one short
+// series (CellHead in xs_internal.cuh has the formulas).
+#include <cuda_runtime.h>
+
+#include <cfloat>
+
+#include "xs_internal.cuh"
+
+namespace xs {
+namespace {
+
+constexpr int kCellWarps = 4;
+
+// Sums over the warp: on return lane L holds in v[0] the sum of v[L] over all
+// lanes.  31 exchanges of doubles instead of 5 for each of the 32 values.
+__device__ __forceinline__ void transpose_sum(double (&v)[32], int lane) {
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+        const bool up = (lane & w) != 0;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+            const double give = up ? v[i] : v[i + w];
+            const double got = __shfl_xor_sync(0xffffffffu, give, w);
+            v[i] = (up ? v[i + w] : v[i]) + got;
+        }
+    }
+}
+
+// One warp per (cell, group of conditions), lanes over the cell's lines.
+// Step one's records give y and pref of each (line, condition):
+//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64), cyp (mixed).
+template <bool MIXED, bool GROUPED, int C>
+__global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
+    constexpr int PM = cell_moments(MIXED);
+    const int lane = threadIdx.x & 31;
+    const int cell = int(blockIdx.x) * kCellWarps + int(threadIdx.x >> 5);
+    if (cell >= a.ncell) return;
+    const int g = int(blockIdx.y);
+    const long i0 = long(cell) << a.cshift;
+    const long i1 = i0 + (1L << a.cshift) < a.n ? i0 + (1L << a.cshift) : a.n;
+    const double c0 = 0.5 * (a.nu[i0] + a.nu[i1 - 1]);
+
+    auto load = [&](long i, int k, double& y, double& pref) {
+        const size_t c = size_t(g) * C + k;
+        if constexpr (GROUPED && MIXED) {
+            const float2 v = a.cyp[c * size_t(a.n) + size_t(i)];
+            y = double(v.x);
+            pref = double(v.y);
+        } else if constexpr (GROUPED) {
+            const CondRec64& r = static_cast<const CondRec64*>(a.rec)[(size_t(g) * size_t(a.n) + size_t(i)) * C + k];
+            y = r.y;
+            pref = r.pref;
+        } else if constexpr (MIXED) {
+            const RecV32& r = static_cast<const RecV32*>(a.rec)[c * size_t(a.n) + size_t(i)];
+            y = double(r.y);
+            pref = double(r.pref);
+        } else {
+            const RecV64& r = static_cast<const RecV64*>(a.rec)[c * size_t(a.n) + size_t(i)];
+            y = r.y;
+            pref = r.pref;
+        }
+    };
+    const double s2 = 0.70710678118654752440;
+
+    // The scale q (every |zeta|), the reach of W4's regions II-IV, and
+    // whether every line is an ordinary one (else the cell is never far).
+    float q = 0.0f, reach = 0.0f;
+    bool good = true;
+    for (long i = i0 + lane; i < i1; i += 32) {
+        const double nu = a.nu[i];
+        const double d = fabs(nu - c0);
+        good = good && nu > 0.0;
+#pragma unroll 1
+        for (int k = 0; k < C; ++k) {
+            double y, pref;
+            load(i, k, y, pref);
+            const double w = nu * a.dpw[g * C + k];
+            const double re = fma(s2, w, d), gam = y * w;
+            const float z = __double2float_ru(sqrt(fma(re, re, gam * gam)));
+            const float h = __double2float_ru(d + (y < 15.0 ? (15.0 - y) * w : 0.0));
+            // (a NaN fails the comparisons)
+            good = good && w > 0.0 && z < 1.0e30f && h < 1.0e30f && fabs(pref) < (MIXED ? double(FLT_MAX) : 1.0e280);
+            q = fmaxf(q, z);
+            reach = fmaxf(reach, h);
+        }
+    }
+    // non-negative floats order as their bit patterns
+    q = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(q)));
+    reach = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(reach)));
+    good = __all_sync(0xffffffffu, good) && q > 0.0f;
+    const size_t at = size_t(g) * size_t(a.ncell) + size_t(cell);
+    if (lane == 0) {
+        CellHead h;
+        h.c0 = c0;
+        // two grid steps beyond the regions: their intervals are placed on the
+        // analytic grid, the tiles by the grid's own values
+        h.dmin = good ? fmaxf(kCellKappa * q * 1.000001f, reach * 1.000001f + __double2float_ru(2.0 * a.df))
+                      : __int_as_float(0x7f800000);
+        h.q = q;
+        a.head[at] = h;
+    }
+    if (!good) return;
+    const double rq = 1.0 / double(q);
+    double* M = a.mom + at * size_t(PM * C);
+#pragma unroll 1
+    for (int k = 0; k < C; ++k) {
+        double m[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) m[j] = 0.0;
+        const double dpw = a.dpw[g * C + k];
+#pragma unroll 1
+        for (long i = i0 + lane; i < i1; i += 32) {
+            double y, pref;
+            load(i, k, y, pref);
+            const double nu = a.nu[i];
+            const double w = nu * dpw;
+            const double A = pref * w * (0.5 * kW4C * rq);
+            const double d = (nu - c0) * rq, s = s2 * w * rq, gam = y * w * rq;
+            // I_k = A Im(zeta^k) of both poles by
+            // I_{k+1} = 2 Re(zeta) I_k - |zeta|^2 I_{k-1}
+            const double p = d + s, n = d - s, g2 = gam * gam;
+            const double p2 = 2.0 * p, n2 = 2.0 * n;
+            const double pp = -fma(p, p, g2), nn = -fma(n, n, g2);
+            double u0 = 0.0, u1 = A * gam, v0 = 0.0, v1 = u1;
+#pragma unroll
+            for (int j = 0; j < PM; ++j) {
+                m[j] += u1 + v1;
+                const double u = fma(p2, u1, pp * u0);
+                u0 = u1;
+                u1 = u;
+                const double v = fma(n2, v1, nn * v0);
+                v0 = v1;
+                v1 = v;
+            }
+        }
+        transpose_sum(m, lane);
+        if (lane < PM) M[size_t(lane) * C + k] = m[0];
+    }
+}
+
+template <bool MIXED>
+cudaError_t run_cells(const CellArgs& a, cudaStream_t st) {
+    const dim3 grid(unsigned((a.ncell + kCellWarps - 1) / kCellWarps),
+                    unsigned(a.group > 1 ? a.ncond / a.group : a.ncond));
+    switch (a.group) {
+        case 0: k_cells<MIXED, false, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        case 2: k_cells<MIXED, true, 2><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        case 4: k_cells<MIXED, true, 4><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        case 8: k_cells<MIXED, true, 8><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_cells(bool mixed, const CellArgs& a, cudaStream_t stream) {
+    if (a.ncell <= 0 || a.ncond <= 0) return cudaSuccess;
+    return mixed ? run_cells<true>(a, stream) : run_cells<false>(a, stream);
+}
+
+}  // namespace xs

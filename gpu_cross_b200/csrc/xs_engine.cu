@@ -48,6 +48,10 @@ int cuda_fail(cudaError_t e, const char* what) {
 // Most slices of a host line list (xs_engine_execute_host).
 constexpr int kMaxPieces = 16;
 
+// Least lines in a window, and least width of the window in tiles, from which
+// the far wings are taken by cells.
+constexpr double kCellMinLines = 1024.0, kCellMinTiles = 4.0;
+
 // Restores the caller's current device on scope exit.
 struct DeviceGuard {
     int prev = -1;
@@ -158,6 +162,34 @@ CondDev make_cond(const xs_options& o, const xs_condition& c) {
         d.cut = o.half_width * 10.0;
     }
     return d;
+}
+
+// Bytes of the cell heads and moments (both multiples of 16) of one launch.
+size_t cell_bytes(bool mixed, long n, int ncond, int group, int cshift) {
+    const size_t ncell = size_t((n + (1L << cshift) - 1) >> cshift);
+    const size_t groups = size_t(group ? ncond / group : ncond);
+    const size_t head = (sizeof(CellHead) * ncell * groups + 255) & ~size_t(255);
+    return head + sizeof(double) * size_t(cell_moments(mixed)) * ncell * size_t(ncond);
+}
+
+// Binary logarithm of the lines per cell, or 0 where the far wings are taken
+// line by line.  With L lines in a window, cells of N lines leave about N to
+// 5 N lines per point to be taken one by one beside the near ones and L / N
+// series to sum: N = sqrt(L) balances the two within a factor of two for both
+// precisions.
+int cell_shift(const xs_options& o, const xs_condition* conds, int ncond, long n, const xs_grid& grid, int group,
+               int CG, bool mixed, int tile_pts) {
+    if (o.profile != XS_VOIGT) return 0;
+    double cutmax = 0.0;
+    for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(o, conds[c]).cut);
+    const double win = 2.0 * cutmax, span = double(grid.points) * o.dfreq;
+    const double lines = double(n) * win / (span + win);
+    if (!(lines >= kCellMinLines) || !(win >= kCellMinTiles * double(tile_pts) * o.dfreq)) return 0;
+    int sh = int(std::lround(0.5 * std::log2(lines)));
+    sh = std::max(5, std::min(sh, 11));
+    if (ncond == 1)
+        while (cell_bytes(mixed, n, group, CG, sh) > kMaxPartBytes / 2) ++sh;
+    return sh;
 }
 
 // A-priori relative error bound of a result against the FP64 path of the
@@ -458,6 +490,13 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         double cutmax = 0.0;
         for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
         default_shape(kind, mixed, 2.0 * cutmax / opt->dfreq, &dP, &dW);
+        // Calls with fewer tiles than the GPU holds warps take narrower tiles:
+        // a line split needs a buffer and a reduction, a narrow tile neither.
+        // (3000 lines, 12000 points, 5000-point windows: step two 71 us with
+        // 94 tiles of 128 points in 3 parts, 39 us with 375 of 32 in 7.)
+        while (P == 0 && dP > 1 && kind == XS_VOIGT &&
+               double(grid->points) / (32.0 * dP) * ncond < 8.0 * e->num_sms)
+            dP /= 2;
         if (P == 0) P = dP;
         if (W == 0) W = dW;
     }
@@ -536,10 +575,11 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // walks a long line list, and with a few items per warp the last items
     // leave a tail.  Each tile's lines are then split into parts taken by
     // different warps -- enough for about 16 items per resident warp, at
-    // least ~256 lines per part, the parts' buffer within kMaxPartBytes.
+    // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
     const int tile_pts = CG ? 32 : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
+    const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, group, CG, mixed, tile_pts);
     int S = opt->line_splits;
     if (ov && ov->scratch) S = 1;  // a fixed caller scratch holds no parts
     if (S == 0) {
@@ -552,15 +592,23 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             const double span = double(grid->points) * opt->dfreq + 2.0 * cutmax;
             const double lpt = double(n) * (double(tile_pts) * opt->dfreq + 2.0 * cutmax) / span;
             long want = (16 * warps + items - 1) / items;
-            want = std::min<long>(want, long(lpt / 256.0));
-            const long cap = long(kMaxPartBytes / (sizeof(double) * size_t(group) * size_t(grid->points)));
+            want = std::min<long>(want, long(lpt / 128.0));
+            // (one condition: cells and parts together stay within kMaxPartBytes,
+            // what the server and the streamed lists reserve beside the records)
+            const size_t cells = cshift && ncond == 1 ? cell_bytes(mixed, n, group, CG, cshift) : 0;
+            const long cap = long((kMaxPartBytes - cells) / (sizeof(double) * size_t(group) * size_t(grid->points)));
             want = std::min<long>(want, std::min<long>(cap, kMaxSplits));
             if (want > 1) S = int(want);
         }
     }
-    const size_t part_off = (plan.need + 255) & ~size_t(255);
+    // Scratch after the records: cell heads and moments, then the split parts.
+    const int ncell = cshift ? int((n + (1L << cshift) - 1) >> cshift) : 0;
+    const size_t head_off = (plan.need + 255) & ~size_t(255);
+    const size_t mom_off = head_off + sizeof(CellHead) * size_t(ncell) * size_t(CG ? group / CG : group);
+    const size_t cell_end = cshift ? head_off + cell_bytes(mixed, n, group, CG, cshift) : plan.need;
+    const size_t part_off = (cell_end + 255) & ~size_t(255);
     const size_t part_end = S > 1 ? part_off + sizeof(double) * size_t(S) * size_t(group) * size_t(grid->points)
-                                  : plan.need;
+                                  : cell_end;
     // sampled FP64 check (mixed Voigt): before/ref values and statistics
     const bool streamed_call = ov && ov->s32;
     const int tiles32 = (grid->points + 31) / 32;
@@ -742,6 +790,25 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             if (err != cudaSuccess) return cuda_fail(err, "step one launch");
             ++launched;
         }
+        if (cshift) {
+            CellArgs la;
+            std::memset(&la, 0, sizeof(la));
+            la.nu = L.nu;
+            la.n = n;
+            la.ncond = nc;
+            la.group = CG;
+            la.rec = pa.rec;
+            la.cyp = pa.cyp;
+            la.cshift = cshift;
+            la.ncell = ncell;
+            la.df = G.df;
+            la.head = reinterpret_cast<CellHead*>(base + head_off);
+            la.mom = reinterpret_cast<double*>(base + ((mom_off + 255) & ~size_t(255)));
+            for (int c = 0; c < nc; ++c) la.dpw[c] = pa.cond[c].dpw;
+            err = launch_cells(mixed, la, st);
+            if (err != cudaSuccess) return cuda_fail(err, "cell moments launch");
+            ++launched;
+        }
         if (timing && c0 == 0) cudaEventRecordWithFlags(e->ev[1], st, ev_flags);
 
         StepArgs sa;
@@ -762,6 +829,12 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         sa.splits = S;
         sa.part = S > 1 ? reinterpret_cast<double*>(base + part_off) : nullptr;
         sa.part_stride = size_t(grid->points);
+        if (cshift) {
+            sa.chead = reinterpret_cast<const CellHead*>(base + head_off);
+            sa.cmom = reinterpret_cast<const double*>(base + ((mom_off + 255) & ~size_t(255)));
+            sa.ncell = ncell;
+            sa.cshift = cshift;
+        }
         sa.x0 = pa.x0;
         sa.xg = pa.xg;
         sa.x0g = pa.x0g;

@@ -175,6 +175,36 @@ struct __align__(16) RecE64 {
 };
 static_assert(sizeof(RecE64) == 48, "RecE64 layout");
 
+// Cells: runs of 2^cshift consecutive lines whose far wings step two sums
+// together.  Region I of W4 is the sum of two Lorentzians half a Doppler
+// width times sqrt 2 off the centre:
+//   Pc (u + 1) / (u^2 + 2 y^2) = A [Im 1/(f - z+) + Im 1/(f - z-)],
+//   z+- = nu +- a / sqrt 2 + i gamma,  A = S c / 2
+// (a = nu dpw the Doppler width, gamma = y a the Lorentz width, S = pref a,
+// c = kW4C), so with zeta = z - c0 a cell's lines add, at a grid point
+// further from the cell's centre c0 than every |zeta|,
+//   sum_k M_k / (f - c0)^(k+1),  M_k = sum over lines A Im(zeta+^k + zeta-^k):
+// one short polynomial in 1 / (f - c0) for all of the cell's lines instead of
+// one rational per line.  The terms after p add at most (p + 1) r^p / (1 - r)^2
+// of each line's own (positive) value, r = |zeta| / |f - c0|.  A cell is used
+// only on tiles that all of its lines' windows cover, from the distance dmin
+// on: kCellKappa times the largest |zeta|, and clear of every line's W4
+// regions II-IV.
+struct __align__(16) CellHead {
+    double c0;   // centre of the cell's lines
+    float dmin;  // least |f - c0| where the moments stand for the lines (inf: never)
+    float q;     // scale: at least every |zeta| of the cell, all conditions of the group
+};
+static_assert(sizeof(CellHead) == 16, "CellHead layout");
+constexpr float kCellKappa = 4.0f;
+// Moments kept, and the bits the terms beyond the ones evaluated are held
+// below: at the least distance (r = 1/4) the rest is 7e-16 of the line's value
+// with 28 terms (FP64) and 7e-9 with 16 (mixed, whose own arithmetic rounds at
+// 6e-8); further out fewer terms are evaluated (cell_terms in xs_kernels.cu).
+constexpr int kCellTerms64 = 28, kCellTermsMixed = 16;
+constexpr float kCellBits64 = 53.0f, kCellBitsMixed = 28.0f;
+constexpr int cell_moments(bool mixed) { return mixed ? kCellTermsMixed : kCellTerms64; }
+
 struct GridDev {
     const double* freq;  // full grid
     double f0, df;       // analytic grid f_j ~ f0 + j * df (f0 = freq[0])
@@ -270,6 +300,12 @@ struct StepArgs {
     int splits;
     double* part;
     size_t part_stride;
+    // Cells of 2^cshift lines (ncell = 0: none): heads and moments, per group
+    // of conditions (per condition in the single-condition layouts), moments
+    // as [cell][k][condition of the group].
+    const CellHead* chead;
+    const double* cmom;
+    int ncell, cshift;
     // Mixed multi-condition kernel: per condition k = 1 / dpw and k^2.
     float kx[kMaxCond];
     float kx2[kMaxCond];
@@ -277,6 +313,22 @@ struct StepArgs {
     // out + row[c] * out_stride.
     int row[kMaxCond];
 };
+
+// Cell moments (xs_cells.cu), from the records step one wrote.
+struct CellArgs {
+    const double* nu;   // line centres
+    long n;             // lines per condition
+    int ncond;
+    int group;          // conditions per group (0: single-condition layout)
+    const void* rec;    // RecV64 / RecV32, or CondRec64 (FP64 groups)
+    const float2* cyp;  // mixed groups: (y, pref)
+    int cshift, ncell;
+    double df;
+    CellHead* head;
+    double* mom;
+    double dpw[kMaxCond];
+};
+cudaError_t launch_cells(bool mixed, const CellArgs& a, cudaStream_t stream);
 
 // Kernel launchers (xs_kernels.cu).  All asynchronous on `stream`.
 cudaError_t launch_grid_check(const GridDev& g, unsigned* err, cudaStream_t stream);

@@ -776,6 +776,164 @@ __device__ __forceinline__ void put_result(const StepArgs& a, int c, int s, int 
 }
 
 // ---------------------------------------------------------------------------
+// Cells: which of a tile's lines are taken through their cells' moments.
+// ---------------------------------------------------------------------------
+// A tile's lines [La, Lb) as three runs taken line by line -- [La, r1),
+// [b2, e2), [b3, Lb) -- and two runs of cells [fa, fb), [fc, fd) taken by their
+// moments.  Without usable cells the first run is all of [La, Lb).
+struct LineRuns {
+    long La, r1, b2, e2, b3, Lb;
+    int fa, fb, fc, fd;
+    int g1, g2, total;  // 32-line groups of the first and the second run, of all three
+
+    // First line of the idx-th 32-line group, and the end of its run.
+    __device__ __forceinline__ long start(int idx, long& end) const {
+        if (idx < g1) {
+            end = r1;
+            return La + 32L * idx;
+        }
+        if (idx < g1 + g2) {
+            end = e2;
+            return b2 + 32L * (idx - g1);
+        }
+        end = Lb;
+        return b3 + 32L * (idx - g1 - g2);
+    }
+    // Groups of split s of S: s, s + S, s + 2 S, ...
+    __device__ __forceinline__ int groups_of(int S, int s) const { return total > s ? (total - s + S - 1) / S : 0; }
+};
+
+// [fs, fe): the lines whose windows cover the tile, whose grid points lie in
+// [ftlo, fthi] cm-1.  The cells inside it are taken by their moments from each
+// end up to the first one that is too near the tile; the cells in between are
+// taken line by line.
+__device__ __forceinline__ LineRuns line_runs(const CellHead* H, int ncell, int shift, long n, long La, long Lb,
+                                              long fs, long fe, double ftlo, double fthi, int lane) {
+    LineRuns r;
+    r.La = La;
+    r.Lb = Lb;
+    r.r1 = r.b2 = r.e2 = r.b3 = Lb;
+    r.fa = r.fb = r.fc = r.fd = 0;
+    if (ncell > 0) {
+        const int ca = int((fs + (1L << shift) - 1) >> shift);
+        const int cb = fe >= n ? ncell : int(fe >> shift);
+        if (ca < cb) {
+            auto near = [&](int ci) {
+                const CellHead h = H[ci];
+                return !(fmax(ftlo - h.c0, h.c0 - fthi) >= double(h.dmin));
+            };
+            int nl = cb, nr;
+            for (int b = ca; b < cb; b += 32) {
+                const unsigned m = __ballot_sync(0xffffffffu, b + lane < cb && near(b + lane));
+                if (m) {
+                    nl = b + __ffs(m) - 1;
+                    break;
+                }
+            }
+            nr = nl;
+            for (int e = cb; e > nl; e -= 32) {
+                const unsigned m = __ballot_sync(0xffffffffu, e - 1 - lane >= nl && near(e - 1 - lane));
+                if (m) {
+                    nr = e - (__ffs(m) - 1);
+                    break;
+                }
+            }
+            auto line_of = [&](int c) { return c >= ncell ? n : long(c) << shift; };
+            r.fa = ca;
+            r.fb = nl;
+            r.fc = nr;
+            r.fd = cb;
+            r.r1 = line_of(ca);
+            r.b2 = line_of(nl);
+            r.e2 = line_of(nr);
+            r.b3 = line_of(cb);
+        }
+    }
+    r.g1 = int((r.r1 - r.La + 31) / 32);
+    r.g2 = int((r.e2 - r.b2 + 31) / 32);
+    r.total = r.g1 + r.g2 + int((r.Lb - r.b3 + 31) / 32);
+    return r;
+}
+
+// Terms evaluated of a cell at the tile's least distance from it: enough for
+// (p + 1) r^p to lie below 2^-bits.  Even, so that moments load in pairs.
+template <int PM>
+__device__ __forceinline__ int cell_terms(float bits, double dist, float q) {
+    const int p = int(__fdividef(bits, __log2f(float(dist) / q))) + 3;
+    return p >= PM ? PM : (p & ~1);
+}
+
+// 1/x to FP64 rounding: the hardware approximation and two Newton-Raphson
+// steps (r <- r + r (1 - x r)).
+__device__ __forceinline__ double rcp_newton2_f64(double x) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    r = fma(r, fma(-x, r, 1.0), r);
+    return fma(r, fma(-x, r, 1.0), r);
+}
+
+// Adds the far cells of split s of S to the sums v of this lane's P points
+// f[] (one condition).
+template <int P, int PM>
+__device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
+                                              float bits, double ftlo, double fthi, const double (&f)[P],
+                                              double (&v)[P]) {
+    auto run = [&](int c0, int c1) {
+        for (int c = c0 + s; c < c1; c += S) {
+            const CellHead h = H[c];
+            const int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
+            const double2* m = reinterpret_cast<const double2*>(M + size_t(c) * PM);
+            double t[P], a[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                t[p] = double(h.q) * rcp_newton2_f64(f[p] - h.c0);
+                a[p] = 0.0;
+            }
+#pragma unroll 2
+            for (int k = np / 2 - 1; k >= 0; --k) {
+                const double2 mk = __ldg(m + k);
+#pragma unroll
+                for (int p = 0; p < P; ++p) a[p] = fma(fma(a[p], t[p], mk.y), t[p], mk.x);
+            }
+#pragma unroll
+            for (int p = 0; p < P; ++p) v[p] = fma(a[p] * t[p], t[p], v[p]);
+        }
+    };
+    run(r.fa, r.fb);
+    run(r.fc, r.fd);
+}
+
+// The same for one point and the C conditions of a group.
+template <int C, int PM>
+__device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
+                                                 float bits, double ftlo, double fthi, double f, double (&v)[C]) {
+    auto run = [&](int c0, int c1) {
+        for (int c = c0 + s; c < c1; c += S) {
+            const CellHead h = H[c];
+            const int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
+            const double2* m = reinterpret_cast<const double2*>(M + size_t(c) * PM * C);
+            const double t = double(h.q) * rcp_newton2_f64(f - h.c0);
+            double a[C];
+#pragma unroll
+            for (int q = 0; q < C; ++q) a[q] = 0.0;
+            for (int k = np - 1; k >= 0; --k) {
+#pragma unroll
+                for (int q = 0; q < C; q += 2) {
+                    const double2 mk = __ldg(m + (k * C + q) / 2);
+                    a[q] = fma(a[q], t, mk.x);
+                    a[q + 1] = fma(a[q + 1], t, mk.y);
+                }
+            }
+            const double t2 = t * t;
+#pragma unroll
+            for (int q = 0; q < C; ++q) v[q] = fma(a[q], t2, v[q]);
+        }
+    };
+    run(r.fa, r.fb);
+    run(r.fc, r.fd);
+}
+
+// ---------------------------------------------------------------------------
 // Step two, Voigt.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rcp_approx_f32(float x) {
@@ -1014,6 +1172,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
         const long E = warp_lower_bound(fs, fe, lane, [&](long i) { return mi[i] >= t0 - kc; });
         const long Fc = warp_lower_bound(E, fe, lane, [&](long i) { return mi[i] > tl + kc; });
         const REC* recs = recs_all + cbase;
+        const LineRuns runs = line_runs(a.chead + size_t(w.c) * size_t(a.ncell), a.ncell, a.cshift, a.n, La, Lb, fs,
+                                        fe, F[t0], F[tl], lane);
 
         int jj[P];
         float jf[P];
@@ -1228,16 +1388,17 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             }
         };
 
-        // this item's groups of 32 lines: gi-th starts at La + 32 (s + gi S)
-        const int ngroups = split_groups(Lb - La, a.splits, w.s);
-        auto gstart = [&](int gi) { return La + 32L * (w.s + long(gi) * a.splits); };
+        // this item's groups of 32 lines
+        const int ngroups = runs.groups_of(a.splits, w.s);
+        auto gstart = [&](int gi, long& end) { return runs.start(w.s + gi * a.splits, end); };
         // kStages-deep cp.async pipeline: groups gi+1 .. gi+kStages-1 are in
         // flight while group gi is evaluated (one commit per step, empty
         // commits past the end keep the group count uniform).
         auto issue = [&](int g) {
             if (g < ngroups) {
-                const long b = gstart(g);
-                const long rem = Lb - b;
+                long end;
+                const long b = gstart(g, end);
+                const long rem = end - b;
                 stage(buf + (g % kStages) * 32, recs + b, int(rem < 32 ? rem : 32), lane);
             }
             cp_async_commit();
@@ -1249,8 +1410,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             cp_async_wait<kStages - 1>();
             __syncwarp();
             const REC* R = buf + (gi % kStages) * 32;
-            const long gb = gstart(gi);
-            const long ge = Lb - gb < 32 ? Lb : gb + 32;
+            long end;
+            const long gb = gstart(gi, end);
+            const long ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](long v) { return int((v < gb ? gb : (v > ge ? ge : v)) - gb); };
             const int a0 = lo_of(La), a1 = lo_of(fs);
             const int b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe), e1 = lo_of(Lb);
@@ -1304,13 +1466,21 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             }
             __syncwarp();
         }
+        double v[P];
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            if (jj[p] < t1) {
-                const double v = MIXED ? double(sumf[p]) - double(cmpf[p]) : accd[p];
-                put_result(a, w.c, w.s, jj[p], v);
-            }
+        for (int p = 0; p < P; ++p) v[p] = MIXED ? double(sumf[p]) - double(cmpf[p]) : accd[p];
+        if (runs.fa < runs.fb || runs.fc < runs.fd) {
+            constexpr int PM = cell_moments(MIXED);
+            const size_t cell0 = size_t(w.c) * size_t(a.ncell);
+            double f[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) f[p] = F[jj[p] < t1 ? jj[p] : tl];
+            add_far_cells<P, PM>(a.chead + cell0, a.cmom + cell0 * PM, runs, a.splits, w.s,
+                                 MIXED ? kCellBitsMixed : kCellBits64, F[t0], F[tl], f, v);
         }
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+            if (jj[p] < t1) put_result(a, w.c, w.s, jj[p], v[p]);
     }
 }
 
@@ -1382,6 +1552,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
         const LineSh64* lsh = reinterpret_cast<const LineSh64*>(a.lsh) + gbase;
         const CondRec64* crec = reinterpret_cast<const CondRec64*>(a.rec) + gbase * C;
 
+        const size_t cell0 = size_t(cg) * size_t(a.ncell);
+        const LineRuns runs =
+            line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
+
         const int jj = t0 + lane;
         const double fj = F[jj < t1 ? jj : tl];
         double accd[C];
@@ -1417,22 +1591,24 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             push(special, ax, r.y, r.pref, c);
         };
 
-        // this item's groups of 32 lines: gi-th starts at La + 32 (s + gi S)
-        const int ngroups = split_groups(Lb - La, a.splits, split);
-        auto gstart = [&](int gi) { return La + 32L * (split + long(gi) * a.splits); };
+        // this item's groups of 32 lines
+        const int ngroups = runs.groups_of(a.splits, split);
+        auto gstart = [&](int gi, long& end) { return runs.start(split + gi * a.splits, end); };
         auto stage_group = [&](int bufi, long b, int cnt) {
             stage(lsb + bufi * 32, lsh + b, cnt, lane);
             stage(crb + bufi * 32 * C, crec + b * C, cnt * C, lane);
         };
         if (ngroups > 0) {
-            const long b = gstart(0);
-            stage_group(0, b, int(Lb - b < 32 ? Lb - b : 32));
+            long end;
+            const long b = gstart(0, end);
+            stage_group(0, b, int(end - b < 32 ? end - b : 32));
             cp_async_commit();
         }
         for (int gi = 0; gi < ngroups; ++gi) {
             if (gi + 1 < ngroups) {
-                const long b = gstart(gi + 1);
-                const long rem = Lb - b;
+                long end;
+                const long b = gstart(gi + 1, end);
+                const long rem = end - b;
                 stage_group((gi + 1) & 1, b, int(rem < 32 ? rem : 32));
                 cp_async_commit();
                 cp_async_wait<1>();
@@ -1442,8 +1618,9 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             __syncwarp();
             const LineSh64* SL = lsb + (gi & 1) * 32;
             const CondRec64* SC = crb + (gi & 1) * 32 * C;
-            const long gb = gstart(gi);
-            const long ge = Lb - gb < 32 ? Lb : gb + 32;
+            long end;
+            const long gb = gstart(gi, end);
+            const long ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](long v) { return int((v < gb ? gb : (v > ge ? ge : v)) - gb); };
             const int a0 = lo_of(La), a1 = lo_of(fs), b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe),
                       e1 = lo_of(Lb);
@@ -1513,6 +1690,9 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             cq.corr[c][lane] = 0.0;
         }
         __syncwarp();
+        if (runs.fa < runs.fb || runs.fc < runs.fd)
+            add_far_cells_mc<C, kCellTerms64>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs, a.splits,
+                                              split, kCellBits64, F[t0], F[tl], fj, accd);
         if (jj < t1) {
 #pragma unroll
             for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, accd[c]);
@@ -1598,6 +1778,11 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
         }
         const LineShX* lsh = reinterpret_cast<const LineShX*>(a.lsh) + wbase;
         const R1* r1 = reinterpret_cast<const R1*>(a.rec) + gbase;
+
+        const double* F = a.G.freq;
+        const size_t cell0 = size_t(cg) * size_t(a.ncell);
+        const LineRuns runs =
+            line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
 
         const int jj = t0 + lane;
         const float jf = float(jj);
@@ -1698,8 +1883,13 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             acc[pB] = __ffma2_rn(nB, f2(q2 ? iB.x : 0.0f, q3 ? iB.y : 0.0f), acc[pB]);
         };
 
-        const int ngroups = split_groups(Lb - La, a.splits, split);
-        auto gstart = [&](int gi) { return La + 32 * (split + gi * a.splits); };
+        const int ngroups = runs.groups_of(a.splits, split);
+        auto gstart = [&](int gi, int& end) {
+            long e;
+            const int b = int(runs.start(split + gi * a.splits, e));
+            end = int(e);
+            return b;
+        };
         auto stage_group = [&](int bufi, int b, int cnt) {
             if (lane < cnt) {
                 cp_async16(lsb + bufi * 32 + lane, lsh + b + lane);
@@ -1708,14 +1898,16 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             stage(rb + bufi * 32, r1 + b, cnt, lane);
         };
         if (ngroups > 0) {
-            const int b = gstart(0);
-            stage_group(0, b, Lb - b < 32 ? Lb - b : 32);
+            int end;
+            const int b = gstart(0, end);
+            stage_group(0, b, end - b < 32 ? end - b : 32);
             cp_async_commit();
         }
         for (int gi = 0; gi < ngroups; ++gi) {
             if (gi + 1 < ngroups) {
-                const int b = gstart(gi + 1);
-                const int rem = Lb - b;
+                int end;
+                const int b = gstart(gi + 1, end);
+                const int rem = end - b;
                 stage_group((gi + 1) & 1, b, rem < 32 ? rem : 32);
                 cp_async_commit();
                 cp_async_wait<1>();
@@ -1726,8 +1918,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             const float4* SL = lsb + (gi & 1) * 32;  // m, df/nu, r/nu, flags
             const int2* SW = lhb + (gi & 1) * 32;    // window [lo, hi)
             const R1* SR = rb + (gi & 1) * 32;
-            const int gb = gstart(gi);
-            const int ge = Lb - gb < 32 ? Lb : gb + 32;
+            int end;
+            const int gb = gstart(gi, end);
+            const int ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](int v) { return (v < gb ? gb : (v > ge ? ge : v)) - gb; };
             const int a0 = lo_of(La), a1 = lo_of(fs), b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe),
                       e1 = lo_of(Lb);
@@ -1890,12 +2083,19 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             }
             __syncwarp();
         }
+        double v[C];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            v[2 * p] = double(sum[p].x) - double(cmp[p].x);
+            v[2 * p + 1] = double(sum[p].y) - double(cmp[p].y);
+        }
+        if (runs.fa < runs.fb || runs.fc < runs.fd)
+            add_far_cells_mc<C, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C), runs,
+                                                 a.splits, split, kCellBitsMixed, F[t0], F[tl],
+                                                 F[jj < t1 ? jj : tl], v);
         if (jj < t1) {
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                put_result(a, cg * C + 2 * p, split, jj, double(sum[p].x) - double(cmp[p].x));
-                put_result(a, cg * C + 2 * p + 1, split, jj, double(sum[p].y) - double(cmp[p].y));
-            }
+            for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, v[c]);
         }
     }
 }

@@ -48,9 +48,12 @@ int cuda_fail(cudaError_t e, const char* what) {
 // Most slices of a host line list (xs_engine_execute_host).
 constexpr int kMaxPieces = 16;
 
-// Least lines in a window, and least width of the window in tiles, from which
-// the far wings are taken by cells.
-constexpr double kCellMinLines = 1024.0, kCellMinTiles = 4.0;
+// Least lines in a window, width of the window in tiles, and pairs of the call
+// from which the far wings are taken by cells.  (Below 1.2e7 pairs, some 10 us
+// of step two, the GPU is not full either way and the series' launch and the
+// search for far cells cost what they save: 2000 lines on 4001 points, 7e6
+// pairs, 26 us without and 69 us with cells.)
+constexpr double kCellMinLines = 1024.0, kCellMinTiles = 4.0, kCellMinPairs = 1.2e7;
 
 // Restores the caller's current device on scope exit.
 struct DeviceGuard {
@@ -98,8 +101,15 @@ int set_error(int code, const char* msg) { return fail(code, msg); }
 // shared by more points), narrow on coarse grids, where a 128-point tile
 // would hold mostly partial and core lines.  4 warps per block (the mixed
 // kernels then fit 28 warps per SM).
-void default_shape(int kind, bool mixed, double window_points, int* P, int* warps) {
-    if (kind == kVoigt) {
+// With the far wings taken by cells, what is left line by line is the lines
+// near the tile and those whose windows end in it, so narrow tiles win: FP64
+// single point (1e7 lines, 7.5e5 points) 10.3 ms of step two at P = 4, 7.6 at
+// 2, 7.1 at 1; mixed 6.6, 4.7 (8 warps), 4.9.
+void default_shape(int kind, bool mixed, bool cells, double window_points, int* P, int* warps) {
+    if (kind == kVoigt && cells) {
+        *P = mixed ? 2 : 1;
+        *warps = mixed ? 8 : 4;
+    } else if (kind == kVoigt) {
         *P = window_points >= 2048.0 ? 4 : (window_points >= 512.0 ? 2 : 1);
         *warps = 4;
     } else {
@@ -177,18 +187,21 @@ size_t cell_bytes(bool mixed, long n, int ncond, int group, int cshift) {
 // 5 N lines per point to be taken one by one beside the near ones and L / N
 // series to sum: N = sqrt(L) balances the two within a factor of two for both
 // precisions.
-int cell_shift(const xs_options& o, const xs_condition* conds, int ncond, long n, const xs_grid& grid, int group,
-               int CG, bool mixed, int tile_pts) {
+int cell_shift(const xs_options& o, const xs_condition* conds, int ncond, long n, const xs_grid& grid,
+               int tile_pts) {
     if (o.profile != XS_VOIGT) return 0;
     double cutmax = 0.0;
     for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(o, conds[c]).cut);
     const double win = 2.0 * cutmax, span = double(grid.points) * o.dfreq;
     const double lines = double(n) * win / (span + win);
-    if (!(lines >= kCellMinLines) || !(win >= kCellMinTiles * double(tile_pts) * o.dfreq)) return 0;
+    const double pairs = lines * double(grid.points) * double(ncond);
+    if (!(lines >= kCellMinLines) || !(win >= kCellMinTiles * double(tile_pts) * o.dfreq) ||
+        !(pairs >= kCellMinPairs))
+        return 0;
     int sh = int(std::lround(0.5 * std::log2(lines)));
     sh = std::max(5, std::min(sh, 11));
     if (ncond == 1)
-        while (cell_bytes(mixed, n, group, CG, sh) > kMaxPartBytes / 2) ++sh;
+        while (cell_bytes(o.precision == XS_MIXED, n, 1, 0, sh) > kMaxPartBytes / 2) ++sh;
     return sh;
 }
 
@@ -485,11 +498,13 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             C = it->second.C;
         }
     }
+    // (32-point tiles decide whether the call's far wings can go by cells)
+    const bool cells = !(ov && ov->scratch) && cell_shift(*opt, conds, ncond, n, *grid, 32) > 0;
     {
         int dP, dW;
         double cutmax = 0.0;
         for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
-        default_shape(kind, mixed, 2.0 * cutmax / opt->dfreq, &dP, &dW);
+        default_shape(kind, mixed, cells, 2.0 * cutmax / opt->dfreq, &dP, &dW);
         // Calls with fewer tiles than the GPU holds warps take narrower tiles:
         // a line split needs a buffer and a reduction, a narrow tile neither.
         // (3000 lines, 12000 points, 5000-point windows: step two 71 us with
@@ -542,9 +557,11 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             C = 1;
         } else if (C == 0) {
             // Measured on B200 (40-condition sweep, 0.1 cm-1 grid): two
-            // conditions per warp is fastest for the mixed path; the FP64
-            // path is faster with one condition and 32*P points per warp.
-            C = (mixed && groups_ok(2)) ? 2 : 1;
+            // conditions per warp is fastest for the mixed path, and for the
+            // FP64 path with cells (8 conditions, 1e6 lines: 2.25 ms of step
+            // two against 2.80 with one); without cells FP64 is faster with
+            // one condition and 32*P points per warp.
+            C = (mixed || cells) && groups_ok(2) ? 2 : 1;
         } else if (C > 1 && !groups_ok(C)) {
             return fail(XS_ERR_INVALID, "conditions_per_warp needs ncond <= 64 and, for every cut, a "
                                         "number of conditions that is a multiple of it");
@@ -579,24 +596,31 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // The count depends only on the call's sizes and the SM count.
     const int tile_pts = CG ? 32 : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
-    const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, group, CG, mixed, tile_pts);
+    const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
     if (ov && ov->scratch) S = 1;  // a fixed caller scratch holds no parts
     if (S == 0) {
         const long items = long(tiles) * (CG ? group / CG : group);
         const long warps = long(occ) * W * e->num_sms;
         S = 1;
-        if (items < 16 * warps) {
+        // With cells the lines taken one by one are those near the tile and
+        // at its window ends, some 8 cells and 3 tile widths: fewer, larger
+        // parts (300k-line FP64 band, 3126 tiles: 0.42 ms of step two in 1
+        // part per tile, 0.33 in 4, 0.43 in 16).
+        const long waves = cshift ? 6 : 16;
+        if (items < waves * warps) {
             double cutmax = 0.0;
             for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
             const double span = double(grid->points) * opt->dfreq + 2.0 * cutmax;
-            const double lpt = double(n) * (double(tile_pts) * opt->dfreq + 2.0 * cutmax) / span;
-            long want = (16 * warps + items - 1) / items;
-            want = std::min<long>(want, long(lpt / 128.0));
+            double lpt = double(n) * (double(tile_pts) * opt->dfreq + 2.0 * cutmax) / span;
+            if (cshift)
+                lpt = std::min(lpt, double(n) * 3.0 * double(tile_pts) * opt->dfreq / span + double(8L << cshift));
+            long want = (waves * warps + items - 1) / items;
+            want = std::min<long>(want, long(lpt / (cshift ? 64.0 : 128.0)));
             // (one condition: cells and parts together stay within kMaxPartBytes,
             // what the server and the streamed lists reserve beside the records)
-            const size_t cells = cshift && ncond == 1 ? cell_bytes(mixed, n, group, CG, cshift) : 0;
-            const long cap = long((kMaxPartBytes - cells) / (sizeof(double) * size_t(group) * size_t(grid->points)));
+            const size_t cell_b = cshift && ncond == 1 ? cell_bytes(mixed, n, group, CG, cshift) : 0;
+            const long cap = long((kMaxPartBytes - cell_b) / (sizeof(double) * size_t(group) * size_t(grid->points)));
             want = std::min<long>(want, std::min<long>(cap, kMaxSplits));
             if (want > 1) S = int(want);
         }

@@ -68,18 +68,20 @@ struct CondDev {
 // rational as c y (0.5 + x^2 + y^2) / ((0.5 + y^2 - x^2)^2 + 4 x^2 y^2), since
 // (0.5 + y^2 - x^2)^2 + 4 x^2 y^2 = (x^2 + y^2 - 0.5)^2 + 2 y^2.  In region I
 // (|x| + y >= 15) u > 190, so nothing cancels.
-// FP64 record: the first three 16-byte chunks are all the fast path reads.
+// FP64 record: the first three 16-byte chunks are all the fast path reads, the
+// first four all that step two's lines need (kRecV64Staged bytes).
 struct __align__(16) RecV64 {
     double nu;     // line centre used for offsets
     double g;      // 1 / Doppler width
     double Cy, D2;
     double Pc, y;  // y = Lorentz / Doppler width ratio
-    double pref;   // S * g
-    double pad;
     int lo, hi;    // window [lo, hi) of grid indices
     int clo, chi;  // grid indices near the core (region I not guaranteed)
+    double pref;   // S * g
+    double pad;
 };
 static_assert(sizeof(RecV64) == 80, "RecV64 layout");
+constexpr int kRecV64Staged = 64;
 
 // Mixed-precision record (FP32).  The offset of grid point j from the line
 // centre is (m - j) * df + r in cm-1, with m the nearest grid index and

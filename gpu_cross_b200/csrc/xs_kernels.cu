@@ -736,6 +736,16 @@ __device__ __forceinline__ void stage(REC* dst, const REC* src, int cnt, int lan
     for (int q = lane; q < total; q += 32) cp_async16(d + 16 * q, s + 16 * q);
 }
 
+// The same for the first BYTES of records STRIDE bytes apart.
+template <int BYTES, int STRIDE>
+__device__ __forceinline__ void stage_rec(void* dst, const void* src, int cnt, int lane) {
+    constexpr int kChunks = BYTES / 16;
+    const char* s = static_cast<const char*>(src);
+    char* d = static_cast<char*>(dst);
+    for (int q = lane; q < cnt * kChunks; q += 32)
+        cp_async16(d + 16 * q, s + (BYTES == STRIDE ? 16 * q : (q / kChunks) * STRIDE + (q % kChunks) * 16));
+}
+
 struct WorkItem {
     int c, t0, t1, s;
 };
@@ -973,6 +983,7 @@ __device__ __forceinline__ fcplx operator*(fcplx a, fcplx b) {
 // denominators lie between about 0.5 and 1e6, far from the range where the
 // approximation fails.  Region IV, which subtracts, keeps the IEEE division.
 __device__ __forceinline__ float region_div(float a, float b) { return __fdividef(a, b); }
+__device__ __forceinline__ double region_div(double a, double b) { return a * rcp_newton2_f64(b); }
 
 template <class R>
 __device__ __forceinline__ R w4_region2_re(R x, R y) {
@@ -1043,69 +1054,88 @@ __device__ float w4_region4_re_f32(float x, float y) {
 //   partial [La, fs) | fast [fs, E) | core [E, F) | fast [F, fe) | partial [fe, Lb)
 // Fast lines evaluate W4 region I on every pair with no test at all.  Core
 // and partial lines classify whole rows (outside the window: skipped; inside
-// and clear of the core band: as fast; otherwise lane by lane).  Pairs that
-// need W4 regions II-IV are not evaluated in place -- that would run the
-// union of the region code paths with a few lanes active -- but pushed to a
-// per-warp queue in shared memory and evaluated 32 at a time, one per lane;
-// each lane then adds the results addressed to it, in queue order, to a
-// per-lane correction column.  The order of every sum is fixed.
-template <class T>
-struct CoreEntry {
-    T x, y, pref;
-    int dest;  // lane | (row << 5)
-};
+// and clear of the core band: as fast; otherwise lane by lane).  Pairs of W4
+// regions II-IV are left out there: the FP64 kernels take them in a pass of
+// their own after the tile's lines (core_row_f64, lane = line), the mixed ones
+// in separate kernels.
 
-template <int P, bool MIXED>
-struct WarpCoreQueue {
-    using T = typename std::conditional<MIXED, float, double>::type;
-    static constexpr int kCap = 32 * (P + 1);  // < 32 left + up to P rows of 32 (rows of
-                                               // points, or conditions)
-    CoreEntry<T> q[kCap];
-    T corr[P][32];
-};
+// W4 regions III and IV in FP64, real parts; complex Horner schemes (T = y - ix).
+__device__ __forceinline__ double w4_region3_re_f64(double x, double y) {
+    const cplx t = {y, -x};
+    const cplx num = 16.4955 + t * (20.20933 + t * (11.96482 + t * (3.778987 + t * .5642236)));
+    const cplx den = 16.4955 + t * (38.82363 + t * (39.27121 + t * (21.69274 + t * (6.699398 + t))));
+    return (num.re * den.re + num.im * den.im) * rcp_newton2_f64(den.re * den.re + den.im * den.im);
+}
+__device__ __forceinline__ double w4_region4_re_f64(double x, double y) {
+    const cplx t = {y, -x};
+    const cplx u = t * t;
+    const cplx num = t * (36183.31 - u * (3321.9905 - u * (1540.787 - u * (219.0313 -
+                          u * (35.76683 - u * (1.320522 - u * .56419))))));
+    const cplx den = 32066.6 - u * (24322.84 - u * (9022.228 - u * (2186.181 -
+                          u * (364.2191 - u * (61.57037 - u * (1.841439 - u))))));
+    return exp(u.re) * cos(u.im) -
+           (num.re * den.re + num.im * den.im) * rcp_newton2_f64(den.re * den.re + den.im * den.im);
+}
 
-// Evaluates the first k (<= 32) queued pairs, one per lane, adds each result
-// to its destination lane's correction column in queue order, and moves the
-// rest of the queue to the front.  Returns the new queue length.  Kept out of
-// line: it runs once per 32 pairs and holds all of W4's regions II-IV.
-template <int P, bool MIXED>
-__device__ __noinline__ int core_queue_flush(WarpCoreQueue<P, MIXED>& cq, int qn, int k, int lane) {
-    static_assert(!MIXED, "the mixed paths evaluate their core pairs in a core pass");
-    using T = typename WarpCoreQueue<P, MIXED>::T;
-    T v = T(0);
-    int dest = 0;
-    if (lane < k) {
-        const CoreEntry<T> e = cq.q[lane];
-        dest = e.dest;
-        v = T(w4_re(double(e.x), double(e.y)) * double(e.pref));
+// Per-warp table of the FP64 core pass: [point of the row][lane].
+constexpr int kCoreRow64 = 33;
+constexpr size_t kCoreTable64 = sizeof(double) * 32 * kCoreRow64;
+
+// W4 regions II-IV of the FP64 path on one row of 32 grid points [r0, r0 + 32):
+// the lines [E, Fc) are taken 32 at a time (batches s, s + S, ...), lane = line,
+// each lane going over its line's points jlo..jhi (core band and window, from
+// `get`) and adding to its own column of the table T; the columns are added up
+// in lane order at the end, so the order of every sum is fixed.  Region II and
+// regions III-IV run in loops of their own: neighbouring lines have nearly the
+// same intervals, so a warp step runs one region's code on most of its lanes.
+// x, y and the region choice are the reference's.  Returns this lane's point's
+// sum.
+//
+// Before, the pairs went through a shared-memory queue, 32 at a time over all
+// regions, between step two's lines.
+template <class Get>
+__device__ __forceinline__ double core_row_f64(double (*T)[kCoreRow64], const double* F, long E, long Fc, int r0,
+                                               int S, int s, int lane, Get get) {
+    // Few candidate lines (sparse lists, small calls): 2 or 4 lanes to a line,
+    // on every second or fourth point, so that one batch's chain is shorter.
+    const int sh = Fc - E <= 8L * S ? 2 : (Fc - E <= 16L * S ? 1 : 0);
+    const int nb = 32 >> sh, sub = lane & ((1 << sh) - 1), step = 1 << sh;
+    if (E + long(nb) * s >= Fc) return 0.0;
+#pragma unroll 4
+    for (int q = 0; q < 32; ++q) T[q][lane] = 0.0;
+    bool any = false;
+    for (long b = E + long(nb) * s; b < Fc; b += long(nb) * S) {
+        const long i = b + (lane >> sh);
+        double nu = 0.0, g = 0.0, y = 0.0, pref = 0.0;
+        int jlo = 1, jhi = 0;
+        if (i < Fc) get(i, nu, g, y, pref, jlo, jhi);
+        int b0 = INT_MAX, b1 = -1;
+        for (int j = jlo + sub; j <= jhi; j += step) {
+            const double ax = fabs((nu - F[j]) * g);
+            const double sx = ax + y;
+            if (sx >= 15.0) continue;
+            any = true;
+            if (sx >= 5.5) {
+                T[j - r0][lane] += pref * w4_region2_re<double>(ax, y);
+            } else {
+                b0 = min(b0, j);
+                b1 = j;
+            }
+        }
+        for (int j = b0; j <= b1; j += step) {
+            const double ax = fabs((nu - F[j]) * g);
+            const double w = y >= 0.195 * ax - 0.176 ? w4_region3_re_f64(ax, y) : w4_region4_re_f64(ax, y);
+            T[j - r0][lane] += pref * w;
+        }
     }
-    // Each push queued a run of consecutive lanes of one row, so the queue is
-    // a sequence of runs (entry s + i is lane first + i).  Runs are visited in
-    // queue order and each lane takes at most one entry per run: every lane's
-    // correction column gets its entries in queue order.
-    const int prev = __shfl_up_sync(0xffffffffu, dest, 1);
-    const bool start = lane < k && (lane == 0 || dest != prev + 1 || (dest & 31) == 0);
-    unsigned starts = __ballot_sync(0xffffffffu, start);
-    while (starts) {
-        const int s0 = __ffs(starts) - 1;
-        starts &= starts - 1;
-        const int e0 = starts ? __ffs(starts) - 1 : k;
-        const int d0 = __shfl_sync(0xffffffffu, dest, s0);
-        const int first = d0 & 31, row = d0 >> 5;
-        const T vv = __shfl_sync(0xffffffffu, v, (s0 + lane - first) & 31);
-        if (lane >= first && lane < first + (e0 - s0)) cq.corr[row][lane] += vv;
-    }
+    any = __any_sync(0xffffffffu, any);
     __syncwarp();
-    const int rem = qn - k;
-    for (int base = 0; base < rem; base += 32) {
-        CoreEntry<T> keep;
-        const int i = base + lane;
-        if (i < rem) keep = cq.q[k + i];
-        __syncwarp();
-        if (i < rem) cq.q[i] = keep;
-        __syncwarp();
-    }
-    return rem;
+    if (!any) return 0.0;
+    double sum = 0.0;
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) sum += T[lane][q];
+    __syncwarp();
+    return sum;
 }
 
 // Resident blocks per SM the step-two Voigt kernel asks the compiler to fit
@@ -1118,43 +1148,26 @@ constexpr int voigt_min_blocks() {
     return (MIXED && P == 4 && WARPS == 4) ? 7 : (MIXED && P <= 2 && WARPS == 4) ? 8 : (MIXED && P <= 4) ? 24 / WARPS : 1;
 }
 
+// Shared memory of one warp of it.
+constexpr size_t voigt_warp_smem(bool mixed) {
+    const size_t staged = size_t(32) * kStages * (mixed ? sizeof(RecV32) : size_t(kRecV64Staged));
+    return mixed || staged > kCoreTable64 ? staged : kCoreTable64;
+}
+
 template <int P, int WARPS, bool MIXED>
 __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>()))
     k_steptwo_voigt(StepArgs a) {
     using REC = typename std::conditional<MIXED, RecV32, RecV64>::type;
     using T = typename std::conditional<MIXED, float, double>::type;
-    using Q = WarpCoreQueue<P, MIXED>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    REC* buf = reinterpret_cast<REC*>(smem_raw) + warp * 32 * kStages;
-    // the core queue (FP64 only: the mixed path leaves regions II-IV to
-    // k_core_v32 and has no queue in shared memory)
-    Q& cq = reinterpret_cast<Q*>(smem_raw + size_t(WARPS) * 32 * kStages * sizeof(REC))[warp];
+    // staged records, kStages groups of 32; the FP64 core pass's table takes
+    // the same space after the tile's lines
+    constexpr int kRec = MIXED ? int(sizeof(REC)) : kRecV64Staged;
+    unsigned char* const mine = smem_raw + size_t(warp) * voigt_warp_smem(MIXED);
     const REC* recs_all = reinterpret_cast<const REC*>(a.rec);
     const double* F = a.G.freq;
-    const unsigned lt_mask = (1u << lane) - 1u;
-
-    if constexpr (!MIXED) {
-#pragma unroll
-        for (int p = 0; p < P; ++p) cq.corr[p][lane] = T(0);
-    }
-    int qn = 0;  // entries in the queue (warp-uniform)
-
-    auto push = [&](bool need, T x, T y, T pref, int p) {
-        const unsigned b = __ballot_sync(0xffffffffu, need);
-        if (b == 0u) return;
-        if (need) {
-            CoreEntry<T> e;
-            e.x = x;
-            e.y = y;
-            e.pref = pref;
-            e.dest = lane | (p << 5);
-            cq.q[qn + __popc(b & lt_mask)] = e;
-        }
-        qn += __popc(b);
-        __syncwarp();
-    };
 
     WorkItem w;
     while (next_item(a, P, lane, w)) {
@@ -1191,9 +1204,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
 
         // Region I on every row: u = x^2 + Cy, acc += Pc (u + 1) / (u^2 + D2);
         // in FP32 two rows at a time as packed FP32x2 operations.
-        auto fast_line = [&](const REC& r) {
+        auto fast_line = [&](const unsigned char* r) {
             if (MIXED) {
-                const float4* q = reinterpret_cast<const float4*>(&r);
+                const float4* q = reinterpret_cast<const float4*>(r);
                 const float4 v0 = q[0], v1 = q[1];
                 if constexpr (P % 2 == 0) {
 #pragma unroll
@@ -1217,7 +1230,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     }
                 }
             } else {
-                const double2* q = reinterpret_cast<const double2*>(&r);
+                const double2* q = reinterpret_cast<const double2*>(r);
                 const double2 v0 = q[0], v1 = q[1], v2 = q[2];
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
@@ -1228,11 +1241,11 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             }
         };
         // `full`: the line's window covers the whole tile.
-        auto slow_line = [&](const REC& r, bool full) {
+        auto slow_line = [&](const unsigned char* r, bool full) {
             if (MIXED) {
                 // region I except the pairs of the region interval [clo, chi]
                 // (the core pass takes those)
-                const float4* q = reinterpret_cast<const float4*>(&r);
+                const float4* q = reinterpret_cast<const float4*>(r);
                 const float4 v0 = q[0], v1 = q[1], v2 = q[2];
                 const float m = v0.x, ra = v0.y, dfa = v0.z, Cy = v0.w;
                 const float D2 = v1.x, Pc = v1.y;
@@ -1244,7 +1257,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     if (!full && (r0 >= hi || r1 < lo)) continue;
                     const bool row_in = full || (r0 >= lo && r1 < hi);
                     const bool row_core = whole || !(r1 < clo || r0 > chi);
-                    const float xs = whole ? float((r.nu - F[jj[p] < t1 ? jj[p] : tl]) / r.nu) * a.kx[w.c]
+                    const float xs = whole ? float((reinterpret_cast<const RecV32*>(r)->nu - F[jj[p] < t1 ? jj[p] : tl]) / reinterpret_cast<const RecV32*>(r)->nu) * a.kx[w.c]
                                            : fmaf(m - jf[p], dfa, ra);
                     const float u = fmaf(xs, xs, Cy);
                     const float num = fmaf(u, Pc, Pc);
@@ -1260,11 +1273,10 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     accf[p] += keep ? num * rr : 0.0f;
                 }
             } else {
-                const double2* q = reinterpret_cast<const double2*>(&r);
-                const double2 v0 = q[0], v1 = q[1], v2 = q[2], v3 = q[3];
-                const int4 vi = reinterpret_cast<const int4*>(&r)[4];
+                const double2* q = reinterpret_cast<const double2*>(r);
+                const double2 v0 = q[0], v1 = q[1], v2 = q[2];
+                const int4 vi = reinterpret_cast<const int4*>(r)[3];
                 const double nu = v0.x, g = v0.y, Cy = v1.x, D2 = v1.y, Pc = v2.x, y = v2.y;
-                const double pref = v3.x;
                 const int lo = vi.x, hi = vi.y, clo = vi.z, chi = vi.w;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
@@ -1287,7 +1299,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                         const double u = fma(xs, xs, Cy);
                         accd[p] = fma(fma(u, Pc, Pc), rcp_refined_f64(fma(u, u, D2)), accd[p]);
                     }
-                    if (row_core) push(in && exact, ax, y, pref, p);
                 }
             }
         };
@@ -1295,9 +1306,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
         // A line whose window covers only part of the tile and whose core
         // band misses it: rows outside the window are skipped, the boundary
         // row is masked lane by lane.
-        auto partial_line = [&](const REC& r) {
+        auto partial_line = [&](const unsigned char* r) {
             if (MIXED) {
-                const float4* q = reinterpret_cast<const float4*>(&r);
+                const float4* q = reinterpret_cast<const float4*>(r);
                 const float4 v0 = q[0], v1 = q[1], v2 = q[2];
                 const float lo = v2.x, hi = v2.y;
                 // region interval reaching the tile, or a whole line
@@ -1316,9 +1327,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     accf[p] = fmaf(fmaf(u, v1.y, v1.y), rr, accf[p]);
                 }
             } else {
-                const double2* q = reinterpret_cast<const double2*>(&r);
+                const double2* q = reinterpret_cast<const double2*>(r);
                 const double2 v0 = q[0], v1 = q[1], v2 = q[2];
-                const int4 vi = reinterpret_cast<const int4*>(&r)[4];
+                const int4 vi = reinterpret_cast<const int4*>(r)[3];
                 const int lo = vi.x, hi = vi.y;
                 if (!(vi.w < t0 || vi.z > tl)) {
                     slow_line(r, false);
@@ -1337,18 +1348,17 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             }
         };
         // A line whose window covers the tile and whose core band may reach
-        // it: region I on every row except the band's pairs outside region
-        // I, which are queued.
-        auto core_line = [&](const REC& r) {
+        // it: region I on every row except the band's pairs outside region I.
+        auto core_line = [&](const unsigned char* r) {
             if (MIXED) {
-                const float4* q = reinterpret_cast<const float4*>(&r);
+                const float4* q = reinterpret_cast<const float4*>(r);
                 const float4 v0 = q[0], v1 = q[1], v2 = q[2];
                 const float clo = v2.z, chi = v2.w;
                 const bool whole = v0.z < 0.0f;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     const float r0 = float(t0 + 32 * p), r1 = r0 + 31.0f;
-                    const float xs = whole ? float((r.nu - F[jj[p] < t1 ? jj[p] : tl]) / r.nu) * a.kx[w.c]
+                    const float xs = whole ? float((reinterpret_cast<const RecV32*>(r)->nu - F[jj[p] < t1 ? jj[p] : tl]) / reinterpret_cast<const RecV32*>(r)->nu) * a.kx[w.c]
                                            : fmaf(v0.x - jf[p], v0.z, v0.y);
                     const float u = fmaf(xs, xs, v0.w);
                     const float num = fmaf(u, v1.y, v1.y);
@@ -1363,11 +1373,11 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     accf[p] += keep ? num * rr : 0.0f;
                 }
             } else {
-                const double2* q = reinterpret_cast<const double2*>(&r);
-                const double2 v0 = q[0], v1 = q[1], v2 = q[2], v3 = q[3];
-                const int4 vi = reinterpret_cast<const int4*>(&r)[4];
+                const double2* q = reinterpret_cast<const double2*>(r);
+                const double2 v0 = q[0], v1 = q[1], v2 = q[2];
+                const int4 vi = reinterpret_cast<const int4*>(r)[3];
                 const int clo = vi.z, chi = vi.w;
-                const double y = v2.y, pref = v3.x;
+                const double y = v2.y;
 #pragma unroll
                 for (int p = 0; p < P; ++p) {
                     const int r0 = t0 + 32 * p, r1 = r0 + 31;
@@ -1383,7 +1393,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                         const double u = fma(xs, xs, v1.x);
                         accd[p] = fma(fma(u, v2.x, v2.x), rcp_refined_f64(fma(u, u, v1.y)), accd[p]);
                     }
-                    push(exact, ax, y, pref, p);
                 }
             }
         };
@@ -1399,7 +1408,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                 long end;
                 const long b = gstart(g, end);
                 const long rem = end - b;
-                stage(buf + (g % kStages) * 32, recs + b, int(rem < 32 ? rem : 32), lane);
+                stage_rec<kRec, int(sizeof(REC))>(mine + (g % kStages) * 32 * kRec, recs + b, int(rem < 32 ? rem : 32),
+                                                  lane);
             }
             cp_async_commit();
         };
@@ -1409,7 +1419,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             issue(gi + kStages - 1);
             cp_async_wait<kStages - 1>();
             __syncwarp();
-            const REC* R = buf + (gi % kStages) * 32;
+            const unsigned char* R0 = mine + (gi % kStages) * 32 * kRec;
+            auto R = [&](int t) { return R0 + t * kRec; };
             long end;
             const long gb = gstart(gi, end);
             const long ge = end - gb < 32 ? end : gb + 32;
@@ -1422,24 +1433,22 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                 if (t == a1) t = b1;  // skip the first fast run
                 if (t == c1) t = d1;  // skip the second fast run
                 if (t >= e1) break;
-                if (t >= b1 && t < c1) core_line(R[t]);
-                else partial_line(R[t]);
-                if constexpr (!MIXED)
-                    while (qn >= 32) qn = core_queue_flush<P, MIXED>(cq, qn, 32, lane);
+                if (t >= b1 && t < c1) core_line(R(t));
+                else partial_line(R(t));
             }
             {
                 int t = a1;
                 for (; t + 1 < b1; t += 2) {
-                    fast_line(R[t]);
-                    fast_line(R[t + 1]);
+                    fast_line(R(t));
+                    fast_line(R(t + 1));
                 }
-                if (t < b1) fast_line(R[t]);
+                if (t < b1) fast_line(R(t));
                 t = c1;
                 for (; t + 1 < d1; t += 2) {
-                    fast_line(R[t]);
-                    fast_line(R[t + 1]);
+                    fast_line(R(t));
+                    fast_line(R(t + 1));
                 }
-                if (t < d1) fast_line(R[t]);
+                if (t < d1) fast_line(R(t));
             }
             if (MIXED) {
                 // compensated (Kahan) fold of this group's FP32 partials
@@ -1457,15 +1466,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
         }
         cp_async_wait<0>();
         __syncwarp();
-        if constexpr (!MIXED) {
-            while (qn > 0) qn = core_queue_flush<P, MIXED>(cq, qn, qn < 32 ? qn : 32, lane);
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                accd[p] += double(cq.corr[p][lane]);
-                cq.corr[p][lane] = T(0);
-            }
-            __syncwarp();
-        }
         double v[P];
 #pragma unroll
         for (int p = 0; p < P; ++p) v[p] = MIXED ? double(sumf[p]) - double(cmpf[p]) : accd[p];
@@ -1477,6 +1477,32 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             for (int p = 0; p < P; ++p) f[p] = F[jj[p] < t1 ? jj[p] : tl];
             add_far_cells<P, PM>(a.chead + cell0, a.cmom + cell0 * PM, runs, a.splits, w.s,
                                  MIXED ? kCellBitsMixed : kCellBits64, F[t0], F[tl], f, v);
+        }
+        if constexpr (!MIXED) {
+            // W4 regions II-IV
+            double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine);
+#pragma unroll 1
+            for (int p = 0; p < P; ++p) {
+                const int r0 = t0 + 32 * p, r1 = min(r0 + 32, t1) - 1;
+                if (r0 > r1) break;
+                const long E0 = warp_lower_bound(La, Lb, lane, [&](long i) { return mi[i] >= r0 - kc; });
+                const long E1 = warp_lower_bound(E0, Lb, lane, [&](long i) { return mi[i] > r1 + kc; });
+                const double add =
+                    core_row_f64(T, F, E0, E1, r0, a.splits, w.s, lane,
+                                 [&](long i, double& nu, double& g, double& y, double& pref, int& jlo, int& jhi) {
+                                     const RecV64& r = recs[i];
+                                     const int4 iv = *reinterpret_cast<const int4*>(&r.lo);
+                                     nu = r.nu;
+                                     g = r.g;
+                                     y = r.y;
+                                     pref = r.pref;
+                                     jlo = max(max(iv.x, iv.z), r0);
+                                     jhi = min(min(iv.y - 1, iv.w), r1);
+                                 });
+#pragma unroll
+                for (int q = 0; q < P; ++q)
+                    if (q == p) v[q] += add;
+            }
         }
 #pragma unroll
         for (int p = 0; p < P; ++p)
@@ -1492,33 +1518,15 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
 // per condition.
 template <int C, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
-    using Q = WarpCoreQueue<C, false>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    LineSh64* lsb = reinterpret_cast<LineSh64*>(smem_raw) + warp * 64;
-    CondRec64* crb = reinterpret_cast<CondRec64*>(smem_raw + size_t(WARPS) * 64 * sizeof(LineSh64)) + warp * 64 * C;
-    Q& cq = reinterpret_cast<Q*>(smem_raw + size_t(WARPS) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64)))[warp];
+    // two stages of 32 lines; the core pass's table takes the same space
+    static_assert(64 * (sizeof(LineSh64) + 2 * sizeof(CondRec64)) >= kCoreTable64, "the table fits the stages");
+    unsigned char* const mine = smem_raw + size_t(warp) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64));
+    LineSh64* lsb = reinterpret_cast<LineSh64*>(mine);
+    CondRec64* crb = reinterpret_cast<CondRec64*>(mine + 64 * sizeof(LineSh64));
     const double* F = a.G.freq;
-    const unsigned lt_mask = (1u << lane) - 1u;
-
-#pragma unroll
-    for (int c = 0; c < C; ++c) cq.corr[c][lane] = 0.0;
-    int qn = 0;
-    auto push = [&](bool need, double x, double y, double pref, int c) {
-        const unsigned b = __ballot_sync(0xffffffffu, need);
-        if (b == 0u) return;
-        if (need) {
-            CoreEntry<double> e;
-            e.x = x;
-            e.y = y;
-            e.pref = pref;
-            e.dest = lane | (c << 5);
-            cq.q[qn + __popc(b & lt_mask)] = e;
-        }
-        qn += __popc(b);
-        __syncwarp();
-    };
 
     for (;;) {
         int item = 0;
@@ -1583,12 +1591,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             // x and y are bit-identical to the reference's, so |x| + y < 15
             // is the reference's region choice.
             const bool special = in && band && sx < 15.0;
-            if (!__any_sync(0xffffffffu, special)) {
-                region1(xs, r, in ? 1.0 : 0.0, c);
-                return;
-            }
             region1(xs, r, (in && !special) ? 1.0 : 0.0, c);
-            push(special, ax, r.y, r.pref, c);
         };
 
         // this item's groups of 32 lines
@@ -1654,7 +1657,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
                     const bool in = full || (jj >= s.lo && jj < s.hi && jj < t1);
                     const double mask = in ? 1.0 : 0.0;
                     const int mline = mi[gb + t];
-                    bool any_core = false;
 #pragma unroll
                     for (int c = 0; c < C; ++c) {
                         const CondRec64& r = SC[t * C + c];
@@ -1667,11 +1669,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
                             region1(offset(s, r), r, mask, c);
                         } else {
                             core_cond(s, r, mline, in, c);
-                            any_core = true;
                         }
                     }
-                    if (any_core)
-                        while (qn >= 32) qn = core_queue_flush<C, false>(cq, qn, 32, lane);
                 }
             };
             fast_run(a1, min(d1, b1));
@@ -1683,16 +1682,31 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             cand_run(b1, c1);
             __syncwarp();
         }
-        while (qn > 0) qn = core_queue_flush<C, false>(cq, qn, qn < 32 ? qn : 32, lane);
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-            accd[c] += cq.corr[c][lane];
-            cq.corr[c][lane] = 0.0;
-        }
-        __syncwarp();
         if (runs.fa < runs.fb || runs.fc < runs.fd)
             add_far_cells_mc<C, kCellTerms64>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs, a.splits,
                                               split, kCellBits64, F[t0], F[tl], fj, accd);
+        // W4 regions II-IV
+        double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine);
+#pragma unroll 1
+        for (int c = 0; c < C; ++c) {
+            const double add = core_row_f64(
+                T, F, E, Fc, t0, a.splits, split, lane,
+                [&](long i, double& nu, double& g, double& y, double& pref, int& jlo, int& jhi) {
+                    const CondRec64& r = crec[i * C + c];
+                    if (r.core == -1) return;
+                    const LineSh64 ls = lsh[i];
+                    const int aa = r.core & 0xffff, bb = (r.core >> 16) & 0xffff, m = mi[i];
+                    nu = ls.nu;
+                    g = r.g;
+                    y = r.y;
+                    pref = r.pref;
+                    jlo = max(aa == 0x7fff ? t0 : max(m - aa, t0), ls.lo);
+                    jhi = min(bb == 0x7fff ? tl : min(m + bb, tl), ls.hi - 1);
+                });
+#pragma unroll
+            for (int q = 0; q < C; ++q)
+                if (q == c) accd[q] += add;
+        }
         if (jj < t1) {
 #pragma unroll
             for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, accd[c]);
@@ -2500,8 +2514,7 @@ int blocks_per_sm(K kernel, int threads, size_t smem) {
 
 template <int P, int WARPS, bool MIXED>
 cudaError_t run_voigt(int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    using REC = typename std::conditional<MIXED, RecV32, RecV64>::type;
-    const size_t smem = size_t(WARPS) * (32 * kStages * sizeof(REC) + (MIXED ? 0 : sizeof(WarpCoreQueue<P, MIXED>)));
+    const size_t smem = size_t(WARPS) * voigt_warp_smem(MIXED);
     if (smem > 48 * 1024) {
         if (cudaFuncSetAttribute(k_steptwo_voigt<P, WARPS, MIXED>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
@@ -2517,8 +2530,7 @@ cudaError_t run_voigt(int blocks, const StepArgs& a, cudaStream_t st, int* occ) 
 
 template <int C, int WARPS>
 cudaError_t run_voigt_mc(int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    const size_t smem = size_t(WARPS) * (64 * (sizeof(LineSh64) + C * sizeof(CondRec64)) +
-                                         sizeof(WarpCoreQueue<C, false>));
+    const size_t smem = size_t(WARPS) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64));
     if (smem > 48 * 1024) {
         if (cudaFuncSetAttribute(k_steptwo_voigt_mc<C, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(smem)) != cudaSuccess)

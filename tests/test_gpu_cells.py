@@ -55,7 +55,7 @@ def reference(convention, fr, lines, cond, df, p):
 
 
 @pytest.mark.parametrize("convention", [capi.CONV_GPU, capi.CONV_CPU])
-@pytest.mark.parametrize("n, df, make", [(4096, 0.05, "even"), (4097, 0.013, "even"), (5999, 0.11, "uneven"),
+@pytest.mark.parametrize("n, df, make", [(4096, 0.01, "even"), (16385, 0.05, "even"), (30001, 0.11, "uneven"),
                                          (9001, 0.02, "uneven")])
 def test_cells_one_condition(engine, cuda, convention, n, df, make):
     lines = uneven(n, 31) if make == "uneven" else synth.random_lines(n, 1000.0, 1100.0, 2500.0, 1e-6, 1e2, seed=30)
@@ -78,7 +78,7 @@ def test_cells_one_condition(engine, cuda, convention, n, df, make):
 
 
 @pytest.mark.parametrize("C", [2, 4, 8])
-@pytest.mark.parametrize("n, df", [(4099, 0.1), (8000, 0.021)])
+@pytest.mark.parametrize("n, df", [(8003, 0.1), (6000, 0.021)])
 def test_cells_groups_of_conditions(engine, cuda, C, n, df):
     lines = uneven(n, 33)
     grid = synth.Grid(985.0, 1117.0, int(132.0 / df))
@@ -97,7 +97,7 @@ def test_cells_groups_of_conditions(engine, cuda, C, n, df):
 
 
 def test_cells_chunk_inside_the_grid(engine, cuda):
-    lines = uneven(6000, 35)
+    lines = uneven(12000, 35)
     grid = synth.Grid(985.0, 1117.0, 6601)
     fr = grid.freq()
     cond = dict(temperature=900.0, partition=synth.partition_poly(900.0), mean_mass=17.03, pressure=1.0,

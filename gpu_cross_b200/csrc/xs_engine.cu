@@ -205,6 +205,17 @@ int cell_shift(const xs_options& o, const xs_condition* conds, int ncond, long n
     return sh;
 }
 
+// Whether a 32-point row holds more lines than 4 cells: three times its width
+// (its own lines and those whose windows end in it) then outweighs the 6 or so
+// cells on both sides that are too near for their series.
+bool row_is_wide(const xs_options& o, const xs_condition* conds, int ncond, long n, const xs_grid& grid) {
+    double cutmax = 0.0;
+    for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(o, conds[c]).cut);
+    const double per_point = double(n) * o.dfreq / (double(grid.points) * o.dfreq + 2.0 * cutmax);
+    const int shift = cell_shift(o, conds, ncond, n, grid, 8);
+    return shift > 0 && 32.0 * per_point > 4.0 * double(1L << shift);
+}
+
 // A-priori relative error bound of a result against the FP64 path of the
 // same convention (see xs_engine_accuracy).
 double error_bound(int kind, bool mixed) {
@@ -568,6 +579,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
     }
     const int CG = C > 1 ? C : 0;
+    // Rows of 8 points and 4 lines at a time where a 32-point row is wider than
+    // what has to be taken line by line beside it (about 6 cells).
+    const int LS = CG && !(ov && ov->scratch) && row_is_wide(*opt, conds, ncond, n, *grid) ? 4 : 1;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
         return fail(XS_ERR_INVALID, "line_splits must be 0 (automatic) .. 64");
 
@@ -577,7 +591,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Scratch layout for one group of conditions.
     const int group = ncond < kMaxCond ? ncond : kMaxCond;
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
-    int occ = CG ? steptwo_mc_blocks_per_sm(mixed, CG, W)
+    int occ = CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, LS)
                  : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
     if (occ < 1) {
         // e.g. 8 FP64 conditions per warp with 8 warps: more shared memory
@@ -594,7 +608,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // different warps -- enough for about 16 items per resident warp, at
     // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
-    const int tile_pts = CG ? 32 : 32 * P;
+    const int tile_pts = CG ? 32 / LS : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
@@ -871,9 +885,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
         if (CG) {
             sa.lsh = pa.lsh;
+            sa.cyp = pa.cyp;
             for (int g = 0; g < nc / CG; ++g) sa.wslot[g] = pa.wslot[g];
             sa.group = CG;
-            sa.tiles_per_cond = (grid->points + 31) / 32;
+            sa.tiles_per_cond = tiles;
             sa.n_items = sa.tiles_per_cond * (nc / CG) * S;
         }
         CheckArgs ck;
@@ -907,7 +922,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
-        err = CG ? launch_steptwo_mc(mixed, CG, W, blocks, sa, st)
+        err = CG ? launch_steptwo_mc(mixed, CG, W, LS, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);
         if (err != cudaSuccess) return cuda_fail(err, "step two launch");
         if (blocks > 0 && sa.n_items > 0) ++launched;
@@ -919,7 +934,6 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             ca.civ = pa.civ;
             ca.cyp = pa.cyp;
             ca.lsh = static_cast<const LineShX*>(pa.lsh);
-            ca.rec = pa.rec;
             ca.mi = pa.mi;
             ca.kc = pa.kc;
             ca.freq = G.freq;

@@ -124,23 +124,6 @@ struct __align__(16) LineShX {
 static_assert(sizeof(LineShX) == 32, "LineShX layout");
 constexpr int kLineWhole = 1;
 constexpr int kLineWide = 2;
-// Region-I constants of a line for the C conditions of its group, each
-// array in condition order: conditions 2k and 2k+1 are one packed FP32x2
-// operand, conditions 4k..4k+3 one 16-byte load.  This is all step two
-// stages per (line, group) besides LineShX: 12 bytes per condition (C = 2 is
-// padded to 32 bytes, a whole number of 16-byte copies).
-template <int C>
-struct __align__(16) LineR1 {
-    float Cy[C], D2[C], Pc[C];
-};
-template <>
-struct __align__(16) LineR1<2> {
-    float Cy[2], D2[2], Pc[2], pad[2];
-};
-static_assert(sizeof(LineR1<8>) == 96 && sizeof(LineR1<4>) == 48 && sizeof(LineR1<2>) == 32,
-              "LineR1 layout");
-// Bytes per (line, group) of the mixed multi-condition region-I records.
-constexpr size_t line_r1_bytes(int C) { return C == 8 ? 96 : (C == 4 ? 48 : 32); }
 // Per (line, condition) of the mixed multi-condition layout, for the core
 // pass: the grid indices of W4 regions II-IV [lo15, hi15] and III-IV
 // [lo55, hi55] (empty: lo > hi) inside the line's window.  Step two adds
@@ -289,6 +272,7 @@ struct StepArgs {
     size_t out_stride;  // elements between conditions
     GridDev G;
     const void* lsh;    // multi-condition layout (LineShX mixed, LineSh64 FP64)
+    const float2* cyp;  // mixed multi-condition: (y, pref), condition-major
     int wslot[kMaxCond];  // window slot of each group (PrepArgs::wslot)
     int group;          // conditions per group (multi-condition kernel)
     int tiles_per_cond;
@@ -360,7 +344,6 @@ struct CoreArgs {
     const CoreIv* civ;
     const float2* cyp;
     const LineShX* lsh;
-    const void* rec;    // LineR1<group> per (line, group): Cy of the condition
     const int* mi;
     const int* kc;
     const double* freq;
@@ -414,9 +397,10 @@ cudaError_t launch_check_snapshot(const CheckArgs& a, cudaStream_t stream);
 // (launched after the call's last kernel).
 cudaError_t launch_check_rows(const CheckArgs& a, cudaStream_t stream);
 
-// Multi-condition step two (Voigt): C conditions per warp, 32 points per warp.
-cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int blocks, const StepArgs& a,
+// Multi-condition step two (Voigt): C conditions per warp.
+// LS lane subsets share a row of 32 / LS points (LS = 1 or 4).
+cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
                               cudaStream_t stream);
-int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps);
+int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int LS);
 
 }  // namespace xs

@@ -495,9 +495,11 @@ __global__ void __launch_bounds__(256) k_prep(PrepArgs a) {
 // condition-free offsets (LineShX) -- is written once per run of such
 // groups; the conditions follow in order, their loop not unrolled, which
 // keeps the code small.  Each value takes the FP64 path's operations in the
-// same order (the W4 region intervals are the FP64 region choice).  A
-// line's LineR1 of a group is written by one thread within a short time, so
-// whole sectors reach memory.  The core-candidate reach (kc) covers the
+// same order (the W4 region intervals are the FP64 region choice).  Every
+// store but the window data's is coalesced (conditions outermost); step two
+// forms the region-I constants from (y, pref) itself, which took 12 bytes per
+// line and condition and the L1's store bandwidth here (4-byte stores 96 bytes
+// apart).  The core-candidate reach (kc) covers the
 // pairs where x^2 + y^2 < kNearR2, at least one grid point beyond: there the
 // region-I rational may exceed W4 by far, and step two tests u on the lines
 // of that reach.
@@ -599,11 +601,6 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
                 }
             }
         }
-        const size_t gi = size_t(cg) * size_t(a.L.n) + size_t(live ? i : 0);
-        LineR1<C>& lr = reinterpret_cast<LineR1<C>*>(a.rec)[gi];
-        if constexpr (C == 2) {
-            if (live) lr.pad[0] = lr.pad[1] = 0.0f;
-        }
 #pragma unroll 1
         for (int k = 0; k < C; ++k) {
             const int c = cg * C + k;
@@ -656,9 +653,6 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
                 const size_t ci = size_t(c) * size_t(a.L.n) + size_t(i);
                 a.civ[ci] = iv;
                 a.cyp[ci] = make_float2(float(y), float(pref));
-                lr.Cy[k] = float(y2 - 0.5);
-                lr.D2[k] = float(2.0 * y2);
-                lr.Pc[k] = float(Pc);
             }
             kcl = __reduce_max_sync(0xffffffffu, kcl);
             rch = __reduce_max_sync(0xffffffffu, rch);
@@ -913,14 +907,18 @@ __device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M
     run(r.fc, r.fd);
 }
 
-// The same for one point and the C conditions of a group.
-template <int C, int PM>
+// The same for one point and the C conditions of a group; the warp's LS lane
+// subsets (sub = this lane's) take every LS-th cell.
+template <int C, int PM, int LS>
 __device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
-                                                 float bits, double ftlo, double fthi, double f, double (&v)[C]) {
+                                                 int sub, float bits, double ftlo, double fthi, double f,
+                                                 double (&v)[C]) {
     auto run = [&](int c0, int c1) {
-        for (int c = c0 + s; c < c1; c += S) {
+        for (int b = c0 + s * LS; b < c1; b += S * LS) {
+            const int c = min(b + sub, c1 - 1);
             const CellHead h = H[c];
-            const int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
+            int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
+            if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
             const double2* m = reinterpret_cast<const double2*>(M + size_t(c) * PM * C);
             const double t = double(h.q) * rcp_newton2_f64(f - h.c0);
             double a[C];
@@ -934,13 +932,21 @@ __device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double
                     a[q + 1] = fma(a[q + 1], t, mk.y);
                 }
             }
-            const double t2 = t * t;
+            const double t2 = b + sub < c1 ? t * t : 0.0;
 #pragma unroll
             for (int q = 0; q < C; ++q) v[q] = fma(a[q], t2, v[q]);
         }
     };
     run(r.fa, r.fb);
     run(r.fc, r.fd);
+}
+
+// Sum of v over the warp's LS lane subsets, to every lane.
+template <int LS>
+__device__ __forceinline__ double sum_subsets(double v) {
+#pragma unroll
+    for (int o = 32 / LS; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // ---------------------------------------------------------------------------
@@ -1511,12 +1517,14 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
 }
 
 // Multi-condition step two, FP64: a work item is (group of C conditions that
-// share one window, row of 32 grid points); each lane owns one grid point and
-// C accumulators.  The line runs are found as in k_steptwo_voigt (windows and
+// share one window, row of 32 / LS grid points); each lane owns one grid point,
+// every LS-th line of the row's and C accumulators (LS = 4: 8-point rows for
+// coarse grids over dense lists, where a 32-point row is much wider than the
+// zone that has to be taken line by line).  The line runs are found as in k_steptwo_voigt (windows and
 // grid indices are shared by the group; the core run uses the group's widest
 // core), and every line loads its shared record once and one small record
 // per condition.
-template <int C, int WARPS>
+template <int C, int WARPS, int LS>
 __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
@@ -1527,6 +1535,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
     LineSh64* lsb = reinterpret_cast<LineSh64*>(mine);
     CondRec64* crb = reinterpret_cast<CondRec64*>(mine + 64 * sizeof(LineSh64));
     const double* F = a.G.freq;
+    constexpr int PT = 32 / LS;  // points of a row
+    const int sub = lane / PT;
 
     for (;;) {
         int item = 0;
@@ -1537,9 +1547,9 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
         const int cg = item / per_cond;
         const int tile = (item - cg * per_cond) / a.splits;
         const int split = item - cg * per_cond - tile * a.splits;
-        const int t0 = a.G.start + tile * 32;
+        const int t0 = a.G.start + tile * PT;
         const int end = a.G.start + a.G.points;
-        const int t1 = t0 + 32 < end ? t0 + 32 : end;
+        const int t1 = t0 + PT < end ? t0 + PT : end;
         const int tl = t1 - 1;
         const size_t gbase = size_t(cg) * size_t(a.n);
         const int* whi = a.whi + gbase;
@@ -1564,7 +1574,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
         const LineRuns runs =
             line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
 
-        const int jj = t0 + lane;
+        const int jj = t0 + lane % PT;
         const double fj = F[jj < t1 ? jj : tl];
         double accd[C];
 #pragma unroll
@@ -1625,36 +1635,30 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             const long gb = gstart(gi, end);
             const long ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](long v) { return int((v < gb ? gb : (v > ge ? ge : v)) - gb); };
-            const int a0 = lo_of(La), a1 = lo_of(fs), b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe),
-                      e1 = lo_of(Lb);
-            // Runs of this group: [a1, d1) cover the row (full), the rest
-            // are partial; [b1, c1) are the core candidates.
-            // Full lines away from every core: region I with no test.
-            auto fast_run = [&](int x, int y) {
-                for (int t = x; t < y; ++t) {
+            const int b1 = lo_of(E), c1 = lo_of(Fc);  // the core candidates
+            // Lines [x, y) that are not core candidates: region I, the window
+            // as a lane mask (one loop for the lines before and after the
+            // candidates, full and partial ones alike); with LS > 1 a lane
+            // past its last line takes the run's last one with weight 0.
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int x = h ? c1 : 0, y = h ? int(ge - gb) : b1;
+                for (int b = x; b < y; b += LS) {
+                    const int t = min(b + sub, y - 1);
                     const LineSh64 s = SL[t];
-#pragma unroll
-                    for (int c = 0; c < C; ++c) region1(offset(s, SC[t * C + c]), SC[t * C + c], 1.0, c);
-                }
-            };
-            // Partial lines away from every core: region I, the window as a
-            // lane mask.
-            auto masked_run = [&](int x, int y) {
-                for (int t = x; t < y; ++t) {
-                    const LineSh64 s = SL[t];
-                    const double mask = (jj >= s.lo && jj < s.hi && jj < t1) ? 1.0 : 0.0;
+                    const double mask = (b + sub < y && jj >= s.lo && jj < s.hi) ? 1.0 : 0.0;
 #pragma unroll
                     for (int c = 0; c < C; ++c) region1(offset(s, SC[t * C + c]), SC[t * C + c], mask, c);
                 }
-            };
+            }
             // Core candidates.  Per condition: when its core band misses the
             // row, region I with the window as a lane mask; otherwise the
             // lane-by-lane core path.
             auto cand_run = [&](int x, int y) {
-                for (int t = x; t < y; ++t) {
+                for (int b = x; b < y; b += LS) {
+                    const int t = min(b + sub, y - 1);
                     const LineSh64 s = SL[t];
-                    const bool full = (t >= a1 && t < d1);
-                    const bool in = full || (jj >= s.lo && jj < s.hi && jj < t1);
+                    const bool in = b + sub < y && jj >= s.lo && jj < s.hi;
                     const double mask = in ? 1.0 : 0.0;
                     const int mline = mi[gb + t];
 #pragma unroll
@@ -1673,19 +1677,15 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
                     }
                 }
             };
-            fast_run(a1, min(d1, b1));
-            fast_run(max(a1, c1), d1);
-            masked_run(a0, min(a1, b1));
-            masked_run(max(a0, c1), a1);
-            masked_run(d1, min(e1, b1));
-            masked_run(max(d1, c1), e1);
             cand_run(b1, c1);
             __syncwarp();
         }
         if (runs.fa < runs.fb || runs.fc < runs.fd)
-            add_far_cells_mc<C, kCellTerms64>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs, a.splits,
-                                              split, kCellBits64, F[t0], F[tl], fj, accd);
-        // W4 regions II-IV
+            add_far_cells_mc<C, kCellTerms64, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs,
+                                                  a.splits, split, sub, kCellBits64, F[t0], F[tl], fj, accd);
+#pragma unroll
+        for (int c = 0; c < C; ++c) accd[c] = sum_subsets<LS>(accd[c]);
+        // W4 regions II-IV (point p of the row in lane p)
         double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine);
 #pragma unroll 1
         for (int c = 0; c < C; ++c) {
@@ -1707,7 +1707,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             for (int q = 0; q < C; ++q)
                 if (q == c) accd[q] += add;
         }
-        if (jj < t1) {
+        if (sub == 0 && jj < t1) {
 #pragma unroll
             for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, accd[c]);
         }
@@ -1727,6 +1727,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
 // of the window except, on core candidates, where u < 1; k_core_mcx adds W4
 // less the rational (where it was added) inside the W4 region intervals
 // (|x| + y < 15, from step one).
+//
+// A row is 32 / LS points; with LS = 4 each lane owns one of 8 points and takes
+// every fourth line, for coarse grids over dense lists: 40 conditions, 1e7
+// lines, 0.1 cm-1 grid -- a 32-point row has 6.4 cm-1 of lines whose windows end
+// in it and 3.2 of its own width beside the 2 near it, an 8-point one 1.6 and
+// 0.8.
 // ---------------------------------------------------------------------------
 // Resident blocks per SM the mixed multi-condition kernel asks the compiler
 // to fit: 24 warps per SM (about 80 registers a thread); 28 at 8 conditions
@@ -1736,10 +1742,28 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
 // the block size.
 template <int C, int WARPS>
 constexpr int voigt_mcx_min_blocks() {
-    return (C == 8 && WARPS == 8) ? 2 : (C == 8 && WARPS == 4) ? 7 : 24 / WARPS;
+    return (C == 8 && WARPS == 8) ? 2 : (C == 8 && WARPS == 4) ? 6 : 24 / WARPS;
 }
 
-template <int C, int WARPS>
+// Region-I constants of a line for the C conditions of its group, in condition
+// order: conditions 2k and 2k+1 are one packed FP32x2 operand, conditions
+// 4k..4k+3 one 16-byte load.  Formed in shared memory from the (y, pref) pairs
+// of step one when a group of lines has arrived.
+template <int C>
+struct __align__(C == 2 ? 8 : 16) LineR1 {
+    float Cy[C], D2[C], Pc[C];
+};
+// (the core pass repeats step two's choice on u = X^2 k^2 + Cy: one definition)
+__device__ __forceinline__ float region1_cy(float y) { return fmaf(y, y, -0.5f); }
+
+// Shared memory of one warp: two stages of 32 lines' offsets and flags (16 B),
+// windows (8 B) and (y, pref) (8 B per condition), and 32 lines' constants.
+template <int C>
+constexpr size_t mcx_warp_smem() {
+    return 64 * (sizeof(float4) + sizeof(int2) + C * sizeof(float2)) + 32 * sizeof(LineR1<C>);
+}
+
+template <int C, int WARPS, int LS>
 __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>()))
     k_steptwo_voigt_mcx(StepArgs a) {
     static_assert(C % 2 == 0, "conditions come in pairs");
@@ -1748,12 +1772,16 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     using R1 = LineR1<C>;
-    // staged per line: the offsets and flags of LineShX (16 B), its window
-    // (8 B) and the group's region-I records; a whole line's FP64 centre is
+    // staged per line: the offsets and flags of LineShX, its window and the
+    // conditions' (y, pref), [condition][line]; a whole line's FP64 centre is
     // read from memory when needed
-    float4* lsb = reinterpret_cast<float4*>(smem_raw) + warp * 64;
-    int2* lhb = reinterpret_cast<int2*>(smem_raw + size_t(WARPS) * 64 * sizeof(float4)) + warp * 64;
-    R1* rb = reinterpret_cast<R1*>(smem_raw + size_t(WARPS) * 64 * (sizeof(float4) + sizeof(int2))) + warp * 64;
+    unsigned char* const mine = smem_raw + size_t(warp) * mcx_warp_smem<C>();
+    float4* lsb = reinterpret_cast<float4*>(mine);
+    R1* SR = reinterpret_cast<R1*>(mine + 64 * sizeof(float4));
+    float2* ypb = reinterpret_cast<float2*>(mine + 64 * sizeof(float4) + 32 * sizeof(R1));
+    int2* lhb = reinterpret_cast<int2*>(ypb + 64 * C);
+    constexpr int PT = 32 / LS;  // points of a row
+    const int sub = lane / PT;
 
     for (;;) {
         int item = 0;
@@ -1764,11 +1792,10 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
         const int cg = item / per_cond;
         const int tile = (item - cg * per_cond) / a.splits;
         const int split = item - cg * per_cond - tile * a.splits;
-        const int t0 = a.G.start + tile * 32;
+        const int t0 = a.G.start + tile * PT;
         const int end = a.G.start + a.G.points;
-        const int t1 = t0 + 32 < end ? t0 + 32 : end;
+        const int t1 = t0 + PT < end ? t0 + PT : end;
         const int tl = t1 - 1;
-        const size_t gbase = size_t(cg) * size_t(a.n);
         const size_t wbase = size_t(a.wslot[cg]) * size_t(a.n);  // the group's window data
         const int* whi = a.whi + wbase;
         const int* wlo = a.wlo + wbase;
@@ -1791,14 +1818,14 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             Fc = int(warp_lower_bound(E, Lb, lane, [&](long i) { return mi[i] > tl + (kc - 1); }));
         }
         const LineShX* lsh = reinterpret_cast<const LineShX*>(a.lsh) + wbase;
-        const R1* r1 = reinterpret_cast<const R1*>(a.rec) + gbase;
+        const float2* yp = a.cyp + size_t(cg) * C * size_t(a.n);
 
         const double* F = a.G.freq;
         const size_t cell0 = size_t(cg) * size_t(a.ncell);
         const LineRuns runs =
             line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
 
-        const int jj = t0 + lane;
+        const int jj = t0 + lane % PT;
         const float jf = float(jj);
         float2 k2[NP];
         float2 acc[NP], sum[NP], cmp[NP];
@@ -1837,14 +1864,13 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
         };
         const std::integral_constant<int, 0> plain;
         const std::integral_constant<int, 2> guarded_near;
-        // Region I of two pairs of conditions (A, B) with one reciprocal per
-        // two line-evals: lane h of A and lane h of B share 1 / (dA dB), so
-        // 1/dA = dB / (dA dB) and 1/dB = dA / (dA dB).  For narrow lines the
-        // product itself stays in range (kPairUMax); for wide ones both
-        // factors are scaled by kPairTau first, 1/dA = (tau dB) / (tau dA dB).
+        // Region I of two pairs of conditions (A, B) of a wide line with one
+        // reciprocal per two line-evals: lane h of A and lane h of B share
+        // 1 / (dA dB), so 1/dA = dB / (dA dB) and 1/dB = dA / (dA dB), both
+        // factors scaled by kPairTau first: 1/dA = (tau dB) / (tau dA dB).
         // pA = 2q, pB = 2q + 1: conditions 4q..4q+3, one 16-byte load for each
         // of Cy, D2 and Pc.  Pairs where `keep` is false add exactly zero.
-        auto region1_ab = [&](auto narrow, float X2, const R1& r, int pA, int pB, bool keep) {
+        auto region1_ab = [&](float X2, const R1& r, int pA, int pB, bool keep) {
             const float4 cy = *reinterpret_cast<const float4*>(&r.Cy[2 * pA]);
             const float4 d2 = *reinterpret_cast<const float4*>(&r.D2[2 * pA]);
             const float4 pc = *reinterpret_cast<const float4*>(&r.Pc[2 * pA]);
@@ -1854,22 +1880,13 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             const float2 dB = __ffma2_rn(uB, uB, f2(d2.z, d2.w));
             const float2 nA = __ffma2_rn(uA, f2(pc.x, pc.y), f2(pc.x, pc.y));
             const float2 nB = __ffma2_rn(uB, f2(pc.z, pc.w), f2(pc.z, pc.w));
-            if constexpr (decltype(narrow)::value) {
-                const float2 q = __fmul2_rn(dA, dB);
-                const float2 rq = keep ? f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)) : f2(0.0f, 0.0f);
-                acc[pA] = __ffma2_rn(nA, __fmul2_rn(dB, rq), acc[pA]);
-                acc[pB] = __ffma2_rn(nB, __fmul2_rn(dA, rq), acc[pB]);
-            } else {
-                const float2 aA = __fmul2_rn(dA, f2s(kPairTau));
-                const float2 bB = __fmul2_rn(dB, f2s(kPairTau));
-                const float2 q = __fmul2_rn(aA, dB);
-                const float2 rq = keep ? f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)) : f2(0.0f, 0.0f);
-                acc[pA] = __ffma2_rn(nA, __fmul2_rn(bB, rq), acc[pA]);
-                acc[pB] = __ffma2_rn(nB, __fmul2_rn(aA, rq), acc[pB]);
-            }
+            const float2 aA = __fmul2_rn(dA, f2s(kPairTau));
+            const float2 bB = __fmul2_rn(dB, f2s(kPairTau));
+            const float2 q = __fmul2_rn(aA, dB);
+            const float2 rq = keep ? f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)) : f2(0.0f, 0.0f);
+            acc[pA] = __ffma2_rn(nA, __fmul2_rn(bB, rq), acc[pA]);
+            acc[pB] = __ffma2_rn(nB, __fmul2_rn(aA, rq), acc[pB]);
         };
-        const std::true_type narrow;
-        const std::false_type scaled;
         // region1_ab for a narrow core-candidate line: a condition's pair is
         // kept where the point takes the line (`in`) and u >= 1 (the core
         // pass takes u < 1); a pair that is not kept enters the shared
@@ -1908,8 +1925,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             if (lane < cnt) {
                 cp_async16(lsb + bufi * 32 + lane, lsh + b + lane);
                 cp_async8(lhb + bufi * 32 + lane, &lsh[b + lane].lo);
+#pragma unroll
+                for (int c = 0; c < C; ++c) cp_async8(ypb + (bufi * C + c) * 32 + lane, yp + size_t(c) * size_t(a.n) + b + lane);
             }
-            stage(rb + bufi * 32, r1 + b, cnt, lane);
         };
         if (ngroups > 0) {
             int end;
@@ -1931,30 +1949,36 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             __syncwarp();
             const float4* SL = lsb + (gi & 1) * 32;  // m, df/nu, r/nu, flags
             const int2* SW = lhb + (gi & 1) * 32;    // window [lo, hi)
-            const R1* SR = rb + (gi & 1) * 32;
+            {
+                // this lane's line's constants (lanes past the group's end
+                // convert what an earlier group left: never used)
+                R1& r = SR[lane];
+#pragma unroll
+                for (int c = 0; c < C; c += 2) {
+                    const float2 v0 = ypb[((gi & 1) * C + c) * 32 + lane], v1 = ypb[((gi & 1) * C + c + 1) * 32 + lane];
+                    *reinterpret_cast<float2*>(&r.Cy[c]) = f2(region1_cy(v0.x), region1_cy(v1.x));
+                    *reinterpret_cast<float2*>(&r.D2[c]) = f2(2.0f * v0.x * v0.x, 2.0f * v1.x * v1.x);
+                    *reinterpret_cast<float2*>(&r.Pc[c]) =
+                        f2(v0.y * float(kW4C) * v0.x, v1.y * float(kW4C) * v1.x);
+                }
+            }
+            __syncwarp();
             int end;
             const int gb = gstart(gi, end);
             const int ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](int v) { return (v < gb ? gb : (v > ge ? ge : v)) - gb; };
-            const int a0 = lo_of(La), a1 = lo_of(fs), b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe),
-                      e1 = lo_of(Lb);
+            const int b1 = lo_of(E), c1 = lo_of(Fc);  // the core candidates
             // One line's region I at this lane's point, conditions in pairs
             // of pairs (keep: the point takes the line).
-            auto line_region1 = [&](float X2, const R1& r, bool wide, bool keep) {
+            auto line_region1 = [&](float X2, const R1& r, bool keep) {
                 if constexpr (NP % 2 == 0) {
-                    if (!wide) {
 #pragma unroll
-                        for (int p = 0; p < NP; p += 2) region1_ab(narrow, X2, r, p, p + 1, keep);
-                    } else {
-#pragma unroll
-                        for (int p = 0; p < NP; p += 2) region1_ab(scaled, X2, r, p, p + 1, keep);
-                    }
+                    for (int p = 0; p < NP; p += 2) region1_ab(X2, r, p, p + 1, keep);
                 } else {
 #pragma unroll
                     for (int p = 0; p < NP; ++p) region1(plain, X2, r, p, keep, keep);
                 }
             };
-            // Full lines away from every core: region I with no test.
             // Two narrow lines A, B that are not core candidates, at once: per
             // condition one reciprocal for both lines, acc += (nA dB + nB dA)
             // / (dA dB) (u >= 1 on such lines, so dA, dB >= 1; narrow lines
@@ -2001,51 +2025,49 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                                   *reinterpret_cast<const float2*>(&rb.Pc[2 * p]), p, inA, inB);
                 }
             };
-            // Lines [x, y) that are not core candidates, two at a time; `full`:
-            // their windows cover the tile, else the window is a lane mask.
-            auto pair_run = [&](int x, int y, auto full) {
-                auto in_of = [&](int t) {
-                    if constexpr (decltype(full)::value) return true;
-                    else return jj >= SW[t].x && jj < SW[t].y && jj < t1;
-                };
-                int t = x;
-                for (; t + 1 < y; t += 2) {
-                    const float4 sA = SL[t];
-                    const float4 sB = SL[t + 1];
+            // Lines [x, y) that are not core candidates, two at a time, the
+            // window as a lane mask.  Lane subset `sub` takes lines x + sub,
+            // x + sub + LS, ...; a lane past the run's end takes its last line
+            // with `in` false.  One loop for the lines before and after the
+            // candidates (and for full and partial ones alike): the body is
+            // large, and six copies of it ran out of the instruction cache.
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int x = h ? c1 : 0, y = h ? ge - gb : b1;
+#pragma unroll 1
+                for (int b = x; b < y; b += 2 * LS) {
+                    const int tA = LS > 1 ? min(b + sub, y - 1) : b, tB = min(b + sub + LS, y - 1);
+                    const float4 sA = SL[tA];
+                    const float4 sB = SL[tB];
+                    const int2 wA = SW[tA], wB = SW[tB];
                     const float XA = fmaf(sA.x - jf, sA.y, sA.z);
                     const float XB = fmaf(sB.x - jf, sB.y, sB.z);
-                    const int fA = __float_as_int(sA.w), fB = __float_as_int(sB.w);
-                    const bool inA = in_of(t), inB = in_of(t + 1);
-                    if (!((fA | fB) & kLineWide)) {
-                        pair_region1(XA * XA, XB * XB, SR[t], SR[t + 1], inA, inB);
+                    const bool wide = ((__float_as_int(sA.w) | __float_as_int(sB.w)) & kLineWide) != 0;
+                    const bool inA = (LS == 1 || b + sub < y) && jj >= wA.x && jj < wA.y;
+                    const bool inB = b + sub + LS < y && jj >= wB.x && jj < wB.y;
+                    if (!(LS > 1 ? __any_sync(0xffffffffu, wide) : wide)) {
+                        pair_region1(XA * XA, XB * XB, SR[tA], SR[tB], inA, inB);
                     } else {
-                        line_region1(XA * XA, SR[t], (fA & kLineWide) != 0, inA);
-                        line_region1(XB * XB, SR[t + 1], (fB & kLineWide) != 0, inB);
+                        // (the scaled form serves narrow lines too)
+#pragma unroll 1
+                        for (int q = 0; q < 2; ++q)
+                            line_region1(q ? XB * XB : XA * XA, SR[q ? tB : tA], q ? inB : inA);
                     }
                 }
-                if (t < y) {
-                    const float4 s = SL[t];
-                    const float X = fmaf(s.x - jf, s.y, s.z);
-                    line_region1(X * X, SR[t], (__float_as_int(s.w) & kLineWide) != 0, in_of(t));
-                }
-            };
-            const std::true_type full_lines;
-            const std::false_type partial_lines;
-            // Full lines away from every core: region I with no test.
-            auto fast_run = [&](int x, int y) { pair_run(x, y, full_lines); };
-            // Partial lines away from every core: the window as a lane mask.
-            auto masked_run = [&](int x, int y) { pair_run(x, y, partial_lines); };
+            }
             // Core candidates: region I where u >= 1, per condition (the
             // core pass takes the pairs with u < 1, deciding on the same FP32
             // u).
             auto cand_run = [&](int x, int y) {
-                for (int t = x; t < y; ++t) {
+                for (int b = x; b < y; b += LS) {
+                    const int t = LS > 1 ? min(b + sub, y - 1) : b;
                     const float4 s = SL[t];
                     const int flags = __float_as_int(s.w);
-                    const bool full = (t >= a1 && t < d1);
-                    const bool in = full || (jj >= SW[t].x && jj < SW[t].y && jj < t1);
+                    const int2 win = SW[t];
+                    const bool in = (LS == 1 || b + sub < y) && jj >= win.x && jj < win.y;
                     if constexpr (NP % 2 == 0) {
-                        if (!(flags & (kLineWhole | kLineWide))) {
+                        const bool odd = (flags & (kLineWhole | kLineWide)) != 0;
+                        if (!(LS > 1 ? __any_sync(0xffffffffu, odd) : odd)) {
                             // narrow: the shared reciprocal
                             const float X = fmaf(s.x - jf, s.y, s.z);
 #pragma unroll
@@ -2075,12 +2097,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                     }
                 }
             };
-            fast_run(a1, min(d1, b1));
-            fast_run(max(a1, c1), d1);
-            masked_run(a0, min(a1, b1));
-            masked_run(max(a0, c1), a1);
-            masked_run(d1, min(e1, b1));
-            masked_run(max(d1, c1), e1);
             cand_run(b1, c1);
             // compensated (Kahan) fold of this group's FP32 partials
             auto kahan = [](float part, float& sm, float& cm) {
@@ -2089,11 +2105,14 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                 cm = (tk - sm) - yk;
                 sm = tk;
             };
+            // (LS groups are 32 lines of each lane)
+            if (LS == 1 || (gi & (LS - 1)) == LS - 1 || gi + 1 == ngroups) {
 #pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                kahan(acc[p].x, sum[p].x, cmp[p].x);
-                kahan(acc[p].y, sum[p].y, cmp[p].y);
-                acc[p] = f2(0.0f, 0.0f);
+                for (int p = 0; p < NP; ++p) {
+                    kahan(acc[p].x, sum[p].x, cmp[p].x);
+                    kahan(acc[p].y, sum[p].y, cmp[p].y);
+                    acc[p] = f2(0.0f, 0.0f);
+                }
             }
             __syncwarp();
         }
@@ -2104,10 +2123,12 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             v[2 * p + 1] = double(sum[p].y) - double(cmp[p].y);
         }
         if (runs.fa < runs.fb || runs.fc < runs.fd)
-            add_far_cells_mc<C, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C), runs,
-                                                 a.splits, split, kCellBitsMixed, F[t0], F[tl],
-                                                 F[jj < t1 ? jj : tl], v);
-        if (jj < t1) {
+            add_far_cells_mc<C, kCellTermsMixed, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C), runs,
+                                                     a.splits, split, sub, kCellBitsMixed, F[t0], F[tl],
+                                                     F[jj < t1 ? jj : tl], v);
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = sum_subsets<LS>(v[c]);
+        if (sub == 0 && jj < t1) {
 #pragma unroll
             for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, v[c]);
         }
@@ -2170,14 +2191,10 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
     float (*T)[kCoreRow] = tab[warp];
     core_table_clear(T, lane);
     const int K = a.kc[kMaxCond + c];  // the condition's core-pass reach
-    const int g = c / a.group, kg = c - g * a.group;
+    const int g = c / a.group;
     const CoreIv* civ = a.civ + size_t(c) * size_t(a.n);
     const float2* cyp = a.cyp + size_t(c) * size_t(a.n);
     const LineShX* lsh = a.lsh + size_t(a.wslot[g]) * size_t(a.n);
-    // Cy of this condition in the group's LineR1 records (step two's u)
-    const size_t r1b = line_r1_bytes(a.group);
-    const unsigned char* r1 = static_cast<const unsigned char*>(a.rec) + size_t(g) * size_t(a.n) * r1b +
-                              sizeof(float) * size_t(kg);
     // step two's core candidates of a row: the group's reach (kc - 1)
     int kcg = 0;
     for (int q = 0; q < a.group; ++q) kcg = max(kcg, a.kc[g * a.group + q]);
@@ -2203,7 +2220,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
                     const float2 yp = cyp[i];
                     const int mline = a.mi[i];
                     const bool cand = kcg > 0 && mline >= t0 - (kcg - 1) && mline <= tl + (kcg - 1);
-                    const float cy = cand ? *reinterpret_cast<const float*>(r1 + size_t(i) * r1b) : 0.0f;
+                    const float cy = region1_cy(yp.x);  // step two's u
                     for (int j = jlo; j <= jhi; ++j) {
                         const float X = (s.flags & kLineWhole) ? float((s.nu - a.freq[j]) / s.nu)
                                                                : fmaf(s.m - float(j), s.dfn, s.rn);
@@ -2528,62 +2545,53 @@ cudaError_t run_voigt(int blocks, const StepArgs& a, cudaStream_t st, int* occ) 
     return cudaGetLastError();
 }
 
-template <int C, int WARPS>
-cudaError_t run_voigt_mc(int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    const size_t smem = size_t(WARPS) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64));
-    if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(k_steptwo_voigt_mc<C, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem)) != cudaSuccess)
-            return cudaGetLastError();
-    }
+template <class K>
+cudaError_t run_group_kernel(K kernel, int threads, size_t smem, int blocks, const StepArgs& a, cudaStream_t st,
+                             int* occ) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
+        return cudaGetLastError();
     if (occ) {
-        *occ = blocks_per_sm(k_steptwo_voigt_mc<C, WARPS>, WARPS * 32, smem);
+        *occ = blocks_per_sm(kernel, threads, smem);
         return cudaSuccess;
     }
-    k_steptwo_voigt_mc<C, WARPS><<<blocks, WARPS * 32, smem, st>>>(a);
+    kernel<<<blocks, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <int C, int WARPS>
-cudaError_t run_voigt_mcx(int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    const size_t smem = size_t(WARPS) * 64 * (sizeof(float4) + sizeof(int2) + sizeof(LineR1<C>));
-    if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(k_steptwo_voigt_mcx<C, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(smem)) != cudaSuccess)
-            return cudaGetLastError();
-    }
-    if (occ) {
-        *occ = blocks_per_sm(k_steptwo_voigt_mcx<C, WARPS>, WARPS * 32, smem);
-        return cudaSuccess;
-    }
-    k_steptwo_voigt_mcx<C, WARPS><<<blocks, WARPS * 32, smem, st>>>(a);
-    return cudaGetLastError();
+template <int C, int WARPS, int LS, bool MIXED>
+cudaError_t run_group(int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+    if constexpr (MIXED)
+        return run_group_kernel(k_steptwo_voigt_mcx<C, WARPS, LS>, WARPS * 32, size_t(WARPS) * mcx_warp_smem<C>(),
+                                blocks, a, st, occ);
+    else
+        return run_group_kernel(k_steptwo_voigt_mc<C, WARPS, LS>, WARPS * 32,
+                                size_t(WARPS) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64)), blocks, a, st, occ);
+}
+
+template <int C, int WARPS, bool MIXED>
+cudaError_t dispatch_mc_ls(int LS, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+    if (LS == 1) return run_group<C, WARPS, 1, MIXED>(blocks, a, st, occ);
+    if (LS == 4) return run_group<C, WARPS, 4, MIXED>(blocks, a, st, occ);
+    return cudaErrorInvalidValue;
 }
 
 template <int WARPS, bool MIXED>
-cudaError_t dispatch_mc_c(int C, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    if (MIXED) {
-        switch (C) {
-            case 2: return run_voigt_mcx<2, WARPS>(blocks, a, st, occ);
-            case 4: return run_voigt_mcx<4, WARPS>(blocks, a, st, occ);
-            case 8: return run_voigt_mcx<8, WARPS>(blocks, a, st, occ);
-            default: return cudaErrorInvalidValue;
-        }
-    }
+cudaError_t dispatch_mc_c(int C, int LS, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
     switch (C) {
-        case 2: return run_voigt_mc<2, WARPS>(blocks, a, st, occ);
-        case 4: return run_voigt_mc<4, WARPS>(blocks, a, st, occ);
-        case 8: return run_voigt_mc<8, WARPS>(blocks, a, st, occ);
+        case 2: return dispatch_mc_ls<2, WARPS, MIXED>(LS, blocks, a, st, occ);
+        case 4: return dispatch_mc_ls<4, WARPS, MIXED>(LS, blocks, a, st, occ);
+        case 8: return dispatch_mc_ls<8, WARPS, MIXED>(LS, blocks, a, st, occ);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t dispatch_mc(bool mixed, int C, int warps, int blocks, const StepArgs& a,
+cudaError_t dispatch_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
                         cudaStream_t st, int* occ) {
-    if (warps == 4) return mixed ? dispatch_mc_c<4, true>(C, blocks, a, st, occ)
-                                 : dispatch_mc_c<4, false>(C, blocks, a, st, occ);
-    if (warps == 8) return mixed ? dispatch_mc_c<8, true>(C, blocks, a, st, occ)
-                                 : dispatch_mc_c<8, false>(C, blocks, a, st, occ);
+    if (warps == 4) return mixed ? dispatch_mc_c<4, true>(C, LS, blocks, a, st, occ)
+                                 : dispatch_mc_c<4, false>(C, LS, blocks, a, st, occ);
+    if (warps == 8) return mixed ? dispatch_mc_c<8, true>(C, LS, blocks, a, st, occ)
+                                 : dispatch_mc_c<8, false>(C, LS, blocks, a, st, occ);
     return cudaErrorInvalidValue;
 }
 
@@ -2749,16 +2757,16 @@ cudaError_t launch_core_mcx(const CoreArgs& a, int ncond, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int blocks, const StepArgs& a,
+cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
                               cudaStream_t stream) {
     if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
-    return dispatch_mc(mixed, C, warps, blocks, a, stream, nullptr);
+    return dispatch_mc(mixed, C, warps, LS, blocks, a, stream, nullptr);
 }
 
-int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps) {
+int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int LS) {
     StepArgs dummy{};
     int occ = 0;
-    if (dispatch_mc(mixed, C, warps, 0, dummy, nullptr, &occ) != cudaSuccess) return 0;
+    if (dispatch_mc(mixed, C, warps, LS, 0, dummy, nullptr, &occ) != cudaSuccess) return 0;
     return occ;
 }
 
@@ -2771,10 +2779,9 @@ ScratchPlan plan_scratch(int kind, bool mixed, size_t n, int ncond, size_t base_
     auto al = [](size_t v) { return (v + 255) / 256 * 256; };
     ScratchPlan p;
     const size_t nwin = group > 0 ? size_t((ncond + group - 1) / group) : size_t(ncond);
-    // records: per (line, condition), or for the mixed multi-condition layout
-    // one LineR1<group> per (line, group)
-    const size_t rec_bytes = group > 0 ? (mixed ? line_r1_bytes(group) * n * nwin
-                                                : sizeof(CondRec64) * n * size_t(ncond))
+    // records: per (line, condition); the mixed multi-condition layout has
+    // (y, pref) and the region intervals below instead
+    const size_t rec_bytes = group > 0 ? (mixed ? 0 : sizeof(CondRec64) * n * size_t(ncond))
                                        : record_bytes(kind, mixed) * n * size_t(ncond);
     p.off_rec = al(base_off);
     p.off_wlo = al(p.off_rec + rec_bytes);

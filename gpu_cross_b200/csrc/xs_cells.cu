@@ -28,7 +28,7 @@ __device__ __forceinline__ void transpose_sum(double (&v)[32], int lane) {
 
 // One warp per (cell, group of conditions), lanes over the cell's lines.
 // Step one's records give y and pref of each (line, condition):
-//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64), cyp (mixed).
+//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64), cyp (mixed, c pref).
 template <bool MIXED, bool GROUPED, int C>
 __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
     constexpr int PM = cell_moments(MIXED);
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
             load(i, k, y, pref);
             const double nu = a.nu[i];
             const double w = nu * dpw;
-            const double A = pref * w * (0.5 * kW4C * rq);
+            const double A = pref * w * ((GROUPED && MIXED ? 0.5 : 0.5 * kW4C) * rq);
             const double d = (nu - c0) * rq, s = s2 * w * rq, gam = y * w * rq;
             // I_k = A Im(zeta^k) of both poles by
             // I_{k+1} = 2 Re(zeta) I_k - |zeta|^2 I_{k-1}
@@ -144,6 +144,7 @@ cudaError_t run_cells(const CellArgs& a, cudaStream_t st) {
                     unsigned(a.group > 1 ? a.ncond / a.group : a.ncond));
     switch (a.group) {
         case 0: k_cells<MIXED, false, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        case 1: k_cells<MIXED, true, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
         case 2: k_cells<MIXED, true, 2><<<grid, kCellWarps * 32, 0, st>>>(a); break;
         case 4: k_cells<MIXED, true, 4><<<grid, kCellWarps * 32, 0, st>>>(a); break;
         case 8: k_cells<MIXED, true, 8><<<grid, kCellWarps * 32, 0, st>>>(a); break;

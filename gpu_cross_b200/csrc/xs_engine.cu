@@ -509,8 +509,12 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             C = it->second.C;
         }
     }
-    // (32-point tiles decide whether the call's far wings can go by cells)
-    const bool cells = !(ov && ov->scratch) && cell_shift(*opt, conds, ncond, n, *grid, 32) > 0;
+    // whether the call's far wings can go by cells on tiles of `pts` points
+    auto cells_at = [&](int pts) {
+        return !(ov && ov->scratch) && cell_shift(*opt, conds, ncond, n, *grid, pts) > 0;
+    };
+    const bool cells = cells_at(32);
+    const bool narrow_tiles = P <= 1;  // the caller did not ask for wide ones
     {
         int dP, dW;
         double cutmax = 0.0;
@@ -573,15 +577,23 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             // two against 2.80 with one); without cells FP64 is faster with
             // one condition and 32*P points per warp.
             C = (mixed || cells) && groups_ok(2) ? 2 : 1;
+            // mixed, 8-point rows (a coarse grid over a dense list): as many
+            // conditions per warp as the batch allows (29.6 ms at 8 and 4,
+            // 37.9 at 2 for the sweep of 40)
+            if (mixed && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid))
+                for (int cg : {4, 8})
+                    if (groups_ok(cg)) C = cg;
         } else if (C > 1 && !groups_ok(C)) {
             return fail(XS_ERR_INVALID, "conditions_per_warp needs ncond <= 64 and, for every cut, a "
                                         "number of conditions that is a multiple of it");
         }
     }
-    const int CG = C > 1 ? C : 0;
+    // Single mixed conditions with cells: lane = line, 32-point tiles.
+    const bool near = mixed && C == 1 && narrow_tiles && cells;
+    const int CG = near || C > 1 ? C : 0;
     // Rows of 8 points and 4 lines at a time where a 32-point row is wider than
     // what has to be taken line by line beside it (about 6 cells).
-    const int LS = CG && !(ov && ov->scratch) && row_is_wide(*opt, conds, ncond, n, *grid) ? 4 : 1;
+    const int LS = C > 1 && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid) ? 4 : 1;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
         return fail(XS_ERR_INVALID, "line_splits must be 0 (automatic) .. 64");
 
@@ -591,8 +603,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Scratch layout for one group of conditions.
     const int group = ncond < kMaxCond ? ncond : kMaxCond;
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
-    int occ = CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, LS)
-                 : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
+    if (near) W = 4;
+    int occ = near ? steptwo_near_blocks_per_sm()
+              : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, LS)
+                   : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
     if (occ < 1) {
         // e.g. 8 FP64 conditions per warp with 8 warps: more shared memory
         // than a block can have
@@ -608,7 +622,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // different warps -- enough for about 16 items per resident warp, at
     // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
-    const int tile_pts = CG ? 32 / LS : 32 * P;
+    const int tile_pts = near ? 32 : CG ? 32 / LS : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
@@ -782,7 +796,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         // window slots: groups with the same cut (consecutive) share the
         // first one's window data
         for (int g = 0; CG && g < nc / CG; ++g)
-            pa.wslot[g] = (g > 0 && pa.cond[g * CG].cut == pa.cond[(g - 1) * CG].cut) ? pa.wslot[g - 1] : g;
+            pa.wslot[g] = (CG > 1 && g > 0 && pa.cond[g * CG].cut == pa.cond[(g - 1) * CG].cut) ? pa.wslot[g - 1] : g;
 
         if (timing && c0 == 0) cudaEventRecordWithFlags(e->ev[0], st, ev_flags);
         err = cudaMemsetAsync(pa.kc, 0, sizeof(int) * size_t(kKcWords), st);
@@ -886,6 +900,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         if (CG) {
             sa.lsh = pa.lsh;
             sa.cyp = pa.cyp;
+            sa.civ = pa.civ;
             for (int g = 0; g < nc / CG; ++g) sa.wslot[g] = pa.wslot[g];
             sa.group = CG;
             sa.tiles_per_cond = tiles;
@@ -922,11 +937,14 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
-        err = CG ? launch_steptwo_mc(mixed, CG, W, LS, blocks, sa, st)
+        err = near ? launch_steptwo_near(blocks, sa, st)
+              : CG ? launch_steptwo_mc(mixed, CG, W, LS, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);
         if (err != cudaSuccess) return cuda_fail(err, "step two launch");
         if (blocks > 0 && sa.n_items > 0) ++launched;
-        if (CG && mixed) {
+        if (near) {
+            // W4 regions II-IV are in step two
+        } else if (CG && mixed) {
             // the pairs inside the lines' region intervals (W4 regions II-IV),
             // into the split parts before they are added up
             CoreArgs ca;

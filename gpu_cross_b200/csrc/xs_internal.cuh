@@ -111,10 +111,12 @@ static_assert(sizeof(RecV32) == 64, "RecV32 layout");
 // X = (nu - f_j) / nu = (m - j) dfn + rn and k = 1 / dpw.  One X per
 // (line, point) then serves every condition of the group, and
 // u = x^2 + Cy = X^2 k^2 + Cy.
+// Groups of one condition (lane = line step two) hold the offsets in Doppler
+// widths instead, x = (m - j) dfn + rn.
 struct __align__(16) LineShX {
     float m;      // nearest grid index (exact below 2^24)
-    float dfn;    // df / nu
-    float rn;     // (nu - f0 - m df) / nu
+    float dfn;    // df / nu (one condition: df g)
+    float rn;     // (nu - f0 - m df) / nu (one condition: times g)
     int flags;    // kLineWhole: X from nu in FP64 and every pair of the line
                   // tested; kLineWide: region-I products need the scaled
                   // shared reciprocal
@@ -242,8 +244,8 @@ struct PrepArgs {
                         // conditions per group (Voigt only)
     void* lsh;          // multi-condition: per-line shared records per group
                         // (LineShX mixed, LineSh64 FP64)
-    CoreIv* civ;        // mixed multi-condition: region intervals and
-    float2* cyp;        //   (y, pref) per (condition, line), condition-major
+    CoreIv* civ;        // mixed group layouts: region intervals and
+    float2* cyp;        //   (y, c pref) per (condition, line), condition-major
     // Multi-condition layouts: the window slot of each group -- groups with
     // the same cut (consecutive, conditions being ordered by cut) share one
     // copy of the per-line window data (LineShX / LineSh64, lo, hi), that of
@@ -272,7 +274,8 @@ struct StepArgs {
     size_t out_stride;  // elements between conditions
     GridDev G;
     const void* lsh;    // multi-condition layout (LineShX mixed, LineSh64 FP64)
-    const float2* cyp;  // mixed multi-condition: (y, pref), condition-major
+    const float2* cyp;  // mixed group layouts: (y, c pref), condition-major,
+    const CoreIv* civ;  //   and the region intervals
     int wslot[kMaxCond];  // window slot of each group (PrepArgs::wslot)
     int group;          // conditions per group (multi-condition kernel)
     int tiles_per_cond;
@@ -307,7 +310,7 @@ struct CellArgs {
     int ncond;
     int group;          // conditions per group (0: single-condition layout)
     const void* rec;    // RecV64 / RecV32, or CondRec64 (FP64 groups)
-    const float2* cyp;  // mixed groups: (y, pref)
+    const float2* cyp;  // mixed groups: (y, c pref), c = kW4C
     int cshift, ncell;
     double df;
     CellHead* head;
@@ -396,6 +399,11 @@ cudaError_t launch_check_snapshot(const CheckArgs& a, cudaStream_t stream);
 // FP64 sums at the sampled points and the per-condition statistics
 // (launched after the call's last kernel).
 cudaError_t launch_check_rows(const CheckArgs& a, cudaStream_t stream);
+
+// Mixed single-condition step two with cells, lane = line (LineShX, civ, cyp
+// records, groups of one condition), W4 regions II-IV included; 4 warps a block.
+cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream);
+int steptwo_near_blocks_per_sm();
 
 // Multi-condition step two (Voigt): C conditions per warp.
 // LS lane subsets share a row of 32 / LS points (LS = 1 or 4).

@@ -380,7 +380,34 @@ __device__ __forceinline__ int prep_line(const PrepArgs& a, long i, int c, int* 
             }
             return kcl;
         }
-        if (MIXED) {
+        if (MIXED && a.group == 1) {
+            // one condition per group of the line-parallel step two: offsets
+            // scaled by g, x = (m - j) dfn + rn
+            LineShX ls;
+            const bool far_m = !(fabs(m) < 16000000.0);
+            const double xw = (cut + double(a.mixed_tile_span + 4) * df) * g;
+            ls.m = float(far_m ? 0.0 : m);
+            ls.dfn = float(df * g);
+            ls.rn = float(((nu_p - f0) - m * df) * g);
+            ls.flags = (far_m ? kLineWhole : 0) |
+                       (!(xw * xw + y2 < kPairUMax) || !(fabs(Pc) < kPairPcMax) ? kLineWide : 0);
+            ls.lo = lo;
+            ls.hi = hi;
+            ls.nu = nu_p;
+            reinterpret_cast<LineShX*>(a.lsh)[ci] = ls;
+            CoreIv iv;
+            region_intervals(nu_p, g, y, lo, hi, f0, df, iv.lo15, iv.hi15, iv.lo55, iv.hi55);
+            int rch = 0;
+            if (iv.lo15 <= iv.hi15) {
+                const double w = fmax(m - double(iv.lo15), double(iv.hi15) - m);
+                rch = w < 3.0e7 ? int(w) : 30000000;
+                if (!(w < 3.0e7)) atomicOr(a.err, kErrReach);
+            }
+            if (reach) *reach = rch;
+            kcl = 0;
+            a.civ[ci] = iv;
+            a.cyp[ci] = make_float2(float(y), float(pref * kW4C));
+        } else if (MIXED) {
             RecV32 rr;
             rr.m = float(fabs(m) < 16000000.0 ? m : 0.0);
             rr.ra = float(((nu_p - f0) - m * df) * g);
@@ -652,7 +679,7 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
                 if (whole) kcl = 30000000;  // a core candidate of every tile
                 const size_t ci = size_t(c) * size_t(a.L.n) + size_t(i);
                 a.civ[ci] = iv;
-                a.cyp[ci] = make_float2(float(y), float(pref));
+                a.cyp[ci] = make_float2(float(y), float(pref * kW4C));
             }
             kcl = __reduce_max_sync(0xffffffffu, kcl);
             rch = __reduce_max_sync(0xffffffffu, rch);
@@ -717,6 +744,12 @@ __device__ long warp_lower_bound(long lo, long hi, int lane, Pred pred) {
     if (b == 0u) return hi;
     const long r = lo + (__ffs(b) - 1);
     return r < hi ? r : hi;
+}
+
+// First i in [lo, hi) with v[i] >= key (v ascending), or hi.  One copy of the
+// search for the kernels whose code has to stay small.
+__device__ __noinline__ int warp_search(const int* v, int lo, int hi, int key, int lane) {
+    return int(warp_lower_bound(lo, hi, lane, [&](long i) { return v[i] >= key; }));
 }
 
 // Copy `cnt` records of REC (sizeof a multiple of 16) into shared memory,
@@ -978,12 +1011,6 @@ __device__ __forceinline__ fcplx operator*(fcplx a, fcplx b) {
     return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re};
 }
 
-// W4 region II (5.5 <= |x| + y < 15) as a real expression with the factor y
-// explicit.  With T = y - ix, U = T^2 = Ur + i Ui, N = a + b U and
-// D = c + U (3 + U):
-//   Re[T N / D] = y [(a + b y^2 - 3 b x^2) Dr + 2 x^2 (3 + 2 Ur)(Nr + 2 b y^2)] / |D|^2
-// (expanding Re[T N conj(D)]); a complex evaluation would cancel by a factor
-// x / y in the wings of narrow lines.
 // a / b for the FP32 W4 forms of regions II and III (no cancellation
 // follows there): the hardware reciprocal and one product, within 2 ulp; the
 // denominators lie between about 0.5 and 1e6, far from the range where the
@@ -991,25 +1018,41 @@ __device__ __forceinline__ fcplx operator*(fcplx a, fcplx b) {
 __device__ __forceinline__ float region_div(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double region_div(double a, double b) { return a * rcp_newton2_f64(b); }
 
+// W4 region II (5.5 <= |x| + y < 15): T (a + b U) / (c + U (3 + U)), T = y - ix,
+// U = T^2, a = 1.410474, b = .5641896, c = .75.  Its denominator has the roots
+// U = -(3 -+ sqrt 6) / 2 = -B1, -B2, so it is T [A1 / (U + B1) + A2 / (U + B2)]
+// with A1 + A2 = b, A1 B2 + A2 B1 = a, and as Re[T / (U + B)] =
+// y (v + B) / ((v - B)^2 + 4 B y^2), v = x^2 + y^2 (region I is the same with
+// B = 1/2), its real part is a sum of positive terms: no cancellation, and half
+// the operations of the complex form's real part.
+constexpr double kW4Root6 = 2.44948974278317809820;
+constexpr double kW4B1 = 0.5 * (3.0 - kW4Root6), kW4B2 = 0.5 * (3.0 + kW4Root6);
+constexpr double kW4A1 = (1.410474 - .5641896 * kW4B1) / kW4Root6;
+constexpr double kW4A2 = (.5641896 * kW4B2 - 1.410474) / kW4Root6;
+// Per unit c = kW4C, from u = x^2 + y^2 - 1/2 = v - 1/2: in FP32 this order and
+// these constants leave an rms error of 0.9e-7 and a mean of 4e-9 over the
+// region (the complex form's real part: 1.8e-7 and 3e-8).
+template <class R>
+__device__ __forceinline__ R w4_region2_c(R x, R y) {
+    const R y2 = y * y, u = x * x + (y2 - R(0.5));
+    const R e1 = u + R(0.5 - kW4B1), e2 = u + R(0.5 - kW4B2);
+    const R d1 = e1 * e1 + R(2) * y2 * R(2.0 * kW4B1), d2 = e2 * e2 + R(2) * y2 * R(2.0 * kW4B2);
+    const R p1 = y * R(kW4A1 / kW4C), p2 = y * R(kW4A2 / kW4C);
+    const R n1 = u * p1 + p1 * R(0.5 + kW4B1), n2 = u * p2 + p2 * R(0.5 + kW4B2);
+    return region_div(n1 * d2 + n2 * d1, d1 * d2);
+}
 template <class R>
 __device__ __forceinline__ R w4_region2_re(R x, R y) {
-    const R a = R(1.410474), b = R(.5641896), c = R(.75);
-    const R x2 = x * x, y2 = y * y;
-    const R ur = y2 - x2, ui = R(-2) * x * y;
-    const R nr = a + b * ur;
-    const R dr = c + R(3) * ur + ur * ur - ui * ui;
-    const R di = ui * (R(3) + R(2) * ur);
-    const R br = (a + b * y2 - R(3) * b * x2) * dr + R(2) * x2 * (R(3) + R(2) * ur) * (nr + R(2) * b * y2);
-    return region_div(y * br, dr * dr + di * di);
+    return R(kW4C) * w4_region2_c(x, y);
 }
 
-// The region-I rational of W4 in FP32 per unit pref, as step two evaluates
-// it: kW4C y (u + 1) / (u^2 + 2 y^2), u = x^2 + y^2 - 0.5.  The core pass
+// The region-I rational of W4 in FP32 per unit c pref, as step two evaluates
+// it: y (u + 1) / (u^2 + 2 y^2), u = x^2 + y^2 - 0.5.  The core pass
 // takes it back off the pairs where step two added it.
-__device__ __forceinline__ float w4_region1_re_f32(float x, float y) {
+__device__ __forceinline__ float w4_region1_c(float x, float y) {
     const float y2 = y * y;
     const float u = fmaf(x, x, y2 - 0.5f);
-    return region_div(float(kW4C) * y * (u + 1.0f), fmaf(u, u, 2.0f * y2));
+    return region_div(y * (u + 1.0f), fmaf(u, u, 2.0f * y2));
 }
 
 // W4 region III in FP32 (there y >= 0.195|x| - 0.176, so Re w is not small
@@ -1852,8 +1895,13 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                 keep0 = keep0 && !(u.x < 1.0f);
                 keep1 = keep1 && !(u.y < 1.0f);
             }
-            const float2 den = __ffma2_rn(u, u, d2);
-            const float2 num = __ffma2_rn(u, pc, pc);
+            float2 den = __ffma2_rn(u, u, d2);
+            float2 num = __ffma2_rn(u, pc, pc);
+            if constexpr (MODE >= 1) {
+                // Pc / u to FP32 rounding, and u^2 overflows from 1.8e19
+                if (u.x > 1.0e12f) den.x = u.x, num.x = pc.x;
+                if (u.y > 1.0e12f) den.y = u.y, num.y = pc.y;
+            }
             const float2 rr = f2(keep0 ? rcp_approx_f32(den.x) : 0.0f, keep1 ? rcp_approx_f32(den.y) : 0.0f);
             if constexpr (MODE >= 1) {
                 acc[p].x += keep0 ? num.x * rr.x : 0.0f;
@@ -1959,7 +2007,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                     *reinterpret_cast<float2*>(&r.Cy[c]) = f2(region1_cy(v0.x), region1_cy(v1.x));
                     *reinterpret_cast<float2*>(&r.D2[c]) = f2(2.0f * v0.x * v0.x, 2.0f * v1.x * v1.x);
                     *reinterpret_cast<float2*>(&r.Pc[c]) =
-                        f2(v0.y * float(kW4C) * v0.x, v1.y * float(kW4C) * v1.x);
+                        f2(v0.y * v0.x, v1.y * v1.x);
                 }
             }
             __syncwarp();
@@ -2089,9 +2137,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const int c = 2 * p + h;
-                            // beyond x ~ 1e9 (lines far off the FP32 offset
-                            // range) region I is taken as 0
-                            keep[h] = in && aX * a.kx[cg * C + c] < 1.0e9f;
+                            // beyond x = 1e18 region I is taken as 0
+                            keep[h] = in && aX * a.kx[cg * C + c] < 1.0e18f;
                         }
                         region1(guarded_near, X2, SR[t], p, keep[0], keep[1]);
                     }
@@ -2227,13 +2274,13 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
                         const float ax = fabsf(X) * k, y = yp.x;
                         float w;
                         if (j >= iv.lo55 && j <= iv.hi55)
-                            w = (y >= fmaf(0.195f, ax, -0.176f)) ? w4_region3_re_f32(ax, y)
-                                                                  : w4_region4_re_f32(ax, y);
+                            w = float(1.0 / kW4C) * ((y >= fmaf(0.195f, ax, -0.176f)) ? w4_region3_re_f32(ax, y)
+                                                                                       : w4_region4_re_f32(ax, y));
                         else
-                            w = w4_region2_re<float>(ax, y);
+                            w = w4_region2_c(ax, y);
                         // step two added the region-I rational here unless the
                         // line was its core candidate and u < 1 (the same FP32 u)
-                        if (!(cand && fmaf(X * X, k2, cy) < 1.0f)) w -= w4_region1_re_f32(ax, y);
+                        if (!(cand && fmaf(X * X, k2, cy) < 1.0f)) w -= w4_region1_c(ax, y);
                         T[j - t0][lane] = yp.y * w;
                     }
                 }
@@ -2310,6 +2357,296 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
             a.out[size_t(a.row[c]) * a.out_stride + size_t(jj)] += acc;
         else
             a.part[(size_t(c) * S + split) * a.part_stride + size_t(jj - a.G.start)] += acc;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Mixed-precision single-condition step two with cells, lane = line.
+//
+// With the far wings taken by cells, what is left of a tile is a few thousand
+// lines on few points, so the lanes go over the lines: a warp takes a tile of
+// 32 points and 32 lines at a time, each lane evaluating its own line at every
+// point of the tile into 32 accumulators.  The line's constants are read once
+// per lane (a broadcast to every lane costs a shared-memory wavefront per 4
+// bytes), and the lines of a group, being neighbours, are in the same W4 region
+// at the same point.  Every 8 groups of lines the accumulators are summed over
+// the lanes (a transposing exchange: lane p ends with point p) and added in
+// FP64 (sums 8 + 5 deep: 4.5e-8 of the result in the 2-norm, 7.0e-8 with 32
+// groups; the point-parallel kernel 5.3e-8).
+//
+// Two evaluations share one reciprocal, 1/dA = dB / (dA dB) (narrow lines,
+// kPairUMax).  Groups with lines of the core reach choose region I or II per
+// pair by the exact region intervals; the pairs of regions III and IV, and all
+// pairs of groups with wide or whole lines, are evaluated in a loop by their
+// own line's lane into a per-warp table with a column per lane.  (Few unrolled
+// bodies: with every region unrolled a third of the time went to instruction
+// fetches.)
+//
+// B200, 1e7 lines, 7.5e5 points: 3.37 ms against 3.5 + 1.2 ms for the
+// point-parallel kernel with cells and its core pass; 96 registers, 57 % of the
+// issue slots.  The same kernel over 4 points and 8 conditions was slower than
+// k_steptwo_voigt_mcx on the coarse sweep (20.7 against 12.6 ms).
+// ---------------------------------------------------------------------------
+constexpr int kNearRow = 33;
+constexpr int kNearWarps = 4;
+// Two stages of offsets and flags, windows and (y, pref), and the table.
+constexpr size_t kNearWarpSmem = 64 * (sizeof(float4) + sizeof(int2) + sizeof(float2)) + sizeof(float) * 32 * kNearRow;
+// Sum over the warp of 32 values per lane: lane L gets that of value L.
+__device__ __forceinline__ float transpose_sum_f32(float2 (&v)[16], int lane) {
+    float w[16];
+    {
+        const bool up = (lane & 16) != 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            // values i and i + 16
+            const float lo = (i & 1) ? v[i / 2].y : v[i / 2].x;
+            const float hi = (i & 1) ? v[8 + i / 2].y : v[8 + i / 2].x;
+            const float got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, 16);
+            w[i] = (up ? hi : lo) + got;
+        }
+    }
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const float got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + o], o);
+            w[i] = (up ? w[i + o] : w[i]) + got;
+        }
+    }
+    return w[0];
+}
+
+__global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    unsigned char* const mine = smem_raw + size_t(threadIdx.x >> 5) * kNearWarpSmem;
+    float4* lsb = reinterpret_cast<float4*>(mine);
+    float2* ypb = reinterpret_cast<float2*>(mine + 64 * sizeof(float4));
+    int2* lhb = reinterpret_cast<int2*>(ypb + 64);
+    float (*T)[kNearRow] = reinterpret_cast<float (*)[kNearRow]>(lhb + 64);
+    const double* F = a.G.freq;
+    const int* mi = a.mi;
+#pragma unroll 4
+    for (int q = 0; q < 32; ++q) T[q][lane] = 0.0f;
+    __syncwarp();
+
+    WorkItem w;
+    while (next_item(a, 1, lane, w)) {
+        const int t0 = w.t0, t1 = w.t1, tl = t1 - 1;
+        const size_t cbase = size_t(w.c) * size_t(a.n);
+        const int* whi = a.whi + cbase;
+        const int* wlo = a.wlo + cbase;
+        const int K = a.kc[kMaxCond + w.c];  // the condition's core reach
+        const int La = warp_search(whi, 0, int(a.n), t0 + 1, lane);
+        const int Lb = warp_search(wlo, La, int(a.n), t1, lane);
+        const int fs = warp_search(whi, La, Lb, t1, lane);
+        const int Cb = warp_search(wlo, La, Lb, t0 + 1, lane);
+        const int fe = Cb > fs ? Cb : fs;
+        const int E = warp_search(mi, La, Lb, t0 - K, lane);
+        const int Fc = warp_search(mi, E, Lb, tl + K + 1, lane);
+        const LineShX* lsh = reinterpret_cast<const LineShX*>(a.lsh) + cbase;
+        const float2* yp = a.cyp + cbase;
+        const CoreIv* civ = a.civ + cbase;
+        const size_t cell0 = size_t(w.c) * size_t(a.ncell);
+        const LineRuns runs =
+            line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
+
+        const float t0f = float(t0);
+        float2 acc[16];  // points 2 q, 2 q + 1
+#pragma unroll
+        for (int v = 0; v < 16; ++v) acc[v] = f2(0.0f, 0.0f);
+        double sum = 0.0;
+        bool cored = false;  // the table holds something
+
+        // Region-I constants of the line.
+        struct R1 {
+            float2 cy, d2, pc;
+        };
+        auto constants = [&](float2 v) {
+            R1 r;
+            r.cy = f2s(region1_cy(v.x));
+            r.d2 = f2s(2.0f * v.x * v.x);
+            r.pc = f2s(v.y * v.x);
+            return r;
+        };
+        auto offsets = [&](float mj, const float4& s, int q) {
+            const float2 d = __fadd2_rn(f2s(mj), f2(-float(2 * q), -float(2 * q + 1)));
+            return __ffma2_rn(d, f2s(s.y), f2s(s.z));
+        };
+        // to += num / den for both halves, one reciprocal.
+        auto add_pair = [&](float2 num, float2 den, float2& to) {
+            const float rq = rcp_approx_f32(den.x * den.y);
+            to = __ffma2_rn(num, __fmul2_rn(f2(den.y, den.x), f2s(rq)), to);
+        };
+        // One group of lines, region I only; MASK: some windows cover the tile
+        // partly (or there are fewer than 32 lines).
+        auto plain_group = [&](auto mask, float4 s, int2 win, float2 v) {
+            const float mj = s.x - t0f;
+            const unsigned wlen = unsigned(win.y - win.x);
+            const int w0 = t0 - win.x;
+            const R1 r = constants(v);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const float2 x = offsets(mj, s, q);
+                const float2 u = __ffma2_rn(x, x, r.cy);
+                float2 num = __ffma2_rn(u, r.pc, r.pc);
+                if constexpr (decltype(mask)::value)
+                    num = f2(unsigned(w0 + 2 * q) < wlen ? num.x : 0.0f, unsigned(w0 + 2 * q + 1) < wlen ? num.y : 0.0f);
+                add_pair(num, __ffma2_rn(u, u, r.d2), acc[q]);
+            }
+        };
+        // A group of narrow lines with core candidates: region I or II chosen
+        // per pair by the region intervals; the pairs of regions III and IV are
+        // left to inner_pairs.
+        auto core_group = [&](float4 s, int2 win, float2 v, const CoreIv& iv) {
+            const float mj = s.x - t0f;
+            const unsigned wlen = unsigned(win.y - win.x);
+            const int w0 = t0 - win.x;
+            // an interval's start relative to t0 and its length (empty: far off)
+            const int d15 = iv.lo15 <= iv.hi15 ? t0 - iv.lo15 : -0x40000000;
+            const int d55 = iv.lo55 <= iv.hi55 ? t0 - iv.lo55 : -0x40000000;
+            const unsigned l15 = unsigned(iv.hi15 - iv.lo15), l55 = unsigned(iv.hi55 - iv.lo55);
+            const unsigned n15 = iv.lo15 <= iv.hi15 ? l15 : 0u, n55 = iv.lo55 <= iv.hi55 ? l55 : 0u;
+            const R1 r = constants(v);
+            const float2 p1 = __fmul2_rn(r.pc, f2s(float(kW4A1 / kW4C)));
+            const float2 p2 = __fmul2_rn(r.pc, f2s(float(kW4A2 / kW4C)));
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const float2 x = offsets(mj, s, q);
+                const float2 u = __ffma2_rn(x, x, r.cy);
+                float2 den = __ffma2_rn(u, u, r.d2);
+                float2 num = __ffma2_rn(u, r.pc, r.pc);
+                // region II, v = u + 1/2 (r.d2 = 2 y^2)
+                const float2 e1 = __fadd2_rn(u, f2s(float(0.5 - kW4B1)));
+                const float2 e2 = __fadd2_rn(u, f2s(float(0.5 - kW4B2)));
+                const float2 d1 = __ffma2_rn(e1, e1, __fmul2_rn(r.d2, f2s(float(2.0 * kW4B1))));
+                const float2 d2 = __ffma2_rn(e2, e2, __fmul2_rn(r.d2, f2s(float(2.0 * kW4B2))));
+                const float2 n1 = __ffma2_rn(u, p1, __fmul2_rn(p1, f2s(float(0.5 + kW4B1))));
+                const float2 n2 = __ffma2_rn(u, p2, __fmul2_rn(p2, f2s(float(0.5 + kW4B2))));
+                const float2 n = __ffma2_rn(n1, d2, __fmul2_rn(n2, d1));
+                const float2 dd = __fmul2_rn(d1, d2);
+                const int pa = 2 * q, pb = 2 * q + 1;
+                const bool ca = unsigned(d15 + pa) <= n15, cb = unsigned(d15 + pb) <= n15;
+                const bool ka = unsigned(w0 + pa) < wlen && !(unsigned(d55 + pa) <= n55);
+                const bool kb = unsigned(w0 + pb) < wlen && !(unsigned(d55 + pb) <= n55);
+                // (a pair left out enters the product as 1)
+                num = f2(ka ? (ca ? n.x : num.x) : 0.0f, kb ? (cb ? n.y : num.y) : 0.0f);
+                den = f2(ka ? (ca ? dd.x : den.x) : 1.0f, kb ? (cb ? dd.y : den.y) : 1.0f);
+                add_pair(num, den, acc[q]);
+            }
+        };
+        // Pairs of regions III and IV of a core group; `all` (wide and whole
+        // lines): every pair of the window (beyond x = 1e18 region I is taken
+        // as 0); whole lines: X from the FP64 centre.
+        auto inner_pairs = [&](float4 s, int2 win, float2 v, const CoreIv& iv, int i, bool all) {
+            const bool whole = (__float_as_int(s.w) & kLineWhole) != 0;
+            const int jlo = max(all ? win.x : iv.lo55, t0), jhi = min(all ? win.y - 1 : iv.hi55, tl);
+            if (!__any_sync(0xffffffffu, jlo <= jhi)) return;
+            cored = true;
+            const double nu = whole ? lsh[i].nu : 0.0;
+            const float y = v.x;
+#pragma unroll 1
+            for (int j = jlo; j <= jhi; ++j) {
+                const float ax =
+                    fabsf(whole ? float((nu - F[j]) / nu) * a.kx[w.c] : fmaf(s.x - float(j), s.y, s.z));
+                float wf;
+                if (!all || (j >= iv.lo55 && j <= iv.hi55)) {
+                    wf = float(1.0 / kW4C) *
+                         ((y >= fmaf(0.195f, ax, -0.176f)) ? w4_region3_re_f32(ax, y) : w4_region4_re_f32(ax, y));
+                } else if (j >= iv.lo15 && j <= iv.hi15) {
+                    wf = w4_region2_c(ax, y);
+                } else {
+                    // (u + 1) / (u^2 + 2 y^2) is 1 / u to FP32 rounding from u = 1e12
+                    // on (2 y^2 < u there), and u^2 overflows from 1.8e19
+                    const float u = fmaf(ax, ax, region1_cy(y));
+                    const float rat = u > 1.0e12f ? rcp_approx_f32(u)
+                                                  : (u + 1.0f) * rcp_approx_f32(fmaf(u, u, 2.0f * y * y));
+                    wf = ax < 1.0e18f ? y * rat : 0.0f;
+                }
+                T[j - t0][lane] += v.y * wf;
+            }
+            __syncwarp();
+        };
+        // The lanes' partial sums, into point `lane`.
+        auto fold = [&]() {
+            sum += double(transpose_sum_f32(acc, lane));
+#pragma unroll
+            for (int v = 0; v < 16; ++v) acc[v] = f2(0.0f, 0.0f);
+            if (cored) {
+                cored = false;
+                __syncwarp();
+                double t = 0.0;
+#pragma unroll 4
+                for (int q = 0; q < 32; ++q) t += double(T[lane][q]);
+                sum += t;
+                __syncwarp();
+#pragma unroll 4
+                for (int q = 0; q < 32; ++q) T[q][lane] = 0.0f;
+            }
+        };
+
+        const int ngroups = runs.groups_of(a.splits, w.s);
+        auto gstart = [&](int gi, int& end) {
+            long e;
+            const int b = int(runs.start(w.s + gi * a.splits, e));
+            end = int(e);
+            return b;
+        };
+        auto issue = [&](int gi) {
+            if (gi < ngroups) {
+                int end;
+                const int b = gstart(gi, end), at = (gi & 1) * 32 + lane;
+                if (b + lane < end) {
+                    cp_async16(lsb + at, lsh + b + lane);
+                    cp_async8(lhb + at, &lsh[b + lane].lo);
+                    cp_async8(ypb + at, yp + b + lane);
+                }
+            }
+            cp_async_commit();
+        };
+        issue(0);
+        for (int gi = 0; gi < ngroups; ++gi) {
+            issue(gi + 1);
+            cp_async_wait<1>();
+            // (each lane reads only what it copied)
+            int end;
+            const int gb = gstart(gi, end);
+            const int ge = end - gb < 32 ? end : gb + 32;
+            float4 s = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0));  // a line that adds nothing
+            int2 win = make_int2(0, 0);
+            float2 v = f2(1.0f, 0.0f);
+            const bool live = gb + lane < ge;
+            if (live) {
+                const int at = (gi & 1) * 32 + lane;
+                s = lsb[at];
+                win = lhb[at];
+                v = ypb[at];
+            }
+            const bool odd = __any_sync(0xffffffffu, (__float_as_int(s.w) & (kLineWhole | kLineWide)) != 0);
+            if (odd || (ge > E && gb < Fc)) {
+                CoreIv iv = {1, 0, 1, 0};
+                if (live) iv = civ[gb + lane];
+                if (!odd) core_group(s, win, v, iv);
+                inner_pairs(s, win, v, iv, gb + lane, odd);
+            } else if (gb >= fs && ge <= fe && ge - gb == 32) {
+                plain_group(std::false_type(), s, win, v);
+            } else {
+                plain_group(std::true_type(), s, win, v);
+            }
+            if ((gi & 7) == 7) fold();
+        }
+        cp_async_wait<0>();
+        fold();
+
+        const int jj = t0 + lane;
+        const double f[1] = {F[jj < t1 ? jj : tl]};
+        double v[1] = {sum};
+        if (runs.fa < runs.fb || runs.fc < runs.fd)
+            add_far_cells<1, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits, w.s,
+                                              kCellBitsMixed, F[t0], F[tl], f, v);
+        if (jj < t1) put_result(a, w.c, w.s, jj, v[0]);
+        __syncwarp();
     }
 }
 
@@ -2686,7 +3023,7 @@ cudaError_t launch_prep(int kind, int conv, bool mixed, const PrepArgs& a, cudaS
     const long count = (a.line1 > 0 ? a.line1 : a.L.n) - a.line0;
     if (count <= 0 || a.ncond <= 0) return cudaSuccess;
     const dim3 grid(unsigned((count + 255) / 256), unsigned(a.ncond));
-    if (kind == kVoigt && mixed && a.group > 0) {
+    if (kind == kVoigt && mixed && a.group > 1) {
         // (precomputed-intensity lists run one condition at a time)
         if (a.L.s32 != nullptr || a.ncond % a.group != 0) return cudaErrorInvalidValue;
         const unsigned nblk = unsigned((count + 255) / 256);
@@ -2761,6 +3098,15 @@ cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int LS, int blocks, 
                               cudaStream_t stream) {
     if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
     return dispatch_mc(mixed, C, warps, LS, blocks, a, stream, nullptr);
+}
+
+cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream) {
+    if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
+    return run_group_kernel(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem, blocks, a, stream, nullptr);
+}
+
+int steptwo_near_blocks_per_sm() {
+    return blocks_per_sm(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem);
 }
 
 int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int LS) {

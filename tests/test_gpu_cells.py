@@ -108,3 +108,22 @@ def test_cells_chunk_inside_the_grid(engine, cuda):
                          start_idx=start, points=points)[0]
         assert_fp64_parity(got[start:start + points], ref[start:start + points])
         assert not got[:start].any() and not got[start + points:].any()
+
+
+@pytest.mark.parametrize("C", [1, 4])
+def test_cells_low_wavenumbers(engine, cuda, C):
+    """Lines from 0 to 60 cm-1: Doppler widths of a few 1e-5
+    cm-1 and less, so the cut reaches x ~ 1e6 and beyond: wide lines, and cells
+    that no series may stand for."""
+    lines = synth.random_lines(9001, 0.001, 60.0, 2500.0, 1e-6, 1e2, seed=41)
+    grid = synth.Grid(0.5, 70.5, 7000)
+    fr = grid.freq()
+    base = dict(mean_mass=17.03, pressure=1.0, ref_temp=296.0, cut=CUT)
+    conds = [dict(base, temperature=t, partition=synth.partition_poly(t), gamma_scale=p)
+             for t in (300.0, 2100.0) for p in (1e-2, 1.0)]
+    f64 = run_engine(engine, capi.VOIGT, lines, fr, base, grid.dfreq, cuda, conds=conds, C=C)
+    mix = run_engine(engine, capi.VOIGT, lines, fr, base, grid.dfreq, cuda, conds=conds, C=C, precision=capi.MIXED)
+    for k, c in enumerate(conds):
+        ref = reference(capi.CONV_GPU, fr, lines, c, grid.dfreq, c["gamma_scale"])
+        assert_fp64_parity(f64[k], ref)
+        assert_mixed_parity(mix[k], ref)

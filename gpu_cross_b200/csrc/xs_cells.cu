@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <type_traits>
 
 #include "xs_internal.cuh"
 
@@ -28,7 +29,7 @@ __device__ __forceinline__ void transpose_sum(double (&v)[32], int lane) {
 
 // One warp per (cell, group of conditions), lanes over the cell's lines.
 // Step one's records give y and pref of each (line, condition):
-//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64), cyp (mixed, c pref).
+//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64).
 template <bool MIXED, bool GROUPED, int C>
 __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
     constexpr int PM = cell_moments(MIXED);
@@ -42,11 +43,7 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
 
     auto load = [&](long i, int k, double& y, double& pref) {
         const size_t c = size_t(g) * C + k;
-        if constexpr (GROUPED && MIXED) {
-            const float2 v = a.cyp[c * size_t(a.n) + size_t(i)];
-            y = double(v.x);
-            pref = double(v.y);
-        } else if constexpr (GROUPED) {
+        if constexpr (GROUPED) {
             const CondRec64& r = static_cast<const CondRec64*>(a.rec)[(size_t(g) * size_t(a.n) + size_t(i)) * C + k];
             y = r.y;
             pref = r.pref;
@@ -114,7 +111,7 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
             load(i, k, y, pref);
             const double nu = a.nu[i];
             const double w = nu * dpw;
-            const double A = pref * w * ((GROUPED && MIXED ? 0.5 : 0.5 * kW4C) * rq);
+            const double A = pref * w * (0.5 * kW4C * rq);
             const double d = (nu - c0) * rq, s = s2 * w * rq, gam = y * w * rq;
             // I_k = A Im(zeta^k) of both poles by
             // I_{k+1} = 2 Re(zeta) I_k - |zeta|^2 I_{k-1}
@@ -138,16 +135,139 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
     }
 }
 
+// Mixed precision, from the (y, c pref) pairs of the group layouts: the same in
+// FP32, the two poles as one packed FP32x2 operand, the sums over the lanes in
+// FP64.  The amplitudes are taken relative to the cell's largest, so their
+// range does not matter; a moment is off by about 1e-7 of itself, as one FP32
+// evaluation of the line is.
+// Bound by the FP32 pipe: 16 terms x 3 packed operations per (line, condition);
+// 40 conditions x 1e7 lines 4.77 ms in FP64, 2.1 in FP32.
+template <int C>
+__global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
+    constexpr int PM = kCellTermsMixed;
+    static_assert(PM == 16, "the transposed sum below is for 16 values");
+    const int lane = threadIdx.x & 31;
+    const int cell = int(blockIdx.x) * kCellWarps + int(threadIdx.x >> 5);
+    if (cell >= a.ncell) return;
+    const int g = int(blockIdx.y);
+    const long i0 = long(cell) << a.cshift;
+    const long i1 = i0 + (1L << a.cshift) < a.n ? i0 + (1L << a.cshift) : a.n;
+    const double c0 = 0.5 * (a.nu[i0] + a.nu[i1 - 1]);
+    const float2* yp = a.cyp + size_t(g) * C * size_t(a.n);
+    const float s2 = 0.70710678f;
+
+    // scale, reach and the largest amplitudes (all widened by 1e-6, far more
+    // than their FP32 rounding)
+    float z2 = 0.0f, reach = 0.0f, big[C];
+    bool good = true;
+#pragma unroll
+    for (int k = 0; k < C; ++k) big[k] = 0.0f;
+    for (long i = i0 + lane; i < i1; i += 32) {
+        const double nu = a.nu[i];
+        const float d = fabsf(float(nu - c0)), nuf = float(nu);
+        good = good && nu > 0.0;
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const float2 v = yp[size_t(k) * size_t(a.n) + size_t(i)];
+            const float w = nuf * float(a.dpw[g * C + k]);
+            const float re = fmaf(s2, w, d), gam = v.x * w;
+            const float z = fmaf(re, re, gam * gam);
+            const float h = d + (v.x < 15.0f ? (15.0f - v.x) * w : 0.0f);
+            const float A = fabsf(v.y) * w;
+            // (a NaN fails the comparisons)
+            good = good && w > 0.0f && z < 1.0e30f && h < 1.0e30f && A < 1.0e37f;
+            z2 = fmaxf(z2, z);
+            reach = fmaxf(reach, h);
+            big[k] = fmaxf(big[k], A);
+        }
+    }
+    // non-negative floats order as their bit patterns
+    auto warp_max = [](float v) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v))); };
+    z2 = warp_max(z2);
+    reach = warp_max(reach);
+    const float q = sqrtf(z2) * 1.000001f;
+    good = __all_sync(0xffffffffu, good) && q > 0.0f;
+    const size_t at = size_t(g) * size_t(a.ncell) + size_t(cell);
+    if (lane == 0) {
+        CellHead h;
+        h.c0 = c0;
+        // two grid steps beyond the regions: their intervals are placed on the
+        // analytic grid, the tiles by the grid's own values
+        h.dmin = good ? fmaxf(kCellKappa * q * 1.000001f, reach * 1.000002f + __double2float_ru(2.0 * a.df))
+                      : __int_as_float(0x7f800000);
+        h.q = q;
+        a.head[at] = h;
+    }
+    if (!good) return;
+    const double rq = 1.0 / double(q);
+    double* M = a.mom + at * size_t(PM * C);
+#pragma unroll 1
+    for (int k = 0; k < C; ++k) {
+        float bk = 0.0f;
+#pragma unroll
+        for (int j = 0; j < C; ++j) bk = j == k ? big[j] : bk;
+        bk = warp_max(bk);
+        const float rb = bk > 0.0f ? 1.0f / bk : 0.0f;
+        const double wq = a.dpw[g * C + k] * rq;
+        float2 m[PM];
+#pragma unroll
+        for (int j = 0; j < PM; ++j) m[j] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+        for (long i = i0 + lane; i < i1; i += 32) {
+            const float2 v = yp[size_t(k) * size_t(a.n) + size_t(i)];
+            const double nu = a.nu[i];
+            const float w = float(nu * wq), d = float((nu - c0) * rq);  // in units of q
+            // |c pref| w / big <= 1, through nu dpw as above
+            const float A = v.y * (float(nu) * float(a.dpw[g * C + k])) * rb;
+            const float s = s2 * w, gam = v.x * w, g2 = gam * gam;
+            // I_k = A Im(zeta^k) of both poles by
+            // I_{k+1} = 2 Re(zeta) I_k - |zeta|^2 I_{k-1}
+            const float p = d + s, n = d - s;
+            const float2 r2 = make_float2(2.0f * p, 2.0f * n);
+            const float2 nn = make_float2(-fmaf(p, p, g2), -fmaf(n, n, g2));
+            float2 u0 = make_float2(0.0f, 0.0f), u1 = make_float2(A * gam, A * gam);
+#pragma unroll
+            for (int j = 0; j < PM; ++j) {
+                m[j] = __fadd2_rn(m[j], u1);
+                const float2 u = __ffma2_rn(r2, u1, __fmul2_rn(nn, u0));
+                u0 = u1;
+                u1 = u;
+            }
+        }
+        // sums over the lanes in FP64: lane L ends with moment L & 15
+        double t[PM];
+#pragma unroll
+        for (int j = 0; j < PM; ++j) t[j] = double(m[j].x) + double(m[j].y);
+#pragma unroll
+        for (int w = PM / 2; w >= 1; w >>= 1) {
+            const bool up = (lane & w) != 0;
+#pragma unroll
+            for (int i = 0; i < w; ++i) {
+                const double got = __shfl_xor_sync(0xffffffffu, up ? t[i] : t[i + w], w);
+                t[i] = (up ? t[i + w] : t[i]) + got;
+            }
+        }
+        t[0] += __shfl_xor_sync(0xffffffffu, t[0], 16);
+        // A stands for c pref w / big; the series wants c pref w / (2 q)
+        if (lane < PM) M[size_t(lane) * C + k] = t[0] * (0.5 * double(bk) * rq);
+    }
+}
+
 template <bool MIXED>
 cudaError_t run_cells(const CellArgs& a, cudaStream_t st) {
     const dim3 grid(unsigned((a.ncell + kCellWarps - 1) / kCellWarps),
                     unsigned(a.group > 1 ? a.ncond / a.group : a.ncond));
+    auto go = [&](auto c) {
+        constexpr int C = decltype(c)::value;
+        if constexpr (MIXED) k_cells_f32<C><<<grid, kCellWarps * 32, 0, st>>>(a);
+        else k_cells<false, true, C><<<grid, kCellWarps * 32, 0, st>>>(a);
+    };
     switch (a.group) {
         case 0: k_cells<MIXED, false, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
-        case 1: k_cells<MIXED, true, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
-        case 2: k_cells<MIXED, true, 2><<<grid, kCellWarps * 32, 0, st>>>(a); break;
-        case 4: k_cells<MIXED, true, 4><<<grid, kCellWarps * 32, 0, st>>>(a); break;
-        case 8: k_cells<MIXED, true, 8><<<grid, kCellWarps * 32, 0, st>>>(a); break;
+        case 1: go(std::integral_constant<int, 1>()); break;
+        case 2: go(std::integral_constant<int, 2>()); break;
+        case 4: go(std::integral_constant<int, 4>()); break;
+        case 8: go(std::integral_constant<int, 8>()); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

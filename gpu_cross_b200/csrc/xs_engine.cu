@@ -591,9 +591,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Single mixed conditions with cells: lane = line, 32-point tiles.
     const bool near = mixed && C == 1 && narrow_tiles && cells;
     const int CG = near || C > 1 ? C : 0;
-    // Rows of 8 points and 4 lines at a time where a 32-point row is wider than
+    // Rows of 8 points, several lines at a time, where a 32-point row is wider than
     // what has to be taken line by line beside it (about 6 cells).
-    const int LS = C > 1 && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid) ? 4 : 1;
+    const int row = C > 1 && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid) ? 8 : 32;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
         return fail(XS_ERR_INVALID, "line_splits must be 0 (automatic) .. 64");
 
@@ -605,7 +605,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
     if (near) W = 4;
     int occ = near ? steptwo_near_blocks_per_sm()
-              : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, LS)
+              : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, row)
                    : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
     if (occ < 1) {
         // e.g. 8 FP64 conditions per warp with 8 warps: more shared memory
@@ -622,7 +622,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // different warps -- enough for about 16 items per resident warp, at
     // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
-    const int tile_pts = near ? 32 : CG ? 32 / LS : 32 * P;
+    const int tile_pts = near ? 32 : CG ? row : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
@@ -938,7 +938,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
         err = near ? launch_steptwo_near(blocks, sa, st)
-              : CG ? launch_steptwo_mc(mixed, CG, W, LS, blocks, sa, st)
+              : CG ? launch_steptwo_mc(mixed, CG, W, row, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);
         if (err != cudaSuccess) return cuda_fail(err, "step two launch");
         if (blocks > 0 && sa.n_items > 0) ++launched;

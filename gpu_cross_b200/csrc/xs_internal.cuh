@@ -118,8 +118,8 @@ struct __align__(16) LineShX {
     float dfn;    // df / nu (one condition: df g)
     float rn;     // (nu - f0 - m df) / nu (one condition: times g)
     int flags;    // kLineWhole: X from nu in FP64 and every pair of the line
-                  // tested; kLineWide: region-I products need the scaled
-                  // shared reciprocal
+                  // tested; kLineWide: region-I products may leave the FP32
+                  // range, a reciprocal per pair
     int lo, hi;   // window [lo, hi) of grid indices
     double nu;    // centre (whole lines)
 };
@@ -406,9 +406,9 @@ cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stre
 int steptwo_near_blocks_per_sm();
 
 // Multi-condition step two (Voigt): C conditions per warp.
-// LS lane subsets share a row of 32 / LS points (LS = 1 or 4).
-cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
+// Rows of `row` = 32 or 8 points.
+cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int row, int blocks, const StepArgs& a,
                               cudaStream_t stream);
-int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int LS);
+int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int row);
 
 }  // namespace xs

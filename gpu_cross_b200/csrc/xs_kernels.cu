@@ -34,15 +34,9 @@ constexpr int kStages = 3;
 // per-pair path, x from its FP64 centre ("whole" lines): FP32 offsets and
 // the region-I sums are exact enough below it.
 constexpr double kWholeXMax = 1.0e8;
-// Scale of the shared-reciprocal products of the region-I rational (2^-100).
-// Where step two evaluates it (u >= 1), the denominators d = u^2 + 2 y^2
-// lie in [1, 1e32] (|x| < 1e8 for lines that are not whole), so tau d lies
-// in [7.9e-31, 79], tau dA dB in [7.9e-31, 7.9e33] and its reciprocal in
-// [1.3e-34, 1.3e30]: all normal FP32 numbers.
-constexpr float kPairTau = 7.88860905221011805e-31f;
 // Lines whose x^2 + y^2 stays below kPairUMax over their tiles and whose
 // |Pc| stays below kPairPcMax, for every condition of the group ("narrow"
-// lines, the usual case), share reciprocals without the scaling: their
+// lines, the usual case), share reciprocals between two lines or points: their
 // denominators lie in [1, 6.3e18], so dA dB lies in [1, 4e37] and its
 // reciprocal is a normal FP32 number, and the numerators |Pc (u + 1)| stay
 // below 2.5e17, so the cross products nA dB of two lines stay below 1.6e36
@@ -940,38 +934,44 @@ __device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M
     run(r.fc, r.fd);
 }
 
-// The same for one point and the C conditions of a group; the warp's LS lane
-// subsets (sub = this lane's) take every LS-th cell.
-template <int C, int PM, int LS>
+// The same for one point and N of the C conditions of a group (M: at the first of
+// them); the warp's LS lane subsets (sub = this lane's) take every LS-th cell.
+template <int C, int N, int PM, int LS = 1>
 __device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
-                                                 int sub, float bits, double ftlo, double fthi, double f,
-                                                 double (&v)[C]) {
-    auto run = [&](int c0, int c1) {
-        for (int b = c0 + s * LS; b < c1; b += S * LS) {
+                                                 float bits, double ftlo, double fthi, double f, double (&v)[N],
+                                                 int sub = 0) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const int c1 = h ? r.fd : r.fb;
+#pragma unroll 1
+        for (int b = (h ? r.fc : r.fa) + s * LS; b < c1; b += S * LS) {
             const int c = min(b + sub, c1 - 1);
-            const CellHead h = H[c];
-            int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
+            const CellHead hd = H[c];
+            int np = cell_terms<PM>(bits, fmax(ftlo - hd.c0, hd.c0 - fthi), hd.q);
             if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
-            const double2* m = reinterpret_cast<const double2*>(M + size_t(c) * PM * C);
-            const double t = double(h.q) * rcp_newton2_f64(f - h.c0);
-            double a[C];
+            const double* m = M + size_t(c) * (PM * C);
+            const double t = double(hd.q) * rcp_newton2_f64(f - hd.c0);
+            double a[N];
 #pragma unroll
-            for (int q = 0; q < C; ++q) a[q] = 0.0;
+            for (int q = 0; q < N; ++q) a[q] = 0.0;
+#pragma unroll 2
             for (int k = np - 1; k >= 0; --k) {
+                if constexpr (N % 2 == 0) {
 #pragma unroll
-                for (int q = 0; q < C; q += 2) {
-                    const double2 mk = __ldg(m + (k * C + q) / 2);
-                    a[q] = fma(a[q], t, mk.x);
-                    a[q + 1] = fma(a[q + 1], t, mk.y);
+                    for (int q = 0; q < N; q += 2) {
+                        const double2 mk = __ldg(reinterpret_cast<const double2*>(m + k * C + q));
+                        a[q] = fma(a[q], t, mk.x);
+                        a[q + 1] = fma(a[q + 1], t, mk.y);
+                    }
+                } else {
+                    a[0] = fma(a[0], t, __ldg(m + k * C));
                 }
             }
             const double t2 = b + sub < c1 ? t * t : 0.0;
 #pragma unroll
-            for (int q = 0; q < C; ++q) v[q] = fma(a[q], t2, v[q]);
+            for (int q = 0; q < N; ++q) v[q] = fma(a[q], t2, v[q]);
         }
-    };
-    run(r.fa, r.fb);
-    run(r.fc, r.fd);
+    }
 }
 
 // Sum of v over the warp's LS lane subsets, to every lane.
@@ -1724,8 +1724,8 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
             __syncwarp();
         }
         if (runs.fa < runs.fb || runs.fc < runs.fd)
-            add_far_cells_mc<C, kCellTerms64, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs,
-                                                  a.splits, split, sub, kCellBits64, F[t0], F[tl], fj, accd);
+            add_far_cells_mc<C, C, kCellTerms64, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs,
+                                                     a.splits, split, kCellBits64, F[t0], F[tl], fj, accd, sub);
 #pragma unroll
         for (int c = 0; c < C; ++c) accd[c] = sum_subsets<LS>(accd[c]);
         // W4 regions II-IV (point p of the row in lane p)
@@ -1760,71 +1760,119 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
 // ---------------------------------------------------------------------------
 // Mixed-precision multi-condition step two (Voigt), packed FP32x2.
 //
-// Work items, line runs and the fixed summation order are those of
-// k_steptwo_voigt_mc.  Per (line, point) one condition-free offset
-// X = (m - j) dfn + rn and X^2 are formed; conditions are then taken in
-// pairs, each pair one packed FP32x2 operation per step of the region-I
-// rational (u = X^2 k^2 + Cy, u^2 + D2, Pc (u + 1), accumulate), so a
-// region-I pair costs two FP32 operations and one reciprocal per condition
-// and about three issue slots in all.  The rational is added at every pair
-// of the window except, on core candidates, where u < 1; k_core_mcx adds W4
-// less the rational (where it was added) inside the W4 region intervals
-// (|x| + y < 15, from step one).
+// Work items and line runs are those of k_steptwo_voigt_mc.  Per (line, point)
+// one condition-free offset X = (m - j) dfn + rn and X^2 are formed; conditions
+// are then taken in pairs, each pair one packed FP32x2 operation per step of
+// the region-I rational (u = X^2 k^2 + Cy, u^2 + D2, Pc (u + 1)), two lines
+// sharing one reciprocal.  The rational is added at every pair of the window
+// except, on core candidates, where u < 1; k_core_mcx adds W4 less the rational
+// (where it was added) inside the W4 region intervals (|x| + y < 15, from step
+// one).
 //
-// A row is 32 / LS points; with LS = 4 each lane owns one of 8 points and takes
-// every fourth line, for coarse grids over dense lists: 40 conditions, 1e7
-// lines, 0.1 cm-1 grid -- a 32-point row has 6.4 cm-1 of lines whose windows end
-// in it and 3.2 of its own width beside the 2 near it, an 8-point one 1.6 and
-// 0.8.
+// A row is 64 / LS points; each lane owns two of them and every LS-th line
+// (LS = 2: rows of 32; LS = 8: rows of 8, for coarse grids over dense lists --
+// 40 conditions, 1e7 lines, 0.1 cm-1 grid: a 32-point row has 6.4 cm-1 of lines
+// whose windows end in it and 3.2 of its own width beside the 2 near it, an
+// 8-point one 1.6 and 0.8).  What bounds it is shared memory: a lane needs 24 +
+// 8 C bytes of every line it takes, 128 bytes a wavefront for the warp, so two
+// points per lane halve it, and 2 y^2 comes from Cy = y^2 - 1/2 instead of a
+// third array.  Every LS groups of 32 lines the FP32 sums (16 deep) are added
+// up over the lane subsets by halving exchanges, each lane keeping 2 C / LS of
+// them in FP64.
 // ---------------------------------------------------------------------------
 // Resident blocks per SM the mixed multi-condition kernel asks the compiler
-// to fit: 24 warps per SM (about 80 registers a thread); 28 at 8 conditions
-// and 4 warps per block (72 registers; 7 blocks of 30.7 KB of staging also
-// fit in shared memory), and 16 at 8 conditions and 8 warps per block (124
-// registers) -- the occupancy points the autotuner chooses between through
-// the block size.
+// to fit (register budget): 20 warps per SM at 8 conditions and 4 warps per
+// block, 16 at 8 and 8, 24 otherwise -- the occupancy points the autotuner
+// chooses between through the block size.
 template <int C, int WARPS>
 constexpr int voigt_mcx_min_blocks() {
-    return (C == 8 && WARPS == 8) ? 2 : (C == 8 && WARPS == 4) ? 6 : 24 / WARPS;
+    return (C == 8 && WARPS == 8) ? 2 : (C == 8 && WARPS == 4) ? 5 : 24 / WARPS;
 }
 
 // Region-I constants of a line for the C conditions of its group, in condition
 // order: conditions 2k and 2k+1 are one packed FP32x2 operand, conditions
-// 4k..4k+3 one 16-byte load.  Formed in shared memory from the (y, pref) pairs
+// 4k..4k+3 one 16-byte load.  Formed in shared memory from the (y, c pref) pairs
 // of step one when a group of lines has arrived.
 template <int C>
 struct __align__(C == 2 ? 8 : 16) LineR1 {
-    float Cy[C], D2[C], Pc[C];
+    float Cy[C], Pc[C];
 };
 // (the core pass repeats step two's choice on u = X^2 k^2 + Cy: one definition)
 __device__ __forceinline__ float region1_cy(float y) { return fmaf(y, y, -0.5f); }
+// D2 = 2 y^2 of a packed pair of conditions: within 6e-8 of max(1, 2 y^2), and it
+// is added to u^2 with u >= 1.
+__device__ __forceinline__ float2 region1_d2(float2 cy) { return __ffma2_rn(cy, f2s(2.0f), f2s(1.0f)); }
 
 // Shared memory of one warp: two stages of 32 lines' offsets and flags (16 B),
-// windows (8 B) and (y, pref) (8 B per condition), and 32 lines' constants.
+// windows (8 B) and (y, c pref) (8 B per condition), and 32 lines' constants.
 template <int C>
 constexpr size_t mcx_warp_smem() {
     return 64 * (sizeof(float4) + sizeof(int2) + C * sizeof(float2)) + 32 * sizeof(LineR1<C>);
 }
+
+// Sums w[0..V) over the lane bits 16 .. LP by halving exchanges: a lane ends
+// with the values base .. base + n - 1 of `kept` (fewer values than lanes: every
+// lane of the remaining bits holds the same one).
+template <int V, int LP>
+struct Halving {
+    static constexpr int kKept = V * LP / 32 > 1 ? V * LP / 32 : 1;
+    __device__ static __forceinline__ void sum(float (&w)[V], int lane) {
+        int n = V;
+#pragma unroll
+        for (int o = 16; o >= LP; o >>= 1) {
+            if (n > 1) {
+                n /= 2;
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int i = 0; i < V / 2; ++i)
+                    if (i < n) {
+                        const float got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + n], o);
+                        w[i] = (up ? w[i + n] : w[i]) + got;
+                    }
+            } else {
+                w[0] += __shfl_xor_sync(0xffffffffu, w[0], o);
+            }
+        }
+    }
+    // First of the lane's values, and whether another lane holds the same ones.
+    __device__ static __forceinline__ int base(int lane, bool& copy) {
+        int n = V, at = 0;
+        copy = false;
+#pragma unroll
+        for (int o = 16; o >= LP; o >>= 1) {
+            if (n > 1) {
+                n /= 2;
+                if (lane & o) at += n;
+            } else if (lane & o) {
+                copy = true;
+            }
+        }
+        return at;
+    }
+};
 
 template <int C, int WARPS, int LS>
 __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>()))
     k_steptwo_voigt_mcx(StepArgs a) {
     static_assert(C % 2 == 0, "conditions come in pairs");
     constexpr int NP = C / 2;
+    constexpr int LP = 32 / LS, PT = 2 * LP;  // lane points, points of a row
+    using Sum = Halving<2 * C, LP>;
+    constexpr int VF = Sum::kKept;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     using R1 = LineR1<C>;
     // staged per line: the offsets and flags of LineShX, its window and the
-    // conditions' (y, pref), [condition][line]; a whole line's FP64 centre is
+    // conditions' (y, c pref), [condition][line]; a whole line's FP64 centre is
     // read from memory when needed
     unsigned char* const mine = smem_raw + size_t(warp) * mcx_warp_smem<C>();
     float4* lsb = reinterpret_cast<float4*>(mine);
     R1* SR = reinterpret_cast<R1*>(mine + 64 * sizeof(float4));
     float2* ypb = reinterpret_cast<float2*>(mine + 64 * sizeof(float4) + 32 * sizeof(R1));
     int2* lhb = reinterpret_cast<int2*>(ypb + 64 * C);
-    constexpr int PT = 32 / LS;  // points of a row
-    const int sub = lane / PT;
+    const int sub = lane / LP;
+    const double* F = a.G.freq;
 
     for (;;) {
         int item = 0;
@@ -1836,8 +1884,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
         const int tile = (item - cg * per_cond) / a.splits;
         const int split = item - cg * per_cond - tile * a.splits;
         const int t0 = a.G.start + tile * PT;
-        const int end = a.G.start + a.G.points;
-        const int t1 = t0 + PT < end ? t0 + PT : end;
+        const int gend = a.G.start + a.G.points;
+        const int t1 = t0 + PT < gend ? t0 + PT : gend;
         const int tl = t1 - 1;
         const size_t wbase = size_t(a.wslot[cg]) * size_t(a.n);  // the group's window data
         const int* whi = a.whi + wbase;
@@ -1847,109 +1895,89 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
 #pragma unroll
         for (int c = 0; c < C; ++c) kc = max(kc, a.kc[cg * C + c]);
         // line indices fit 32 bits (at most 2^31 - 1 lines per call)
-        const int La = int(warp_lower_bound(0, a.n, lane, [&](long i) { return whi[i] > t0; }));
-        const int Lb = int(warp_lower_bound(La, a.n, lane, [&](long i) { return wlo[i] >= t1; }));
-        const int fs = int(warp_lower_bound(La, Lb, lane, [&](long i) { return whi[i] >= t1; }));
-        const int Cb = int(warp_lower_bound(La, Lb, lane, [&](long i) { return wlo[i] > t0; }));
+        const int La = warp_search(whi, 0, int(a.n), t0 + 1, lane);
+        const int Lb = warp_search(wlo, La, int(a.n), t1, lane);
+        const int fs = warp_search(whi, La, Lb, t1, lane);
+        const int Cb = warp_search(wlo, La, Lb, t0 + 1, lane);
         const int fe = Cb > fs ? Cb : fs;
         // core candidates [E, Fc): the lines whose near-centre pairs may
         // fall in the tile (kc: the group's widest reach plus one; 0: no
         // line of the group has such pairs)
         int E = La, Fc = La;
         if (kc > 0) {
-            E = int(warp_lower_bound(La, Lb, lane, [&](long i) { return mi[i] >= t0 - (kc - 1); }));
-            Fc = int(warp_lower_bound(E, Lb, lane, [&](long i) { return mi[i] > tl + (kc - 1); }));
+            E = warp_search(mi, La, Lb, t0 - (kc - 1), lane);
+            Fc = warp_search(mi, E, Lb, tl + kc, lane);
         }
         const LineShX* lsh = reinterpret_cast<const LineShX*>(a.lsh) + wbase;
         const float2* yp = a.cyp + size_t(cg) * C * size_t(a.n);
-
-        const double* F = a.G.freq;
         const size_t cell0 = size_t(cg) * size_t(a.ncell);
         const LineRuns runs =
             line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
 
-        const int jj = t0 + lane % PT;
-        const float jf = float(jj);
+        const int j0 = t0 + lane % LP, j1 = j0 + LP;  // this lane's points
+        const float jf0 = float(j0), jf1 = float(j1);
         float2 k2[NP];
-        float2 acc[NP], sum[NP], cmp[NP];
+        float2 acc[2][NP];
+        double sum[VF];
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
             k2[p] = f2(a.kx2[cg * C + 2 * p], a.kx2[cg * C + 2 * p + 1]);
-            acc[p] = sum[p] = cmp[p] = f2(0.0f, 0.0f);
+            acc[0][p] = acc[1][p] = f2(0.0f, 0.0f);
         }
+#pragma unroll
+        for (int v = 0; v < VF; ++v) sum[v] = 0.0;
 
-        // Region I of one pair of conditions: u = X^2 k^2 + Cy,
-        // acc += Pc (u + 1) / (u^2 + D2).  Pairs where `keep` is false add
-        // exactly zero: the reciprocal is replaced by 0 (not multiplied by a
-        // mask, so that an infinite reciprocal of a skipped pair never
-        // reaches the sum).  MODE 0: plain; 1: the product itself is selected,
-        // for lines whose u may overflow; 2: as 1, and a pair is kept only
-        // where u >= 1 (core candidates: the core pass takes u < 1).
-        auto region1 = [&](auto mode, float X2, const R1& r, int p, bool keep0, bool keep1) {
-            constexpr int MODE = decltype(mode)::value;
+        // Two narrow lines A, B that are not core candidates, at once: per
+        // condition one reciprocal for both lines, to += (nA dB + nB dA)
+        // / (dA dB) (u >= 1 on such lines, so dA, dB >= 1; narrow lines
+        // keep dA dB and the products with Pc in range, kPairUMax).  inA,
+        // inB: the point takes the line (a line left out adds exactly 0).
+        auto pair_step = [&](float XA2, float XB2, float2 cyA, float2 d2A, float2 pcA, float2 cyB, float2 d2B,
+                             float2 pcB, int p, bool inA, bool inB, float2& to) {
+            const float2 uA = __ffma2_rn(f2s(XA2), k2[p], cyA);
+            const float2 uB = __ffma2_rn(f2s(XB2), k2[p], cyB);
+            const float2 dA = __ffma2_rn(uA, uA, d2A);
+            const float2 dB = __ffma2_rn(uB, uB, d2B);
+            float2 nA = __ffma2_rn(uA, pcA, pcA);
+            float2 nB = __ffma2_rn(uB, pcB, pcB);
+            if (!inA) nA = f2(0.0f, 0.0f);
+            if (!inB) nB = f2(0.0f, 0.0f);
+            const float2 q = __fmul2_rn(dA, dB);
+            const float2 sn = __ffma2_rn(nB, dA, __fmul2_rn(nA, dB));
+            to = __ffma2_rn(sn, f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)), to);
+        };
+        // One line (wide, whole or a core candidate, or any in their company)
+        // at one point: a reciprocal per pair.  NEAR: a pair is kept only where
+        // u >= 1 (core candidates: the core pass takes u < 1).  Pc / u to FP32
+        // rounding from u = 1e12 on (u^2 overflows from 1.8e19); beyond x = 1e18
+        // region I is taken as 0.  A pair that is left out adds exactly 0: the
+        // product itself is selected, so an infinite reciprocal never counts.
+        auto line_step = [&](bool near, float X, const R1& r, int p, bool in, float2& to) {
             const float2 cy = *reinterpret_cast<const float2*>(&r.Cy[2 * p]);
-            const float2 d2 = *reinterpret_cast<const float2*>(&r.D2[2 * p]);
             const float2 pc = *reinterpret_cast<const float2*>(&r.Pc[2 * p]);
-            const float2 u = __ffma2_rn(f2(X2, X2), k2[p], cy);
-            if constexpr (MODE == 2) {
-                keep0 = keep0 && !(u.x < 1.0f);
-                keep1 = keep1 && !(u.y < 1.0f);
-            }
-            float2 den = __ffma2_rn(u, u, d2);
+            const float2 u = __ffma2_rn(f2s(X * X), k2[p], cy);
+            float2 den = __ffma2_rn(u, u, region1_d2(cy));
             float2 num = __ffma2_rn(u, pc, pc);
-            if constexpr (MODE >= 1) {
-                // Pc / u to FP32 rounding, and u^2 overflows from 1.8e19
-                if (u.x > 1.0e12f) den.x = u.x, num.x = pc.x;
-                if (u.y > 1.0e12f) den.y = u.y, num.y = pc.y;
-            }
-            const float2 rr = f2(keep0 ? rcp_approx_f32(den.x) : 0.0f, keep1 ? rcp_approx_f32(den.y) : 0.0f);
-            if constexpr (MODE >= 1) {
-                acc[p].x += keep0 ? num.x * rr.x : 0.0f;
-                acc[p].y += keep1 ? num.y * rr.y : 0.0f;
-            } else {
-                acc[p] = __ffma2_rn(num, rr, acc[p]);
-            }
+            if (u.x > 1.0e12f) den.x = u.x, num.x = pc.x;
+            if (u.y > 1.0e12f) den.y = u.y, num.y = pc.y;
+            const float aX = fabsf(X);
+            const bool k0 = in && !(near && u.x < 1.0f) && aX * a.kx[cg * C + 2 * p] < 1.0e18f;
+            const bool k1 = in && !(near && u.y < 1.0f) && aX * a.kx[cg * C + 2 * p + 1] < 1.0e18f;
+            to.x += k0 ? num.x * rcp_approx_f32(den.x) : 0.0f;
+            to.y += k1 ? num.y * rcp_approx_f32(den.y) : 0.0f;
         };
-        const std::integral_constant<int, 0> plain;
-        const std::integral_constant<int, 2> guarded_near;
-        // Region I of two pairs of conditions (A, B) of a wide line with one
-        // reciprocal per two line-evals: lane h of A and lane h of B share
-        // 1 / (dA dB), so 1/dA = dB / (dA dB) and 1/dB = dA / (dA dB), both
-        // factors scaled by kPairTau first: 1/dA = (tau dB) / (tau dA dB).
-        // pA = 2q, pB = 2q + 1: conditions 4q..4q+3, one 16-byte load for each
-        // of Cy, D2 and Pc.  Pairs where `keep` is false add exactly zero.
-        auto region1_ab = [&](float X2, const R1& r, int pA, int pB, bool keep) {
-            const float4 cy = *reinterpret_cast<const float4*>(&r.Cy[2 * pA]);
-            const float4 d2 = *reinterpret_cast<const float4*>(&r.D2[2 * pA]);
-            const float4 pc = *reinterpret_cast<const float4*>(&r.Pc[2 * pA]);
-            const float2 uA = __ffma2_rn(f2(X2, X2), k2[pA], f2(cy.x, cy.y));
-            const float2 uB = __ffma2_rn(f2(X2, X2), k2[pB], f2(cy.z, cy.w));
-            const float2 dA = __ffma2_rn(uA, uA, f2(d2.x, d2.y));
-            const float2 dB = __ffma2_rn(uB, uB, f2(d2.z, d2.w));
-            const float2 nA = __ffma2_rn(uA, f2(pc.x, pc.y), f2(pc.x, pc.y));
-            const float2 nB = __ffma2_rn(uB, f2(pc.z, pc.w), f2(pc.z, pc.w));
-            const float2 aA = __fmul2_rn(dA, f2s(kPairTau));
-            const float2 bB = __fmul2_rn(dB, f2s(kPairTau));
-            const float2 q = __fmul2_rn(aA, dB);
-            const float2 rq = keep ? f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)) : f2(0.0f, 0.0f);
-            acc[pA] = __ffma2_rn(nA, __fmul2_rn(bB, rq), acc[pA]);
-            acc[pB] = __ffma2_rn(nB, __fmul2_rn(aA, rq), acc[pB]);
-        };
-        // region1_ab for a narrow core-candidate line: a condition's pair is
-        // kept where the point takes the line (`in`) and u >= 1 (the core
-        // pass takes u < 1); a pair that is not kept enters the shared
-        // product as 1 and adds exactly zero, so the kept ones keep their
-        // ranges.
-        auto region1_ab_near = [&](float X2, const R1& r, int pA, int pB, bool in) {
-            const float4 cy = *reinterpret_cast<const float4*>(&r.Cy[2 * pA]);
-            const float4 d2 = *reinterpret_cast<const float4*>(&r.D2[2 * pA]);
-            const float4 pc = *reinterpret_cast<const float4*>(&r.Pc[2 * pA]);
-            const float2 uA = __ffma2_rn(f2(X2, X2), k2[pA], f2(cy.x, cy.y));
-            const float2 uB = __ffma2_rn(f2(X2, X2), k2[pB], f2(cy.z, cy.w));
+        // A narrow core candidate at one point, two pairs of conditions with one
+        // reciprocal per two evaluations: a condition's pair is kept where the
+        // point takes the line (`in`) and u >= 1; a pair that is not kept enters
+        // the shared product as 1 and adds exactly zero.
+        auto near_step = [&](float X2, const float4& cy, const float4& pc, int p, bool in, float2& toA, float2& toB) {
+            const float2 cA = f2(cy.x, cy.y), cB = f2(cy.z, cy.w);
+            const float2 uA = __ffma2_rn(f2s(X2), k2[p], cA);
+            const float2 uB = __ffma2_rn(f2s(X2), k2[p + 1], cB);
             const bool q0 = in && !(uA.x < 1.0f), q1 = in && !(uA.y < 1.0f);
             const bool q2 = in && !(uB.x < 1.0f), q3 = in && !(uB.y < 1.0f);
-            const float2 dA0 = __ffma2_rn(uA, uA, f2(d2.x, d2.y));
-            const float2 dB0 = __ffma2_rn(uB, uB, f2(d2.z, d2.w));
+            const float2 dA0 = __ffma2_rn(uA, uA, region1_d2(cA));
+            const float2 dB0 = __ffma2_rn(uB, uB, region1_d2(cB));
             const float2 nA = __ffma2_rn(uA, f2(pc.x, pc.y), f2(pc.x, pc.y));
             const float2 nB = __ffma2_rn(uB, f2(pc.z, pc.w), f2(pc.z, pc.w));
             const float2 dA = f2(q0 ? dA0.x : 1.0f, q1 ? dA0.y : 1.0f);
@@ -1958,8 +1986,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             const float2 rq = f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y));
             const float2 iA = __fmul2_rn(dB, rq);
             const float2 iB = __fmul2_rn(dA, rq);
-            acc[pA] = __ffma2_rn(nA, f2(q0 ? iA.x : 0.0f, q1 ? iA.y : 0.0f), acc[pA]);
-            acc[pB] = __ffma2_rn(nB, f2(q2 ? iB.x : 0.0f, q3 ? iB.y : 0.0f), acc[pB]);
+            toA = __ffma2_rn(nA, f2(q0 ? iA.x : 0.0f, q1 ? iA.y : 0.0f), toA);
+            toB = __ffma2_rn(nB, f2(q2 ? iB.x : 0.0f, q3 ? iB.y : 0.0f), toB);
         };
 
         const int ngroups = runs.groups_of(a.splits, split);
@@ -1969,27 +1997,21 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             end = int(e);
             return b;
         };
-        auto stage_group = [&](int bufi, int b, int cnt) {
-            if (lane < cnt) {
+        auto stage_group = [&](int gi) {
+            int end;
+            const int b = gstart(gi, end), bufi = gi & 1;
+            if (b + lane < end) {
                 cp_async16(lsb + bufi * 32 + lane, lsh + b + lane);
                 cp_async8(lhb + bufi * 32 + lane, &lsh[b + lane].lo);
 #pragma unroll
                 for (int c = 0; c < C; ++c) cp_async8(ypb + (bufi * C + c) * 32 + lane, yp + size_t(c) * size_t(a.n) + b + lane);
             }
-        };
-        if (ngroups > 0) {
-            int end;
-            const int b = gstart(0, end);
-            stage_group(0, b, end - b < 32 ? end - b : 32);
             cp_async_commit();
-        }
+        };
+        if (ngroups > 0) stage_group(0);
         for (int gi = 0; gi < ngroups; ++gi) {
             if (gi + 1 < ngroups) {
-                int end;
-                const int b = gstart(gi + 1, end);
-                const int rem = end - b;
-                stage_group((gi + 1) & 1, b, rem < 32 ? rem : 32);
-                cp_async_commit();
+                stage_group(gi + 1);
                 cp_async_wait<1>();
             } else {
                 cp_async_wait<0>();
@@ -2005,9 +2027,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                 for (int c = 0; c < C; c += 2) {
                     const float2 v0 = ypb[((gi & 1) * C + c) * 32 + lane], v1 = ypb[((gi & 1) * C + c + 1) * 32 + lane];
                     *reinterpret_cast<float2*>(&r.Cy[c]) = f2(region1_cy(v0.x), region1_cy(v1.x));
-                    *reinterpret_cast<float2*>(&r.D2[c]) = f2(2.0f * v0.x * v0.x, 2.0f * v1.x * v1.x);
-                    *reinterpret_cast<float2*>(&r.Pc[c]) =
-                        f2(v0.y * v0.x, v1.y * v1.x);
+                    *reinterpret_cast<float2*>(&r.Pc[c]) = f2(v0.y * v0.x, v1.y * v1.x);
                 }
             }
             __syncwarp();
@@ -2016,63 +2036,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             const int ge = end - gb < 32 ? end : gb + 32;
             auto lo_of = [&](int v) { return (v < gb ? gb : (v > ge ? ge : v)) - gb; };
             const int b1 = lo_of(E), c1 = lo_of(Fc);  // the core candidates
-            // One line's region I at this lane's point, conditions in pairs
-            // of pairs (keep: the point takes the line).
-            auto line_region1 = [&](float X2, const R1& r, bool keep) {
-                if constexpr (NP % 2 == 0) {
-#pragma unroll
-                    for (int p = 0; p < NP; p += 2) region1_ab(X2, r, p, p + 1, keep);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) region1(plain, X2, r, p, keep, keep);
-                }
-            };
-            // Two narrow lines A, B that are not core candidates, at once: per
-            // condition one reciprocal for both lines, acc += (nA dB + nB dA)
-            // / (dA dB) (u >= 1 on such lines, so dA, dB >= 1; narrow lines
-            // keep dA dB and the products with Pc in range, kPairUMax).  inA,
-            // inB: the point takes the line (a line left out adds exactly 0).
-            auto pair_step = [&](float XA2, float XB2, float2 cyA, float2 d2A, float2 pcA, float2 cyB,
-                                 float2 d2B, float2 pcB, int p, bool inA, bool inB) {
-                const float2 uA = __ffma2_rn(f2(XA2, XA2), k2[p], cyA);
-                const float2 uB = __ffma2_rn(f2(XB2, XB2), k2[p], cyB);
-                const float2 dA = __ffma2_rn(uA, uA, d2A);
-                const float2 dB = __ffma2_rn(uB, uB, d2B);
-                float2 nA = __ffma2_rn(uA, pcA, pcA);
-                float2 nB = __ffma2_rn(uB, pcB, pcB);
-                if (!inA) nA = f2(0.0f, 0.0f);
-                if (!inB) nB = f2(0.0f, 0.0f);
-                const float2 q = __fmul2_rn(dA, dB);
-                const float2 sn = __ffma2_rn(nB, dA, __fmul2_rn(nA, dB));
-                acc[p] = __ffma2_rn(sn, f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)), acc[p]);
-            };
-            auto pair_region1 = [&](float XA2, float XB2, const R1& ra, const R1& rb, bool inA, bool inB) {
-                if constexpr (NP % 2 == 0) {
-                    // conditions 4q..4q+3: one 16-byte load per array and line
-#pragma unroll
-                    for (int p = 0; p < NP; p += 2) {
-                        const float4 cyA = *reinterpret_cast<const float4*>(&ra.Cy[2 * p]);
-                        const float4 d2A = *reinterpret_cast<const float4*>(&ra.D2[2 * p]);
-                        const float4 pcA = *reinterpret_cast<const float4*>(&ra.Pc[2 * p]);
-                        const float4 cyB = *reinterpret_cast<const float4*>(&rb.Cy[2 * p]);
-                        const float4 d2B = *reinterpret_cast<const float4*>(&rb.D2[2 * p]);
-                        const float4 pcB = *reinterpret_cast<const float4*>(&rb.Pc[2 * p]);
-                        pair_step(XA2, XB2, f2(cyA.x, cyA.y), f2(d2A.x, d2A.y), f2(pcA.x, pcA.y), f2(cyB.x, cyB.y),
-                                  f2(d2B.x, d2B.y), f2(pcB.x, pcB.y), p, inA, inB);
-                        pair_step(XA2, XB2, f2(cyA.z, cyA.w), f2(d2A.z, d2A.w), f2(pcA.z, pcA.w), f2(cyB.z, cyB.w),
-                                  f2(d2B.z, d2B.w), f2(pcB.z, pcB.w), p + 1, inA, inB);
-                    }
-                } else {
-#pragma unroll
-                    for (int p = 0; p < NP; ++p)
-                        pair_step(XA2, XB2, *reinterpret_cast<const float2*>(&ra.Cy[2 * p]),
-                                  *reinterpret_cast<const float2*>(&ra.D2[2 * p]),
-                                  *reinterpret_cast<const float2*>(&ra.Pc[2 * p]),
-                                  *reinterpret_cast<const float2*>(&rb.Cy[2 * p]),
-                                  *reinterpret_cast<const float2*>(&rb.D2[2 * p]),
-                                  *reinterpret_cast<const float2*>(&rb.Pc[2 * p]), p, inA, inB);
-                }
-            };
             // Lines [x, y) that are not core candidates, two at a time, the
             // window as a lane mask.  Lane subset `sub` takes lines x + sub,
             // x + sub + LS, ...; a lane past the run's end takes its last line
@@ -2084,100 +2047,110 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                 const int x = h ? c1 : 0, y = h ? ge - gb : b1;
 #pragma unroll 1
                 for (int b = x; b < y; b += 2 * LS) {
-                    const int tA = LS > 1 ? min(b + sub, y - 1) : b, tB = min(b + sub + LS, y - 1);
+                    const int tA = min(b + sub, y - 1), tB = min(b + sub + LS, y - 1);
                     const float4 sA = SL[tA];
                     const float4 sB = SL[tB];
                     const int2 wA = SW[tA], wB = SW[tB];
-                    const float XA = fmaf(sA.x - jf, sA.y, sA.z);
-                    const float XB = fmaf(sB.x - jf, sB.y, sB.z);
+                    const float XA0 = fmaf(sA.x - jf0, sA.y, sA.z), XA1 = fmaf(sA.x - jf1, sA.y, sA.z);
+                    const float XB0 = fmaf(sB.x - jf0, sB.y, sB.z), XB1 = fmaf(sB.x - jf1, sB.y, sB.z);
                     const bool wide = ((__float_as_int(sA.w) | __float_as_int(sB.w)) & kLineWide) != 0;
-                    const bool inA = (LS == 1 || b + sub < y) && jj >= wA.x && jj < wA.y;
-                    const bool inB = b + sub + LS < y && jj >= wB.x && jj < wB.y;
-                    if (!(LS > 1 ? __any_sync(0xffffffffu, wide) : wide)) {
-                        pair_region1(XA * XA, XB * XB, SR[tA], SR[tB], inA, inB);
+                    const bool okA = b + sub < y, okB = b + sub + LS < y;
+                    const bool inA0 = okA && j0 >= wA.x && j0 < wA.y, inA1 = okA && j1 >= wA.x && j1 < wA.y;
+                    const bool inB0 = okB && j0 >= wB.x && j0 < wB.y, inB1 = okB && j1 >= wB.x && j1 < wB.y;
+                    const R1 &rA = SR[tA], &rB = SR[tB];
+                    if (!__any_sync(0xffffffffu, wide)) {
+                        auto both = [&](float2 cyA, float2 pcA, float2 cyB, float2 pcB, int p) {
+                            const float2 d2A = region1_d2(cyA), d2B = region1_d2(cyB);
+                            pair_step(XA0 * XA0, XB0 * XB0, cyA, d2A, pcA, cyB, d2B, pcB, p, inA0, inB0, acc[0][p]);
+                            pair_step(XA1 * XA1, XB1 * XB1, cyA, d2A, pcA, cyB, d2B, pcB, p, inA1, inB1, acc[1][p]);
+                        };
+                        if constexpr (NP % 2 == 0) {
+                            // conditions 4q..4q+3: one 16-byte load per array and line
+#pragma unroll
+                            for (int p = 0; p < NP; p += 2) {
+                                const float4 cyA = *reinterpret_cast<const float4*>(&rA.Cy[2 * p]);
+                                const float4 pcA = *reinterpret_cast<const float4*>(&rA.Pc[2 * p]);
+                                const float4 cyB = *reinterpret_cast<const float4*>(&rB.Cy[2 * p]);
+                                const float4 pcB = *reinterpret_cast<const float4*>(&rB.Pc[2 * p]);
+                                both(f2(cyA.x, cyA.y), f2(pcA.x, pcA.y), f2(cyB.x, cyB.y), f2(pcB.x, pcB.y), p);
+                                both(f2(cyA.z, cyA.w), f2(pcA.z, pcA.w), f2(cyB.z, cyB.w), f2(pcB.z, pcB.w), p + 1);
+                            }
+                        } else {
+                            both(*reinterpret_cast<const float2*>(&rA.Cy[0]), *reinterpret_cast<const float2*>(&rA.Pc[0]),
+                                 *reinterpret_cast<const float2*>(&rB.Cy[0]), *reinterpret_cast<const float2*>(&rB.Pc[0]), 0);
+                        }
                     } else {
-                        // (the scaled form serves narrow lines too)
+#pragma unroll
+                        for (int p = 0; p < NP; ++p)
 #pragma unroll 1
-                        for (int q = 0; q < 2; ++q)
-                            line_region1(q ? XB * XB : XA * XA, SR[q ? tB : tA], q ? inB : inA);
+                            for (int q = 0; q < 2; ++q) {
+                                line_step(false, q ? XB0 : XA0, q ? rB : rA, p, q ? inB0 : inA0, acc[0][p]);
+                                line_step(false, q ? XB1 : XA1, q ? rB : rA, p, q ? inB1 : inA1, acc[1][p]);
+                            }
                     }
                 }
             }
             // Core candidates: region I where u >= 1, per condition (the
             // core pass takes the pairs with u < 1, deciding on the same FP32
             // u).
-            auto cand_run = [&](int x, int y) {
-                for (int b = x; b < y; b += LS) {
-                    const int t = LS > 1 ? min(b + sub, y - 1) : b;
-                    const float4 s = SL[t];
-                    const int flags = __float_as_int(s.w);
-                    const int2 win = SW[t];
-                    const bool in = (LS == 1 || b + sub < y) && jj >= win.x && jj < win.y;
-                    if constexpr (NP % 2 == 0) {
-                        const bool odd = (flags & (kLineWhole | kLineWide)) != 0;
-                        if (!(LS > 1 ? __any_sync(0xffffffffu, odd) : odd)) {
-                            // narrow: the shared reciprocal
-                            const float X = fmaf(s.x - jf, s.y, s.z);
+#pragma unroll 1
+            for (int b = b1; b < c1; b += LS) {
+                const int t = min(b + sub, c1 - 1);
+                const float4 s = SL[t];
+                const int flags = __float_as_int(s.w);
+                const int2 win = SW[t];
+                const bool ok = b + sub < c1;
+                const bool in0 = ok && j0 >= win.x && j0 < win.y, in1 = ok && j1 >= win.x && j1 < win.y;
+                const R1& r = SR[t];
+                if (NP % 2 == 0 && !__any_sync(0xffffffffu, (flags & (kLineWhole | kLineWide)) != 0)) {
+                    const float X0 = fmaf(s.x - jf0, s.y, s.z), X1 = fmaf(s.x - jf1, s.y, s.z);
 #pragma unroll
-                            for (int p = 0; p < NP; p += 2) region1_ab_near(X * X, SR[t], p, p + 1, in);
-                            continue;
-                        }
+                    for (int p = 0; p + 1 < NP; p += 2) {
+                        const float4 cy = *reinterpret_cast<const float4*>(&r.Cy[2 * p]);
+                        const float4 pc = *reinterpret_cast<const float4*>(&r.Pc[2 * p]);
+                        near_step(X0 * X0, cy, pc, p, in0, acc[0][p], acc[0][p + 1]);
+                        near_step(X1 * X1, cy, pc, p, in1, acc[1][p], acc[1][p + 1]);
                     }
-                    // whole lines: X from the FP64 centre (rare; the grid
-                    // value is read here rather than held for every line)
-                    double nu = 0.0;
-                    if (flags & kLineWhole) nu = lsh[gb + t].nu;
-                    const float X = (flags & kLineWhole) ? float((nu - a.G.freq[jj < t1 ? jj : tl]) / nu)
-                                                         : fmaf(s.x - jf, s.y, s.z);
-                    const float X2 = X * X;
-                    const float aX = fabsf(X);
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) {
-                        bool keep[2];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int c = 2 * p + h;
-                            // beyond x = 1e18 region I is taken as 0
-                            keep[h] = in && aX * a.kx[cg * C + c] < 1.0e18f;
-                        }
-                        region1(guarded_near, X2, SR[t], p, keep[0], keep[1]);
-                    }
+                    continue;
                 }
-            };
-            cand_run(b1, c1);
-            // compensated (Kahan) fold of this group's FP32 partials
-            auto kahan = [](float part, float& sm, float& cm) {
-                const float yk = part - cm;
-                const float tk = sm + yk;
-                cm = (tk - sm) - yk;
-                sm = tk;
-            };
-            // (LS groups are 32 lines of each lane)
-            if (LS == 1 || (gi & (LS - 1)) == LS - 1 || gi + 1 == ngroups) {
+                // whole lines: X from the FP64 centre (rare; the grid value is
+                // read here rather than held for every line)
+                double nu = 0.0;
+                if (flags & kLineWhole) nu = lsh[gb + t].nu;
+                const float X0 = (flags & kLineWhole) ? float((nu - F[min(j0, tl)]) / nu) : fmaf(s.x - jf0, s.y, s.z);
+                const float X1 = (flags & kLineWhole) ? float((nu - F[min(j1, tl)]) / nu) : fmaf(s.x - jf1, s.y, s.z);
 #pragma unroll
                 for (int p = 0; p < NP; ++p) {
-                    kahan(acc[p].x, sum[p].x, cmp[p].x);
-                    kahan(acc[p].y, sum[p].y, cmp[p].y);
-                    acc[p] = f2(0.0f, 0.0f);
+                    line_step(true, X0, r, p, in0, acc[0][p]);
+                    line_step(true, X1, r, p, in1, acc[1][p]);
                 }
+            }
+            if ((gi & (LS - 1)) == LS - 1 || gi + 1 == ngroups) {
+                float w[2 * C];
+#pragma unroll
+                for (int v = 0; v < C; ++v) {
+                    const float2 x = acc[v / NP][v % NP];  // values 2 v, 2 v + 1
+                    w[2 * v] = x.x;
+                    w[2 * v + 1] = x.y;
+                    acc[v / NP][v % NP] = f2(0.0f, 0.0f);
+                }
+                Sum::sum(w, lane);
+#pragma unroll
+                for (int v = 0; v < VF; ++v) sum[v] += double(w[v]);
             }
             __syncwarp();
         }
-        double v[C];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            v[2 * p] = double(sum[p].x) - double(cmp[p].x);
-            v[2 * p + 1] = double(sum[p].y) - double(cmp[p].y);
-        }
+        // value (point, condition) = point * C + condition
+        bool copy;
+        const int base = Sum::base(lane, copy);
+        const int c0 = base % C, jj = base / C ? j1 : j0;
         if (runs.fa < runs.fb || runs.fc < runs.fd)
-            add_far_cells_mc<C, kCellTermsMixed, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C), runs,
-                                                     a.splits, split, sub, kCellBitsMixed, F[t0], F[tl],
-                                                     F[jj < t1 ? jj : tl], v);
+            add_far_cells_mc<C, VF, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C) + c0, runs,
+                                                     a.splits, split, kCellBitsMixed, F[t0], F[tl],
+                                                     F[jj < t1 ? jj : tl], sum);
+        if (!copy && jj < t1) {
 #pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = sum_subsets<LS>(v[c]);
-        if (sub == 0 && jj < t1) {
-#pragma unroll
-            for (int c = 0; c < C; ++c) put_result(a, cg * C + c, split, jj, v[c]);
+            for (int v = 0; v < VF; ++v) put_result(a, cg * C + c0 + v, split, jj, sum[v]);
         }
     }
 }
@@ -2906,29 +2879,30 @@ cudaError_t run_group(int blocks, const StepArgs& a, cudaStream_t st, int* occ) 
                                 size_t(WARPS) * 64 * (sizeof(LineSh64) + C * sizeof(CondRec64)), blocks, a, st, occ);
 }
 
+// Rows of 32 or 8 points (FP64: one point per lane, mixed: two).
 template <int C, int WARPS, bool MIXED>
-cudaError_t dispatch_mc_ls(int LS, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
-    if (LS == 1) return run_group<C, WARPS, 1, MIXED>(blocks, a, st, occ);
-    if (LS == 4) return run_group<C, WARPS, 4, MIXED>(blocks, a, st, occ);
+cudaError_t dispatch_mc_ls(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+    if (row == 32) return run_group<C, WARPS, MIXED ? 2 : 1, MIXED>(blocks, a, st, occ);
+    if (row == 8) return run_group<C, WARPS, MIXED ? 8 : 4, MIXED>(blocks, a, st, occ);
     return cudaErrorInvalidValue;
 }
 
 template <int WARPS, bool MIXED>
-cudaError_t dispatch_mc_c(int C, int LS, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+cudaError_t dispatch_mc_c(int C, int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
     switch (C) {
-        case 2: return dispatch_mc_ls<2, WARPS, MIXED>(LS, blocks, a, st, occ);
-        case 4: return dispatch_mc_ls<4, WARPS, MIXED>(LS, blocks, a, st, occ);
-        case 8: return dispatch_mc_ls<8, WARPS, MIXED>(LS, blocks, a, st, occ);
+        case 2: return dispatch_mc_ls<2, WARPS, MIXED>(row, blocks, a, st, occ);
+        case 4: return dispatch_mc_ls<4, WARPS, MIXED>(row, blocks, a, st, occ);
+        case 8: return dispatch_mc_ls<8, WARPS, MIXED>(row, blocks, a, st, occ);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t dispatch_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
+cudaError_t dispatch_mc(bool mixed, int C, int warps, int row, int blocks, const StepArgs& a,
                         cudaStream_t st, int* occ) {
-    if (warps == 4) return mixed ? dispatch_mc_c<4, true>(C, LS, blocks, a, st, occ)
-                                 : dispatch_mc_c<4, false>(C, LS, blocks, a, st, occ);
-    if (warps == 8) return mixed ? dispatch_mc_c<8, true>(C, LS, blocks, a, st, occ)
-                                 : dispatch_mc_c<8, false>(C, LS, blocks, a, st, occ);
+    if (warps == 4) return mixed ? dispatch_mc_c<4, true>(C, row, blocks, a, st, occ)
+                                 : dispatch_mc_c<4, false>(C, row, blocks, a, st, occ);
+    if (warps == 8) return mixed ? dispatch_mc_c<8, true>(C, row, blocks, a, st, occ)
+                                 : dispatch_mc_c<8, false>(C, row, blocks, a, st, occ);
     return cudaErrorInvalidValue;
 }
 
@@ -3094,10 +3068,10 @@ cudaError_t launch_core_mcx(const CoreArgs& a, int ncond, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int LS, int blocks, const StepArgs& a,
+cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int row, int blocks, const StepArgs& a,
                               cudaStream_t stream) {
     if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
-    return dispatch_mc(mixed, C, warps, LS, blocks, a, stream, nullptr);
+    return dispatch_mc(mixed, C, warps, row, blocks, a, stream, nullptr);
 }
 
 cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream) {
@@ -3109,10 +3083,10 @@ int steptwo_near_blocks_per_sm() {
     return blocks_per_sm(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem);
 }
 
-int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int LS) {
+int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int row) {
     StepArgs dummy{};
     int occ = 0;
-    if (dispatch_mc(mixed, C, warps, LS, 0, dummy, nullptr, &occ) != cudaSuccess) return 0;
+    if (dispatch_mc(mixed, C, warps, row, 0, dummy, nullptr, &occ) != cudaSuccess) return 0;
     return occ;
 }
 

@@ -183,12 +183,14 @@ struct __align__(16) CellHead {
     float q;     // scale: at least every |zeta| of the cell, all conditions of the group
 };
 static_assert(sizeof(CellHead) == 16, "CellHead layout");
-constexpr float kCellKappa = 4.0f;
+constexpr float kCellKappa = 3.5f;
 // Moments kept, and the bits the terms beyond the ones evaluated are held
-// below: at the least distance (r = 1/4) the rest is 7e-16 of the line's value
-// with 28 terms (FP64) and 7e-9 with 16 (mixed, whose own arithmetic rounds at
-// 6e-8); further out fewer terms are evaluated (cell_terms in xs_kernels.cu).
-constexpr int kCellTerms64 = 28, kCellTermsMixed = 16;
+// below: at the least distance (r = 1 / 3.5) the rest is 3e-15 of the line's
+// value with 30 terms (FP64) and 7e-8 with 16 (mixed, whose own arithmetic rounds
+// at 6e-8), for a line at the cell's very edge; further out fewer terms are
+// evaluated (cell_terms in xs_kernels.cu).  At 4 instead of 3.5 (28 and 16 terms)
+// the near zone is an eighth wider.
+constexpr int kCellTerms64 = 30, kCellTermsMixed = 16;
 constexpr float kCellBits64 = 53.0f, kCellBitsMixed = 28.0f;
 constexpr int cell_moments(bool mixed) { return mixed ? kCellTermsMixed : kCellTerms64; }
 

@@ -2156,34 +2156,35 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
 }
 
 // The core passes' per-warp table: row = point of the 32-point row, column =
-// line of the batch (stride kCoreRow floats keeps rows 16-byte aligned and a
-// quarter-warp's 128-bit row reads on distinct banks).  It starts all zero;
-// each lane writes its line's entries, every lane then sums its point's row in
-// line order, and each lane clears what it wrote.
+// lane (stride kCoreRow floats keeps rows 16-byte aligned and a quarter-warp's
+// 128-bit row reads on distinct banks).  It starts all zero; each lane adds its
+// lines' entries to its own column, and every kCoreBatches batches of 32 lines
+// every lane sums its point's row into FP64 and clears it: FP32 sums at most
+// kCoreBatches + 9 deep in a fixed order.  (One sum and one clearing per batch
+// took a quarter of the pass: few entries per batch and line.)
 constexpr int kCoreRow = 36;
+constexpr int kCoreBatches = 8;
 __device__ __forceinline__ void core_table_clear(float (*T)[kCoreRow], int lane) {
 #pragma unroll
     for (int q = 0; q < 32; q += 4) *reinterpret_cast<float4*>(&T[lane][q]) = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
 }
-// Sum of this lane's row in line order.  Entries of lines that wrote nothing
-// are +0, so adding only the columns of `written` (the lines that wrote
-// something; few in a sparse batch) gives the same sum.  Warp-uniform.
-__device__ __forceinline__ float core_table_column(float (*T)[kCoreRow], int lane, unsigned written) {
-    float part = 0.0f;
-    if (__popc(written) <= 8) {
-        for (unsigned m = written; m != 0u; m &= m - 1u) part += T[lane][__ffs(m) - 1];
-        return part;
-    }
+// Sum of this lane's row, which is cleared.  Warp-uniform.
+__device__ __forceinline__ double core_table_take(float (*T)[kCoreRow], int lane) {
+    __syncwarp();
+    float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int q = 0; q < 32; q += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(&T[lane][q]);
-        part += v.x;
-        part += v.y;
-        part += v.z;
-        part += v.w;
+        float4* row = reinterpret_cast<float4*>(&T[lane][q]);
+        const float4 v = *row;
+        s.x += v.x;
+        s.y += v.y;
+        s.z += v.z;
+        s.w += v.w;
+        *row = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    return part;
+    __syncwarp();
+    return double(s.x) + double(s.y) + double(s.z) + double(s.w);
 }
 
 // Core pass of the mixed multi-condition layout.  A warp takes a (condition,
@@ -2192,10 +2193,9 @@ __device__ __forceinline__ float core_table_column(float (*T)[kCoreRow], int lan
 // widest interval bounds the reach), taken 32 at a time: each lane evaluates
 // W4 regions II-IV (region III-IV interval from step one, region III or IV
 // by Humlicek's test on the FP32 x, y) at the row's points inside its line's
-// interval, less the region-I rational where step two added it, and writes
-// them to a per-warp table, then each lane adds its point's column in line
-// order.  Sums are FP32 per batch of 32 lines and FP64
-// across batches, in a fixed order.  With line splits (blockIdx.z = split) a
+// interval, less the region-I rational where step two added it, and adds
+// them to its column of a per-warp table; every few batches each lane sums its
+// point's row into FP64, in a fixed order.  With line splits (blockIdx.z = split) a
 // row's batches are shared out as in step two and the sums go to the parts.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
@@ -2228,6 +2228,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
         const long E = warp_lower_bound(0, a.n, lane, [&](long i) { return a.mi[i] >= t0 - K; });
         const long F = warp_lower_bound(E, a.n, lane, [&](long i) { return a.mi[i] > tl + K; });
         double acc = 0.0;
+        int held = 0;  // batches in the table
         for (long b = E + 32L * split; b < F; b += 32L * S) {
             const long i = b + lane;
             int jlo = 1, jhi = 0;
@@ -2254,17 +2255,17 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_mcx(CoreArgs a) {
                         // step two added the region-I rational here unless the
                         // line was its core candidate and u < 1 (the same FP32 u)
                         if (!(cand && fmaf(X * X, k2, cy) < 1.0f)) w -= w4_region1_c(ax, y);
-                        T[j - t0][lane] = yp.y * w;
+                        T[j - t0][lane] += yp.y * w;
                     }
                 }
             }
-            const unsigned written = __ballot_sync(0xffffffffu, jlo <= jhi);
-            if (written == 0u) continue;  // no pair in this batch
-            __syncwarp();
-            acc += double(core_table_column(T, lane, written));
-            __syncwarp();
-            for (int j = jlo; j <= jhi; ++j) T[j - t0][lane] = 0.0f;  // back to all zeros
+            held += __any_sync(0xffffffffu, jlo <= jhi) ? 1 : 0;
+            if (held == kCoreBatches) {
+                acc += core_table_take(T, lane);
+                held = 0;
+            }
         }
+        if (held > 0) acc += core_table_take(T, lane);
         const int jj = t0 + lane;
         if (jj < t1) {
             if (S <= 1)
@@ -2298,6 +2299,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
     const float k = a.kx[c];
     const int split = int(blockIdx.z), S = a.splits;
     double acc = 0.0;
+    int held = 0;  // batches in the table
     for (long b = E + 32L * split; b < F; b += 32L * S) {
         const long i = b + lane;
         int jlo = 1, jhi = 0;
@@ -2314,16 +2316,16 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
                     w = (y >= fmaf(0.195f, ax, -0.176f)) ? w4_region3_re_f32(ax, y) : w4_region4_re_f32(ax, y);
                 else
                     w = w4_region2_re<float>(ax, y);
-                T[j - t0][lane] = r.pref * w;
+                T[j - t0][lane] += r.pref * w;
             }
         }
-        const unsigned written = __ballot_sync(0xffffffffu, jlo <= jhi);
-        if (written == 0u) continue;  // no pair in this batch
-        __syncwarp();
-        acc += double(core_table_column(T, lane, written));
-        __syncwarp();
-        for (int j = jlo; j <= jhi; ++j) T[j - t0][lane] = 0.0f;  // back to all zeros
+        held += __any_sync(0xffffffffu, jlo <= jhi) ? 1 : 0;
+        if (held == kCoreBatches) {
+            acc += core_table_take(T, lane);
+            held = 0;
+        }
     }
+    if (held > 0) acc += core_table_take(T, lane);
     const int jj = t0 + lane;
     if (jj < t1) {
         if (S <= 1)

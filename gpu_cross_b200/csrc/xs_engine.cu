@@ -572,11 +572,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             C = 1;
         } else if (C == 0) {
             // Measured on B200 (40-condition sweep, 0.1 cm-1 grid): two
-            // conditions per warp is fastest for the mixed path, and for the
-            // FP64 path with cells (8 conditions, 1e6 lines: 2.25 ms of step
-            // two against 2.80 with one); without cells FP64 is faster with
-            // one condition and 32*P points per warp.
-            C = (mixed || cells) && groups_ok(2) ? 2 : 1;
+            // conditions per warp or more is fastest for the mixed path; the
+            // FP64 path takes one (8 conditions, 1e6 lines, cells: 1.37 ms of
+            // step two against 1.63 with two).
+            C = mixed && groups_ok(2) ? 2 : 1;
             // mixed, 8-point rows (a coarse grid over a dense list): as many
             // conditions per warp as the batch allows (29.6 ms at 8 and 4,
             // 37.9 at 2 for the sweep of 40)
@@ -593,7 +592,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     const int CG = near || C > 1 ? C : 0;
     // Rows of 8 points, several lines at a time, where a 32-point row is wider than
     // what has to be taken line by line beside it (about 6 cells).
-    const int row = C > 1 && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid) ? 8 : 32;
+    const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1 && !(ov && ov->scratch);
+    const bool wide_row = cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid);
+    const int row = C > 1 ? (wide_row ? 8 : 32) : near64 ? (wide_row ? 8 : 16) : 0;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
         return fail(XS_ERR_INVALID, "line_splits must be 0 (automatic) .. 64");
 
@@ -603,8 +604,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Scratch layout for one group of conditions.
     const int group = ncond < kMaxCond ? ncond : kMaxCond;
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
-    if (near) W = 4;
+    if (near || near64) W = 4;
     int occ = near ? steptwo_near_blocks_per_sm()
+              : near64 ? steptwo_near64_blocks_per_sm(row)
               : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, row)
                    : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
     if (occ < 1) {
@@ -622,7 +624,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // different warps -- enough for about 16 items per resident warp, at
     // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
-    const int tile_pts = near ? 32 : CG ? row : 32 * P;
+    const int tile_pts = near ? 32 : (CG || near64) ? row : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
@@ -875,7 +877,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         sa.out_stride = out_stride;
         for (int c = 0; c < nc; ++c) sa.row[c] = order[size_t(c0 + c)];
         sa.G = G;
-        sa.tiles_per_cond = (grid->points + 32 * P - 1) / (32 * P);
+        sa.tiles_per_cond = tiles;
         sa.n_items = sa.tiles_per_cond * nc * S;
         sa.counter = words + 1;
         sa.splits = S;
@@ -938,6 +940,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
         err = near ? launch_steptwo_near(blocks, sa, st)
+              : near64 ? launch_steptwo_near64(row, blocks, sa, st)
               : CG ? launch_steptwo_mc(mixed, CG, W, row, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);
         if (err != cudaSuccess) return cuda_fail(err, "step two launch");

@@ -406,6 +406,9 @@ cudaError_t launch_check_rows(const CheckArgs& a, cudaStream_t stream);
 // records, groups of one condition), W4 regions II-IV included; 4 warps a block.
 cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream);
 int steptwo_near_blocks_per_sm();
+// FP64 single-condition step two on tiles of `row` = 32 or 8 points, lane = line.
+cudaError_t launch_steptwo_near64(int row, int blocks, const StepArgs& a, cudaStream_t stream);
+int steptwo_near64_blocks_per_sm(int row);
 
 // Multi-condition step two (Voigt): C conditions per warp.
 // Rows of `row` = 32 or 8 points.

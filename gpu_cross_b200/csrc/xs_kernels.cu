@@ -904,72 +904,121 @@ __device__ __forceinline__ double rcp_newton2_f64(double x) {
 }
 
 // Adds the far cells of split s of S to the sums v of this lane's P points
-// f[] (one condition).
-template <int P, int PM>
+// f[] (one condition).  The heads of 32 cells are read at once, a cell per lane,
+// and handed round; two cells are summed side by side, so that the latency of
+// their moments' loads and of the chain is shared.  The warp's LS lane subsets
+// (sub = this lane's) take every LS-th cell; their sums are left apart.
+template <int P, int PM, int LS = 1>
 __device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
                                               float bits, double ftlo, double fthi, const double (&f)[P],
-                                              double (&v)[P]) {
-    auto run = [&](int c0, int c1) {
-        for (int c = c0 + s; c < c1; c += S) {
-            const CellHead h = H[c];
-            const int np = cell_terms<PM>(bits, fmax(ftlo - h.c0, h.c0 - fthi), h.q);
-            const double2* m = reinterpret_cast<const double2*>(M + size_t(c) * PM);
-            double t[P], a[P];
-#pragma unroll
-            for (int p = 0; p < P; ++p) {
-                t[p] = double(h.q) * rcp_newton2_f64(f[p] - h.c0);
-                a[p] = 0.0;
-            }
-#pragma unroll 2
-            for (int k = np / 2 - 1; k >= 0; --k) {
-                const double2 mk = __ldg(m + k);
-#pragma unroll
-                for (int p = 0; p < P; ++p) a[p] = fma(fma(a[p], t[p], mk.y), t[p], mk.x);
-            }
-#pragma unroll
-            for (int p = 0; p < P; ++p) v[p] = fma(a[p] * t[p], t[p], v[p]);
-        }
-    };
-    run(r.fa, r.fb);
-    run(r.fc, r.fd);
-}
-
-// The same for one point and N of the C conditions of a group (M: at the first of
-// them); the warp's LS lane subsets (sub = this lane's) take every LS-th cell.
-template <int C, int N, int PM, int LS = 1>
-__device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
-                                                 float bits, double ftlo, double fthi, double f, double (&v)[N],
-                                                 int sub = 0) {
+                                              double (&v)[P], int lane, int sub = 0) {
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         const int c1 = h ? r.fd : r.fb;
 #pragma unroll 1
-        for (int b = (h ? r.fc : r.fa) + s * LS; b < c1; b += S * LS) {
-            const int c = min(b + sub, c1 - 1);
-            const CellHead hd = H[c];
-            int np = cell_terms<PM>(bits, fmax(ftlo - hd.c0, hd.c0 - fthi), hd.q);
-            if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
-            const double* m = M + size_t(c) * (PM * C);
-            const double t = double(hd.q) * rcp_newton2_f64(f - hd.c0);
-            double a[N];
+        for (int b = (h ? r.fc : r.fa) + s; b < c1; b += 32 * S) {
+            const int cnt = min(32, (c1 - b + S - 1) / S);
+            const CellHead hd = H[min(b + lane * S, c1 - 1)];
+            const int terms = cell_terms<PM>(bits, fmax(ftlo - hd.c0, hd.c0 - fthi), hd.q);
+#pragma unroll 1
+            for (int k = 0; k < cnt; k += 2 * LS) {
+                double t[2][P], a[2][P];
+                const double2* m[2];
+                int np = 0;
 #pragma unroll
-            for (int q = 0; q < N; ++q) a[q] = 0.0;
-#pragma unroll 2
-            for (int k = np - 1; k >= 0; --k) {
-                if constexpr (N % 2 == 0) {
+                for (int w = 0; w < 2; ++w) {
+                    const int kk = k + w * LS + sub;
+                    const bool ok = kk < cnt;
+                    const int at = ok ? kk : cnt - 1;
+                    const double cc = __shfl_sync(0xffffffffu, hd.c0, at);
+                    const float q = __shfl_sync(0xffffffffu, hd.q, at);
+                    const int n = __shfl_sync(0xffffffffu, terms, at);
+                    np = max(np, n);
+                    m[w] = reinterpret_cast<const double2*>(M + size_t(b + at * S) * PM);
 #pragma unroll
-                    for (int q = 0; q < N; q += 2) {
-                        const double2 mk = __ldg(reinterpret_cast<const double2*>(m + k * C + q));
-                        a[q] = fma(a[q], t, mk.x);
-                        a[q + 1] = fma(a[q + 1], t, mk.y);
+                    for (int p = 0; p < P; ++p) {
+                        // (a cell past the end adds 0: t = 0)
+                        t[w][p] = ok ? double(q) * rcp_newton2_f64(f[p] - cc) : 0.0;
+                        a[w][p] = 0.0;
                     }
-                } else {
-                    a[0] = fma(a[0], t, __ldg(m + k * C));
+                }
+                if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
+#pragma unroll 2
+                for (int i = np / 2 - 1; i >= 0; --i) {
+                    const double2 m0 = __ldg(m[0] + i), m1 = __ldg(m[1] + i);
+#pragma unroll
+                    for (int p = 0; p < P; ++p) {
+                        a[0][p] = fma(fma(a[0][p], t[0][p], m0.y), t[0][p], m0.x);
+                        a[1][p] = fma(fma(a[1][p], t[1][p], m1.y), t[1][p], m1.x);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < P; ++p) {
+                    v[p] = fma(a[0][p] * t[0][p], t[0][p], v[p]);
+                    v[p] = fma(a[1][p] * t[1][p], t[1][p], v[p]);
                 }
             }
-            const double t2 = b + sub < c1 ? t * t : 0.0;
+        }
+    }
+}
+
+// The same for one point and N of the C conditions of a group (M: at the first of
+// them).
+template <int C, int N, int PM, int LS = 1>
+__device__ __forceinline__ void add_far_cells_mc(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
+                                                 float bits, double ftlo, double fthi, double f, double (&v)[N],
+                                                 int lane, int sub = 0) {
+    constexpr int W = N <= 4 ? 2 : 1;  // cells side by side
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const int c1 = h ? r.fd : r.fb;
+#pragma unroll 1
+        for (int b = (h ? r.fc : r.fa) + s; b < c1; b += 32 * S) {
+            const int cnt = min(32, (c1 - b + S - 1) / S);
+            const CellHead hd = H[min(b + lane * S, c1 - 1)];
+            const int terms = cell_terms<PM>(bits, fmax(ftlo - hd.c0, hd.c0 - fthi), hd.q);
+#pragma unroll 1
+            for (int k = 0; k < cnt; k += W * LS) {
+                double t[W], a[W][N];
+                const double* m[W];
+                int np = 0;
 #pragma unroll
-            for (int q = 0; q < N; ++q) v[q] = fma(a[q], t2, v[q]);
+                for (int w = 0; w < W; ++w) {
+                    const int kk = k + w * LS + sub;
+                    const bool ok = kk < cnt;
+                    const int at = ok ? kk : cnt - 1;
+                    const double cc = __shfl_sync(0xffffffffu, hd.c0, at);
+                    const float q = __shfl_sync(0xffffffffu, hd.q, at);
+                    np = max(np, __shfl_sync(0xffffffffu, terms, at));
+                    m[w] = M + size_t(b + at * S) * (PM * C);
+                    t[w] = ok ? double(q) * rcp_newton2_f64(f - cc) : 0.0;  // (past the end: adds 0)
+#pragma unroll
+                    for (int q2 = 0; q2 < N; ++q2) a[w][q2] = 0.0;
+                }
+                if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
+#pragma unroll 2
+                for (int i = np - 1; i >= 0; --i) {
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        if constexpr (N % 2 == 0) {
+#pragma unroll
+                            for (int q = 0; q < N; q += 2) {
+                                const double2 mk = __ldg(reinterpret_cast<const double2*>(m[w] + i * C + q));
+                                a[w][q] = fma(a[w][q], t[w], mk.x);
+                                a[w][q + 1] = fma(a[w][q + 1], t[w], mk.y);
+                            }
+                        } else {
+                            a[w][0] = fma(a[w][0], t[w], __ldg(m[w] + i * C));
+                        }
+                    }
+                }
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    const double t2 = t[w] * t[w];
+#pragma unroll
+                    for (int q = 0; q < N; ++q) v[q] = fma(a[w][q], t2, v[q]);
+                }
+            }
         }
     }
 }
@@ -1045,6 +1094,25 @@ template <class R>
 __device__ __forceinline__ R w4_region2_re(R x, R y) {
     return R(kW4C) * w4_region2_c(x, y);
 }
+// The same for one line at several points: what depends on y alone, times f.
+struct Region2F64 {
+    double d1, d2, p1, p2, q1, q2;
+    __device__ __forceinline__ Region2F64(double y, double f) {
+        const double y2 = y * y;
+        d1 = y2 * (4.0 * kW4B1);
+        d2 = y2 * (4.0 * kW4B2);
+        p1 = y * (f * kW4A1);
+        p2 = y * (f * kW4A2);
+        q1 = p1 * (0.5 + kW4B1);
+        q2 = p2 * (0.5 + kW4B2);
+    }
+    // u = x^2 + y^2 - 1/2
+    __device__ __forceinline__ double operator()(double u) const {
+        const double e1 = u + (0.5 - kW4B1), e2 = u + (0.5 - kW4B2);
+        const double g1 = fma(e1, e1, d1), g2 = fma(e2, e2, d2);
+        return fma(fma(u, p1, q1), g2, fma(u, p2, q2) * g1) * rcp_newton2_f64(g1 * g2);
+    }
+};
 
 // The region-I rational of W4 in FP32 per unit c pref, as step two evaluates
 // it: y (u + 1) / (u^2 + 2 y^2), u = x^2 + y^2 - 0.5.  The core pass
@@ -1525,7 +1593,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
 #pragma unroll
             for (int p = 0; p < P; ++p) f[p] = F[jj[p] < t1 ? jj[p] : tl];
             add_far_cells<P, PM>(a.chead + cell0, a.cmom + cell0 * PM, runs, a.splits, w.s,
-                                 MIXED ? kCellBitsMixed : kCellBits64, F[t0], F[tl], f, v);
+                                 MIXED ? kCellBitsMixed : kCellBits64, F[t0], F[tl], f, v, lane);
         }
         if constexpr (!MIXED) {
             // W4 regions II-IV
@@ -1725,7 +1793,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
         }
         if (runs.fa < runs.fb || runs.fc < runs.fd)
             add_far_cells_mc<C, C, kCellTerms64, LS>(a.chead + cell0, a.cmom + cell0 * (kCellTerms64 * C), runs,
-                                                     a.splits, split, kCellBits64, F[t0], F[tl], fj, accd, sub);
+                                                     a.splits, split, kCellBits64, F[t0], F[tl], fj, accd, lane, sub);
 #pragma unroll
         for (int c = 0; c < C; ++c) accd[c] = sum_subsets<LS>(accd[c]);
         // W4 regions II-IV (point p of the row in lane p)
@@ -2147,7 +2215,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
         if (runs.fa < runs.fb || runs.fc < runs.fd)
             add_far_cells_mc<C, VF, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * (kCellTermsMixed * C) + c0, runs,
                                                      a.splits, split, kCellBitsMixed, F[t0], F[tl],
-                                                     F[jj < t1 ? jj : tl], sum);
+                                                     F[jj < t1 ? jj : tl], sum, lane);
         if (!copy && jj < t1) {
 #pragma unroll
             for (int v = 0; v < VF; ++v) put_result(a, cg * C + c0 + v, split, jj, sum[v]);
@@ -2599,9 +2667,15 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
                 v = ypb[at];
             }
             const bool odd = __any_sync(0xffffffffu, (__float_as_int(s.w) & (kLineWhole | kLineWide)) != 0);
+            // (the reach is the widest of the whole list: the group's own
+            // intervals decide)
+            CoreIv iv = {1, 0, 1, 0};
+            bool core = odd;
             if (odd || (ge > E && gb < Fc)) {
-                CoreIv iv = {1, 0, 1, 0};
                 if (live) iv = civ[gb + lane];
+                core = __any_sync(0xffffffffu, odd || (iv.lo15 <= tl && iv.hi15 >= t0 && iv.lo15 <= iv.hi15));
+            }
+            if (core) {
                 if (!odd) core_group(s, win, v, iv);
                 inner_pairs(s, win, v, iv, gb + lane, odd);
             } else if (gb >= fs && ge <= fe && ge - gb == 32) {
@@ -2619,8 +2693,222 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
         double v[1] = {sum};
         if (runs.fa < runs.fb || runs.fc < runs.fd)
             add_far_cells<1, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits, w.s,
-                                              kCellBitsMixed, F[t0], F[tl], f, v);
+                                              kCellBitsMixed, F[t0], F[tl], f, v, lane);
         if (jj < t1) put_result(a, w.c, w.s, jj, v[0]);
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 single-condition step two on narrow tiles, lane = line.
+//
+// As k_steptwo_near: a warp takes a tile of PT points and 32 lines at a time,
+// each lane evaluating its own line (80-byte record, staged; a lane's reads of
+// its record are conflict-free at that stride) at the tile's points, whose grid
+// values are read from shared memory.  Groups without core candidates add
+// region I into PT accumulators; groups with core candidates go over the points
+// in a loop, choosing the region per pair with the reference's own test on x
+// and y, into a per-warp table with a column per lane.  At the end the lanes'
+// sums are added up by halving exchanges (lane p keeps point p).  PT = 8: coarse
+// grids over dense lists, where a 32-point tile is wider than the near zone.
+//
+// Bound by the FP64 pipe and the instructions around it: 8 FP64 operations and
+// about 4 others per region-I pair.  B200, 1e7 lines, 7.5e5 points with cells:
+// the point-parallel kernel needed 7.0 ms, 26 % of the FP64 pipe and three other
+// instructions for each FP64 one.
+// ---------------------------------------------------------------------------
+template <int PT>
+constexpr size_t near64_warp_smem() {
+    return 64 * sizeof(RecV64) + sizeof(double) * PT * kCoreRow64 + sizeof(double) * PT;
+}
+
+template <int PT>
+__global__ void __launch_bounds__(kNearWarps * 32, 4) k_steptwo_near64(StepArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31;
+    unsigned char* const mine = smem_raw + size_t(threadIdx.x >> 5) * near64_warp_smem<PT>();
+    RecV64* buf = reinterpret_cast<RecV64*>(mine);
+    double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine + 64 * sizeof(RecV64));
+    double* fj = &T[PT][0];  // the tile's grid values
+    const double* F = a.G.freq;
+    const int* mi = a.mi;
+#pragma unroll 4
+    for (int q = 0; q < PT; ++q) T[q][lane] = 0.0;
+
+    for (;;) {
+        int item = 0;
+        if (lane == 0) item = int(atomicAdd(a.counter, 1u));
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= a.n_items) break;
+        const int per_cond = a.tiles_per_cond * a.splits;
+        const int c = item / per_cond;
+        const int tile = (item - c * per_cond) / a.splits;
+        const int split = item - c * per_cond - tile * a.splits;
+        const int t0 = a.G.start + tile * PT;
+        const int gend = a.G.start + a.G.points;
+        const int t1 = t0 + PT < gend ? t0 + PT : gend;
+        const int tl = t1 - 1;
+        const size_t cbase = size_t(c) * size_t(a.n);
+        const int* whi = a.whi + cbase;
+        const int* wlo = a.wlo + cbase;
+        const int kc = a.kc[c];
+        const int La = warp_search(whi, 0, int(a.n), t0 + 1, lane);
+        const int Lb = warp_search(wlo, La, int(a.n), t1, lane);
+        const int fs = warp_search(whi, La, Lb, t1, lane);
+        const int Cb = warp_search(wlo, La, Lb, t0 + 1, lane);
+        const int fe = Cb > fs ? Cb : fs;
+        const int E = warp_search(mi, La, Lb, t0 - kc, lane);
+        const int Fc = warp_search(mi, E, Lb, tl + kc + 1, lane);
+        const RecV64* recs = reinterpret_cast<const RecV64*>(a.rec) + cbase;
+        const size_t cell0 = size_t(c) * size_t(a.ncell);
+        const LineRuns runs =
+            line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
+
+        if (lane < PT) fj[lane] = F[min(t0 + lane, tl)];
+        double acc[PT];
+#pragma unroll
+        for (int p = 0; p < PT; ++p) acc[p] = 0.0;
+        bool cored = false;  // the table holds something
+        __syncwarp();
+
+        // One group of lines, region I only; MASK: some windows cover the tile
+        // partly (or there are fewer than 32 lines).
+        auto plain_group = [&](auto mask, const RecV64& r, int w0, unsigned wlen) {
+            const double nu = r.nu, g = r.g, Cy = r.Cy, D2 = r.D2, Pc = r.Pc;
+#pragma unroll
+            for (int p = 0; p < PT; ++p) {
+                const double xs = (nu - fj[p]) * g;
+                const double u = fma(xs, xs, Cy);
+                double rr = rcp_refined_f64(fma(u, u, D2));
+                if constexpr (decltype(mask)::value) rr = unsigned(w0 + p) < wlen ? rr : 0.0;
+                acc[p] = fma(fma(u, Pc, Pc), rr, acc[p]);
+            }
+        };
+        // A group whose core bands reach the tile, two points at a time.  x, y
+        // and the region choice are the reference's.
+        auto core_group = [&](const RecV64& r, int w0, unsigned wlen) {
+            const double nu = r.nu, g = r.g, Cy = r.Cy, D2 = r.D2, Pc = r.Pc, y = r.y, pref = r.pref;
+            const Region2F64 region2(y, pref);
+            cored = true;
+#pragma unroll 1
+            for (int p0 = 0; p0 < PT; p0 += 2) {
+                double ax[2], sx[2], u[2], v[2];
+                bool in[2], core[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const double xs = (nu - fj[p0 + h]) * g;
+                    ax[h] = fabs(xs);
+                    sx[h] = ax[h] + y;
+                    u[h] = fma(xs, xs, Cy);
+                    in[h] = unsigned(w0 + p0 + h) < wlen;
+                    core[h] = in[h] && sx[h] < 15.0;
+                    v[h] = 0.0;
+                }
+                if (__any_sync(0xffffffffu, (in[0] && !core[0]) || (in[1] && !core[1]))) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double rr = rcp_refined_f64(fma(u[h], u[h], D2));
+                        v[h] = in[h] && !core[h] ? fma(u[h], Pc, Pc) * rr : 0.0;
+                    }
+                }
+                if (__any_sync(0xffffffffu, core[0] || core[1])) {
+                    const bool c0 = core[0] && sx[0] < 5.5, c1 = core[1] && sx[1] < 5.5;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double w = region2(u[h]);
+                        if (core[h] && sx[h] >= 5.5) v[h] = w;
+                    }
+                    if (__any_sync(0xffffffffu, c0 || c1)) {
+#pragma unroll 1
+                        for (int h = 0; h < 2; ++h) {
+                            if (!(h ? c1 : c0)) continue;
+                            const double x = h ? ax[1] : ax[0];
+                            const double w = pref * (y >= 0.195 * x - 0.176 ? w4_region3_re_f64(x, y) : w4_region4_re_f64(x, y));
+                            if (h) v[1] = w;
+                            else v[0] = w;
+                        }
+                    }
+                }
+                T[p0][lane] += v[0];
+                T[p0 + 1][lane] += v[1];
+            }
+        };
+
+        const int ngroups = runs.groups_of(a.splits, split);
+        auto gstart = [&](int gi, int& end) {
+            long e;
+            const int b = int(runs.start(split + gi * a.splits, e));
+            end = int(e);
+            return b;
+        };
+        auto issue = [&](int gi) {
+            if (gi < ngroups) {
+                int end;
+                const int b = gstart(gi, end);
+                stage(buf + (gi & 1) * 32, recs + b, min(end - b, 32), lane);
+            }
+            cp_async_commit();
+        };
+        issue(0);
+        for (int gi = 0; gi < ngroups; ++gi) {
+            issue(gi + 1);
+            cp_async_wait<1>();
+            __syncwarp();
+            int end;
+            const int gb = gstart(gi, end);
+            const int cnt = min(end - gb, 32);
+            // (a lane past the group's end takes its last line, outside every
+            // window)
+            const RecV64& r = buf[(gi & 1) * 32 + min(lane, cnt - 1)];
+            const int w0 = t0 - r.lo;
+            const unsigned wlen = lane < cnt ? unsigned(r.hi - r.lo) : 0u;
+            // (kc is the widest band of the whole list: the group's own decide)
+            const bool core = gb + cnt > E && gb < Fc && __any_sync(0xffffffffu, r.clo <= tl && r.chi >= t0);
+            if (core) core_group(r, w0, wlen);
+            else if (gb >= fs && gb + cnt <= fe && cnt == 32) plain_group(std::false_type(), r, w0, wlen);
+            else plain_group(std::true_type(), r, w0, wlen);
+            __syncwarp();
+        }
+        cp_async_wait<0>();
+        // lane p: point p (p < PT), the lanes' sums by halving exchanges
+        int n = PT;
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) {
+            if (o < PT) {
+                n /= 2;
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int i = 0; i < PT / 2; ++i)
+                    if (i < n) {
+                        const double got = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + n], o);
+                        acc[i] = (up ? acc[i + n] : acc[i]) + got;
+                    }
+            } else {
+#pragma unroll
+                for (int i = 0; i < PT; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+            }
+        }
+        double v[1] = {acc[0]};
+        __syncwarp();
+        if (cored) {
+            if (lane < PT) {
+#pragma unroll 8
+                for (int q = 0; q < 32; ++q) v[0] += T[lane][q];
+            }
+            __syncwarp();
+#pragma unroll 4
+            for (int q = 0; q < PT; ++q) T[q][lane] = 0.0;
+        }
+        const int jj = t0 + lane % PT;
+        if (runs.fa < runs.fb || runs.fc < runs.fd) {
+            // 32 / PT lanes to a point, each every 32 / PT-th cell
+            const double f[1] = {F[min(jj, tl)]};
+            double far[1] = {0.0};
+            add_far_cells<1, kCellTerms64, 32 / PT>(a.chead + cell0, a.cmom + cell0 * kCellTerms64, runs, a.splits, split,
+                                                    kCellBits64, F[t0], F[tl], f, far, lane, lane / PT);
+            v[0] += sum_subsets<32 / PT>(far[0]);
+        }
+        if (lane < PT && jj < t1) put_result(a, c, split, jj, v[0]);
         __syncwarp();
     }
 }
@@ -3079,6 +3367,27 @@ cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int row, int blocks,
 cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream) {
     if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
     return run_group_kernel(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem, blocks, a, stream, nullptr);
+}
+
+static cudaError_t dispatch_near64(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+    if (row == 16)
+        return run_group_kernel(k_steptwo_near64<16>, kNearWarps * 32, kNearWarps * near64_warp_smem<16>(), blocks, a, st,
+                                occ);
+    if (row == 8)
+        return run_group_kernel(k_steptwo_near64<8>, kNearWarps * 32, kNearWarps * near64_warp_smem<8>(), blocks, a, st,
+                                occ);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_steptwo_near64(int row, int blocks, const StepArgs& a, cudaStream_t stream) {
+    if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
+    return dispatch_near64(row, blocks, a, stream, nullptr);
+}
+
+int steptwo_near64_blocks_per_sm(int row) {
+    StepArgs dummy{};
+    int occ = 0;
+    return dispatch_near64(row, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
 }
 
 int steptwo_near_blocks_per_sm() {

@@ -576,25 +576,29 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             // FP64 path takes one (8 conditions, 1e6 lines, cells: 1.37 ms of
             // step two against 1.63 with two).
             C = mixed && groups_ok(2) ? 2 : 1;
-            // mixed, 8-point rows (a coarse grid over a dense list): as many
-            // conditions per warp as the batch allows (29.6 ms at 8 and 4,
-            // 37.9 at 2 for the sweep of 40)
-            if (mixed && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid))
+            // mixed with cells: on 8-point rows (a coarse grid over a dense
+            // list) as many conditions per warp as the batch allows (24.2 ms at
+            // 8, 26.4 at 4 for the sweep of 40), else one (8 conditions on a
+            // 0.01 cm-1 grid, 1e6 lines: 2.55 ms at 1, 2.65 at 2 and 4)
+            if (mixed && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid)) {
                 for (int cg : {4, 8})
                     if (groups_ok(cg)) C = cg;
+            } else if (mixed && cells) {
+                C = 1;
+            }
         } else if (C > 1 && !groups_ok(C)) {
             return fail(XS_ERR_INVALID, "conditions_per_warp needs ncond <= 64 and, for every cut, a "
                                         "number of conditions that is a multiple of it");
         }
     }
-    // Single mixed conditions with cells: lane = line, 32-point tiles.
-    const bool near = mixed && C == 1 && narrow_tiles && cells;
-    const int CG = near || C > 1 ? C : 0;
-    // Rows of 8 points, several lines at a time, where a 32-point row is wider than
-    // what has to be taken line by line beside it (about 6 cells).
-    const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1 && !(ov && ov->scratch);
+    // Single conditions on narrow tiles: lane = line (mixed: with cells only).
+    // Tiles and rows of 8 points where a 32-point one is wider than what has to be
+    // taken line by line beside it (about 6 cells).
     const bool wide_row = cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid);
-    const int row = C > 1 ? (wide_row ? 8 : 32) : near64 ? (wide_row ? 8 : 16) : 0;
+    const bool near = mixed && C == 1 && narrow_tiles && (cells || wide_row);
+    const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1 && !(ov && ov->scratch);
+    const int CG = near || C > 1 ? C : 0;
+    const int row = C > 1 ? (wide_row ? 8 : 32) : wide_row ? 8 : 16;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
         return fail(XS_ERR_INVALID, "line_splits must be 0 (automatic) .. 64");
 
@@ -605,7 +609,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     const int group = ncond < kMaxCond ? ncond : kMaxCond;
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
     if (near || near64) W = 4;
-    int occ = near ? steptwo_near_blocks_per_sm()
+    int occ = near ? steptwo_near_blocks_per_sm(row)
               : near64 ? steptwo_near64_blocks_per_sm(row)
               : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, row)
                    : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
@@ -624,7 +628,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // different warps -- enough for about 16 items per resident warp, at
     // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
-    const int tile_pts = near ? 32 : (CG || near64) ? row : 32 * P;
+    const int tile_pts = (CG || near64) ? row : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
     int S = opt->line_splits;
@@ -939,7 +943,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
-        err = near ? launch_steptwo_near(blocks, sa, st)
+        err = near ? launch_steptwo_near(row, blocks, sa, st)
               : near64 ? launch_steptwo_near64(row, blocks, sa, st)
               : CG ? launch_steptwo_mc(mixed, CG, W, row, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);

@@ -1881,10 +1881,10 @@ constexpr size_t mcx_warp_smem() {
 // Sums w[0..V) over the lane bits 16 .. LP by halving exchanges: a lane ends
 // with the values base .. base + n - 1 of `kept` (fewer values than lanes: every
 // lane of the remaining bits holds the same one).
-template <int V, int LP>
+template <int V, int LP, class R = float>
 struct Halving {
     static constexpr int kKept = V * LP / 32 > 1 ? V * LP / 32 : 1;
-    __device__ static __forceinline__ void sum(float (&w)[V], int lane) {
+    __device__ static __forceinline__ void sum(R (&w)[V], int lane) {
         int n = V;
 #pragma unroll
         for (int o = 16; o >= LP; o >>= 1) {
@@ -1894,7 +1894,7 @@ struct Halving {
 #pragma unroll
                 for (int i = 0; i < V / 2; ++i)
                     if (i < n) {
-                        const float got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + n], o);
+                        const R got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + n], o);
                         w[i] = (up ? w[i + n] : w[i]) + got;
                     }
             } else {
@@ -2407,15 +2407,17 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // Mixed-precision single-condition step two with cells, lane = line.
 //
 // With the far wings taken by cells, what is left of a tile is a few thousand
-// lines on few points, so the lanes go over the lines: a warp takes a tile of
-// 32 points and 32 lines at a time, each lane evaluating its own line at every
-// point of the tile into 32 accumulators.  The line's constants are read once
+// lines on few points, so the lanes go over the lines: a warp takes a tile of PT
+// points and 32 lines at a time, each lane evaluating its own line at every
+// point of the tile into PT accumulators.  The line's constants are read once
 // per lane (a broadcast to every lane costs a shared-memory wavefront per 4
 // bytes), and the lines of a group, being neighbours, are in the same W4 region
 // at the same point.  Every 8 groups of lines the accumulators are summed over
-// the lanes (a transposing exchange: lane p ends with point p) and added in
-// FP64 (sums 8 + 5 deep: 4.5e-8 of the result in the 2-norm, 7.0e-8 with 32
-// groups; the point-parallel kernel 5.3e-8).
+// the lanes by halving exchanges and added in FP64 (sums 8 + 5 deep: 4.5e-8 of
+// the result in the 2-norm, 7.0e-8 with 32 groups; the point-parallel kernel
+// 5.3e-8).  Tiles of 16 points (32: 2.72 against 2.50 ms at the sizes below), of
+// 8 on coarse grids over dense lists, where 16 points are wider than the near
+// zone.
 //
 // Two evaluations share one reciprocal, 1/dA = dB / (dA dB) (narrow lines,
 // kPairUMax).  Groups with lines of the core reach choose region I or II per
@@ -2425,45 +2427,33 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // bodies: with every region unrolled a third of the time went to instruction
 // fetches.)
 //
-// B200, 1e7 lines, 7.5e5 points: 3.37 ms against 3.5 + 1.2 ms for the
-// point-parallel kernel with cells and its core pass; 96 registers, 57 % of the
-// issue slots.  The same kernel over 4 points and 8 conditions was slower than
-// k_steptwo_voigt_mcx on the coarse sweep (20.7 against 12.6 ms).
+// B200, 1e7 lines, 7.5e5 points: 2.5 ms against 3.5 + 1.2 ms for the
+// point-parallel kernel with cells and its core pass.  The same kernel over
+// 32 / C points and C = 8 conditions was slower than k_steptwo_voigt_mcx on the
+// coarse sweep (20.7 against 12.6 ms).
 // ---------------------------------------------------------------------------
 constexpr int kNearRow = 33;
 constexpr int kNearWarps = 4;
 // Two stages of offsets and flags, windows and (y, pref), and the table.
-constexpr size_t kNearWarpSmem = 64 * (sizeof(float4) + sizeof(int2) + sizeof(float2)) + sizeof(float) * 32 * kNearRow;
-// Sum over the warp of 32 values per lane: lane L gets that of value L.
-__device__ __forceinline__ float transpose_sum_f32(float2 (&v)[16], int lane) {
-    float w[16];
-    {
-        const bool up = (lane & 16) != 0;
+template <int PT>
+constexpr size_t near_warp_smem() {
+    return 64 * (sizeof(float4) + sizeof(int2) + sizeof(float2)) + sizeof(float) * PT * kNearRow;
+}
+// Sum over the lanes of one tile point's sub-lanes (neighbours), to each of them.
+template <int SUB>
+__device__ __forceinline__ double sum_neighbours(double v) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            // values i and i + 16
-            const float lo = (i & 1) ? v[i / 2].y : v[i / 2].x;
-            const float hi = (i & 1) ? v[8 + i / 2].y : v[8 + i / 2].x;
-            const float got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, 16);
-            w[i] = (up ? hi : lo) + got;
-        }
-    }
-#pragma unroll
-    for (int o = 8; o >= 1; o >>= 1) {
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int i = 0; i < o; ++i) {
-            const float got = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[i + o], o);
-            w[i] = (up ? w[i + o] : w[i]) + got;
-        }
-    }
-    return w[0];
+    for (int o = 1; o < SUB; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
+template <int PT>
 __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
-    unsigned char* const mine = smem_raw + size_t(threadIdx.x >> 5) * kNearWarpSmem;
+    constexpr int SUB = 32 / PT;  // lanes to a point where lanes stand for points
+    using Sum = Halving<PT, 1>;   // lane ends with point lane / SUB
+    unsigned char* const mine = smem_raw + size_t(threadIdx.x >> 5) * near_warp_smem<PT>();
     float4* lsb = reinterpret_cast<float4*>(mine);
     float2* ypb = reinterpret_cast<float2*>(mine + 64 * sizeof(float4));
     int2* lhb = reinterpret_cast<int2*>(ypb + 64);
@@ -2471,16 +2461,26 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
     const double* F = a.G.freq;
     const int* mi = a.mi;
 #pragma unroll 4
-    for (int q = 0; q < 32; ++q) T[q][lane] = 0.0f;
+    for (int q = 0; q < PT; ++q) T[q][lane] = 0.0f;
     __syncwarp();
 
-    WorkItem w;
-    while (next_item(a, 1, lane, w)) {
-        const int t0 = w.t0, t1 = w.t1, tl = t1 - 1;
-        const size_t cbase = size_t(w.c) * size_t(a.n);
+    for (;;) {
+        int item = 0;
+        if (lane == 0) item = int(atomicAdd(a.counter, 1u));
+        item = __shfl_sync(0xffffffffu, item, 0);
+        if (item >= a.n_items) break;
+        const int per_cond = a.tiles_per_cond * a.splits;
+        const int cond = item / per_cond;
+        const int tile = (item - cond * per_cond) / a.splits;
+        const int split = item - cond * per_cond - tile * a.splits;
+        const int t0 = a.G.start + tile * PT;
+        const int gend = a.G.start + a.G.points;
+        const int t1 = t0 + PT < gend ? t0 + PT : gend;
+        const int tl = t1 - 1;
+        const size_t cbase = size_t(cond) * size_t(a.n);
         const int* whi = a.whi + cbase;
         const int* wlo = a.wlo + cbase;
-        const int K = a.kc[kMaxCond + w.c];  // the condition's core reach
+        const int K = a.kc[kMaxCond + cond];  // the condition's core reach
         const int La = warp_search(whi, 0, int(a.n), t0 + 1, lane);
         const int Lb = warp_search(wlo, La, int(a.n), t1, lane);
         const int fs = warp_search(whi, La, Lb, t1, lane);
@@ -2491,14 +2491,14 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
         const LineShX* lsh = reinterpret_cast<const LineShX*>(a.lsh) + cbase;
         const float2* yp = a.cyp + cbase;
         const CoreIv* civ = a.civ + cbase;
-        const size_t cell0 = size_t(w.c) * size_t(a.ncell);
+        const size_t cell0 = size_t(cond) * size_t(a.ncell);
         const LineRuns runs =
             line_runs(a.chead + cell0, a.ncell, a.cshift, a.n, La, Lb, fs, fe, F[t0], F[tl], lane);
 
         const float t0f = float(t0);
-        float2 acc[16];  // points 2 q, 2 q + 1
+        float2 acc[PT / 2];  // points 2 q, 2 q + 1
 #pragma unroll
-        for (int v = 0; v < 16; ++v) acc[v] = f2(0.0f, 0.0f);
+        for (int v = 0; v < PT / 2; ++v) acc[v] = f2(0.0f, 0.0f);
         double sum = 0.0;
         bool cored = false;  // the table holds something
 
@@ -2530,7 +2530,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
             const int w0 = t0 - win.x;
             const R1 r = constants(v);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
+            for (int q = 0; q < PT / 2; ++q) {
                 const float2 x = offsets(mj, s, q);
                 const float2 u = __ffma2_rn(x, x, r.cy);
                 float2 num = __ffma2_rn(u, r.pc, r.pc);
@@ -2555,7 +2555,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
             const float2 p1 = __fmul2_rn(r.pc, f2s(float(kW4A1 / kW4C)));
             const float2 p2 = __fmul2_rn(r.pc, f2s(float(kW4A2 / kW4C)));
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
+            for (int q = 0; q < PT / 2; ++q) {
                 const float2 x = offsets(mj, s, q);
                 const float2 u = __ffma2_rn(x, x, r.cy);
                 float2 den = __ffma2_rn(u, u, r.d2);
@@ -2592,7 +2592,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
 #pragma unroll 1
             for (int j = jlo; j <= jhi; ++j) {
                 const float ax =
-                    fabsf(whole ? float((nu - F[j]) / nu) * a.kx[w.c] : fmaf(s.x - float(j), s.y, s.z));
+                    fabsf(whole ? float((nu - F[j]) / nu) * a.kx[cond] : fmaf(s.x - float(j), s.y, s.z));
                 float wf;
                 if (!all || (j >= iv.lo55 && j <= iv.hi55)) {
                     wf = float(1.0 / kW4C) *
@@ -2611,28 +2611,34 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
             }
             __syncwarp();
         };
-        // The lanes' partial sums, into point `lane`.
+        // The lanes' partial sums, into point lane / SUB.
         auto fold = [&]() {
-            sum += double(transpose_sum_f32(acc, lane));
+            float s[PT];
 #pragma unroll
-            for (int v = 0; v < 16; ++v) acc[v] = f2(0.0f, 0.0f);
+            for (int v = 0; v < PT / 2; ++v) {
+                s[2 * v] = acc[v].x;
+                s[2 * v + 1] = acc[v].y;
+                acc[v] = f2(0.0f, 0.0f);
+            }
+            Sum::sum(s, lane);
+            sum += double(s[0]);
             if (cored) {
                 cored = false;
                 __syncwarp();
                 double t = 0.0;
 #pragma unroll 4
-                for (int q = 0; q < 32; ++q) t += double(T[lane][q]);
-                sum += t;
+                for (int q = 0; q < 32; q += SUB) t += double(T[lane / SUB][q + lane % SUB]);
+                sum += sum_neighbours<SUB>(t);
                 __syncwarp();
 #pragma unroll 4
-                for (int q = 0; q < 32; ++q) T[q][lane] = 0.0f;
+                for (int q = 0; q < PT; ++q) T[q][lane] = 0.0f;
             }
         };
 
-        const int ngroups = runs.groups_of(a.splits, w.s);
+        const int ngroups = runs.groups_of(a.splits, split);
         auto gstart = [&](int gi, int& end) {
             long e;
-            const int b = int(runs.start(w.s + gi * a.splits, e));
+            const int b = int(runs.start(split + gi * a.splits, e));
             end = int(e);
             return b;
         };
@@ -2688,13 +2694,15 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
         cp_async_wait<0>();
         fold();
 
-        const int jj = t0 + lane;
-        const double f[1] = {F[jj < t1 ? jj : tl]};
-        double v[1] = {sum};
-        if (runs.fa < runs.fb || runs.fc < runs.fd)
-            add_far_cells<1, kCellTermsMixed>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits, w.s,
-                                              kCellBitsMixed, F[t0], F[tl], f, v, lane);
-        if (jj < t1) put_result(a, w.c, w.s, jj, v[0]);
+        const int jj = t0 + lane / SUB;
+        if (runs.fa < runs.fb || runs.fc < runs.fd) {
+            const double f[1] = {F[min(jj, tl)]};
+            double far[1] = {0.0};
+            add_far_cells<1, kCellTermsMixed, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits,
+                                                   split, kCellBitsMixed, F[t0], F[tl], f, far, lane, lane % SUB);
+            sum += sum_neighbours<SUB>(far[0]);
+        }
+        if (lane % SUB == 0 && jj < t1) put_result(a, cond, split, jj, sum);
         __syncwarp();
     }
 }
@@ -2709,7 +2717,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
 // region I into PT accumulators; groups with core candidates go over the points
 // in a loop, choosing the region per pair with the reference's own test on x
 // and y, into a per-warp table with a column per lane.  At the end the lanes'
-// sums are added up by halving exchanges (lane p keeps point p).  PT = 8: coarse
+// sums are added up by halving exchanges.  PT = 8: coarse
 // grids over dense lists, where a 32-point tile is wider than the near zone.
 //
 // Bound by the FP64 pipe and the instructions around it: 8 FP64 operations and
@@ -2726,6 +2734,8 @@ template <int PT>
 __global__ void __launch_bounds__(kNearWarps * 32, 4) k_steptwo_near64(StepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
+    constexpr int SUB = 32 / PT;        // lanes to a point where lanes stand for points
+    using Sum = Halving<PT, 1, double>;  // lane ends with point lane / SUB
     unsigned char* const mine = smem_raw + size_t(threadIdx.x >> 5) * near64_warp_smem<PT>();
     RecV64* buf = reinterpret_cast<RecV64*>(mine);
     double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine + 64 * sizeof(RecV64));
@@ -2870,45 +2880,28 @@ __global__ void __launch_bounds__(kNearWarps * 32, 4) k_steptwo_near64(StepArgs 
             __syncwarp();
         }
         cp_async_wait<0>();
-        // lane p: point p (p < PT), the lanes' sums by halving exchanges
-        int n = PT;
-#pragma unroll
-        for (int o = 16; o >= 1; o >>= 1) {
-            if (o < PT) {
-                n /= 2;
-                const bool up = (lane & o) != 0;
-#pragma unroll
-                for (int i = 0; i < PT / 2; ++i)
-                    if (i < n) {
-                        const double got = __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + n], o);
-                        acc[i] = (up ? acc[i + n] : acc[i]) + got;
-                    }
-            } else {
-#pragma unroll
-                for (int i = 0; i < PT; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-            }
-        }
-        double v[1] = {acc[0]};
-        __syncwarp();
+        // point lane / SUB, the lanes' sums by halving exchanges
+        Sum::sum(acc, lane);
+        double sum = acc[0];
         if (cored) {
-            if (lane < PT) {
+            __syncwarp();
+            double t = 0.0;
 #pragma unroll 8
-                for (int q = 0; q < 32; ++q) v[0] += T[lane][q];
-            }
+            for (int q = 0; q < 32; q += SUB) t += T[lane / SUB][q + lane % SUB];
+            sum += sum_neighbours<SUB>(t);
             __syncwarp();
 #pragma unroll 4
             for (int q = 0; q < PT; ++q) T[q][lane] = 0.0;
         }
-        const int jj = t0 + lane % PT;
+        const int jj = t0 + lane / SUB;
         if (runs.fa < runs.fb || runs.fc < runs.fd) {
-            // 32 / PT lanes to a point, each every 32 / PT-th cell
             const double f[1] = {F[min(jj, tl)]};
             double far[1] = {0.0};
-            add_far_cells<1, kCellTerms64, 32 / PT>(a.chead + cell0, a.cmom + cell0 * kCellTerms64, runs, a.splits, split,
-                                                    kCellBits64, F[t0], F[tl], f, far, lane, lane / PT);
-            v[0] += sum_subsets<32 / PT>(far[0]);
+            add_far_cells<1, kCellTerms64, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTerms64, runs, a.splits, split,
+                                                kCellBits64, F[t0], F[tl], f, far, lane, lane % SUB);
+            sum += sum_neighbours<SUB>(far[0]);
         }
-        if (lane < PT && jj < t1) put_result(a, c, split, jj, v[0]);
+        if (lane % SUB == 0 && jj < t1) put_result(a, c, split, jj, sum);
         __syncwarp();
     }
 }
@@ -3364,9 +3357,26 @@ cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int row, int blocks,
     return dispatch_mc(mixed, C, warps, row, blocks, a, stream, nullptr);
 }
 
-cudaError_t launch_steptwo_near(int blocks, const StepArgs& a, cudaStream_t stream) {
+static cudaError_t dispatch_near(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+    auto go = [&](auto kernel, size_t smem) {
+        return run_group_kernel(kernel, kNearWarps * 32, kNearWarps * smem, blocks, a, st, occ);
+    };
+    switch (row) {
+        case 8: return go(k_steptwo_near<8>, near_warp_smem<8>());
+        case 16: return go(k_steptwo_near<16>, near_warp_smem<16>());
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_steptwo_near(int row, int blocks, const StepArgs& a, cudaStream_t stream) {
     if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
-    return run_group_kernel(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem, blocks, a, stream, nullptr);
+    return dispatch_near(row, blocks, a, stream, nullptr);
+}
+
+int steptwo_near_blocks_per_sm(int row) {
+    StepArgs dummy{};
+    int occ = 0;
+    return dispatch_near(row, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
 }
 
 static cudaError_t dispatch_near64(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
@@ -3388,10 +3398,6 @@ int steptwo_near64_blocks_per_sm(int row) {
     StepArgs dummy{};
     int occ = 0;
     return dispatch_near64(row, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
-}
-
-int steptwo_near_blocks_per_sm() {
-    return blocks_per_sm(k_steptwo_near, kNearWarps * 32, kNearWarps * kNearWarpSmem);
 }
 
 int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int row) {

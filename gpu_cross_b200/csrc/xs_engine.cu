@@ -591,11 +591,12 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
                                         "number of conditions that is a multiple of it");
         }
     }
-    // Single conditions on narrow tiles: lane = line (mixed: with cells only).
+    // Single conditions on narrow tiles: lane = line.
     // Tiles and rows of 8 points where a 32-point one is wider than what has to be
     // taken line by line beside it (about 6 cells).
     const bool wide_row = cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid);
-    const bool near = mixed && C == 1 && narrow_tiles && (cells || wide_row);
+    const bool near =
+        mixed && C == 1 && !(ov && ov->scratch) && (P == 1 || (narrow_tiles && (cells || wide_row)));
     const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1 && !(ov && ov->scratch);
     const int CG = near || C > 1 ? C : 0;
     const int row = C > 1 ? (wide_row ? 8 : 32) : wide_row ? 8 : 16;
@@ -746,9 +747,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         cap = cudaStreamCaptureStatusNone;
     }
     const unsigned ev_flags = (cap == cudaStreamCaptureStatusActive) ? cudaEventRecordExternal : 0u;
-    cudaError_t err = launch_grid_check(G, words, st);
+    cudaError_t err = launch_grid_check(G, words, reinterpret_cast<int*>(base + plan.off_kc), words + 1, st);
     if (err != cudaSuccess) return cuda_fail(err, "grid check launch");
-    int launched = G.npoints_total >= 2 ? 1 : 0;
+    int launched = 1;
 
     for (int c0 = 0; c0 < ncond; c0 += group) {
         const int nc = std::min(group, ncond - c0);
@@ -805,8 +806,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             pa.wslot[g] = (CG > 1 && g > 0 && pa.cond[g * CG].cut == pa.cond[(g - 1) * CG].cut) ? pa.wslot[g - 1] : g;
 
         if (timing && c0 == 0) cudaEventRecordWithFlags(e->ev[0], st, ev_flags);
-        err = cudaMemsetAsync(pa.kc, 0, sizeof(int) * size_t(kKcWords), st);
-        if (err != cudaSuccess) return cuda_fail(err, "core-width reset");
+        if (c0 > 0) {  // (the grid check cleared it for the first launch)
+            err = cudaMemsetAsync(pa.kc, 0, sizeof(int) * size_t(kKcWords), st);
+            if (err != cudaSuccess) return cuda_fail(err, "core-width reset");
+        }
         if (c0 == 0 && h2d_pieces > 0) {
             // host lines: slice k is copied on the copy stream (after the
             // work already on this stream, which may still read the device
@@ -896,8 +899,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         sa.x0 = pa.x0;
         sa.xg = pa.xg;
         sa.x0g = pa.x0g;
-        err = cudaMemsetAsync(sa.counter, 0, sizeof(unsigned), st);
-        if (err != cudaSuccess) return cuda_fail(err, "counter reset");
+        if (c0 > 0) {
+            err = cudaMemsetAsync(sa.counter, 0, sizeof(unsigned), st);
+            if (err != cudaSuccess) return cuda_fail(err, "counter reset");
+        }
         for (int c = 0; c < nc; ++c) {
             const double k = 1.0 / pa.cond[c].dpw;
             sa.kx[c] = float(k);

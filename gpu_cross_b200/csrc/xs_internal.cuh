@@ -322,7 +322,8 @@ struct CellArgs {
 cudaError_t launch_cells(bool mixed, const CellArgs& a, cudaStream_t stream);
 
 // Kernel launchers (xs_kernels.cu).  All asynchronous on `stream`.
-cudaError_t launch_grid_check(const GridDev& g, unsigned* err, cudaStream_t stream);
+// kc, counter (may be NULL): words cleared for the call's first launches.
+cudaError_t launch_grid_check(const GridDev& g, unsigned* err, int* kc, unsigned* counter, cudaStream_t stream);
 cudaError_t launch_prep(int kind, int conv, bool mixed, const PrepArgs& a, cudaStream_t stream);
 // P = points per thread (1, 2, 4, 8), warps per block (4 or 8).
 cudaError_t launch_steptwo(int kind, int conv, bool mixed, int P, int warps, int blocks,

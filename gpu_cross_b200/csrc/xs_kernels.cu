@@ -129,7 +129,13 @@ __device__ __forceinline__ int clamp_index(double v, int lo, int hi) {
 // ---------------------------------------------------------------------------
 // Grid check.
 // ---------------------------------------------------------------------------
-__global__ void k_grid_check(GridDev g, unsigned* err) {
+// Also clears the words step one and step two start from (kc, counter; NULL:
+// left alone), which saves two memsets per call.
+__global__ void k_grid_check(GridDev g, unsigned* err, int* kc, unsigned* counter) {
+    if (blockIdx.x == 0 && kc) {
+        for (int t = threadIdx.x; t < kKcWords; t += blockDim.x) kc[t] = 0;
+        if (threadIdx.x == 0) *counter = 0;
+    }
     const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
     if (j >= g.npoints_total) return;
     const double f0 = g.freq[0];
@@ -3245,10 +3251,10 @@ cudaError_t dispatch_steptwo(int kind, int conv, bool mixed, int P, int warps, i
 
 }  // namespace
 
-cudaError_t launch_grid_check(const GridDev& g, unsigned* err, cudaStream_t stream) {
-    if (g.npoints_total < 2) return cudaSuccess;
-    const int n = g.npoints_total - 1;
-    k_grid_check<<<(n + 255) / 256, 256, 0, stream>>>(g, err);
+cudaError_t launch_grid_check(const GridDev& g, unsigned* err, int* kc, unsigned* counter, cudaStream_t stream) {
+    if (g.npoints_total < 2 && !kc) return cudaSuccess;
+    const int n = g.npoints_total > 2 ? g.npoints_total - 1 : 1;
+    k_grid_check<<<(n + 255) / 256, 256, 0, stream>>>(g, err, kc, counter);
     return cudaGetLastError();
 }
 

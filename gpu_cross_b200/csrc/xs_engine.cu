@@ -114,7 +114,7 @@ void default_shape(int kind, bool mixed, bool cells, double window_points, int* 
         *warps = 4;
     } else {
         *P = 1;
-        *warps = 8;
+        *warps = 4;
     }
 }
 
@@ -642,7 +642,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         // at its window ends, some 8 cells and 3 tile widths: fewer, larger
         // parts (300k-line FP64 band, 3126 tiles: 0.42 ms of step two in 1
         // part per tile, 0.33 in 4, 0.43 in 16).
-        const long waves = cshift ? 6 : 16;
+        // Doppler and Gaussian lines reach a few points only: parts when there
+        // are fewer than 4 tiles per resident warp (1e6 lines on 1e6 points, 9
+        // tiles per warp: 200 us in 1 part, 228 in 2).
+        const long waves = cshift ? 6 : kind == XS_VOIGT ? 16 : 4;
         if (items < waves * warps) {
             double cutmax = 0.0;
             for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
@@ -651,7 +654,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             if (cshift)
                 lpt = std::min(lpt, double(n) * 3.0 * double(tile_pts) * opt->dfreq / span + double(8L << cshift));
             long want = (waves * warps + items - 1) / items;
-            want = std::min<long>(want, long(lpt / (cshift ? 64.0 : 128.0)));
+            want = std::min<long>(want, long(lpt / (cshift ? 64.0 : kind == XS_VOIGT ? 128.0 : 256.0)));
             // (one condition: cells and parts together stay within kMaxPartBytes,
             // what the server and the streamed lists reserve beside the records)
             const size_t cell_b = cshift && ncond == 1 ? cell_bytes(mixed, n, group, CG, cshift) : 0;

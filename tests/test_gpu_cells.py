@@ -78,7 +78,7 @@ def test_cells_one_condition(engine, cuda, convention, n, df, make):
 
 
 @pytest.mark.parametrize("C", [2, 4, 8])
-@pytest.mark.parametrize("n, df", [(8003, 0.1), (6000, 0.021)])
+@pytest.mark.parametrize("n, df", [(8003, 0.1), (6000, 0.021), (40001, 0.1)])
 def test_cells_groups_of_conditions(engine, cuda, C, n, df):
     lines = uneven(n, 33)
     grid = synth.Grid(985.0, 1117.0, int(132.0 / df))

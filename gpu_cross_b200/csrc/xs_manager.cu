@@ -13,7 +13,6 @@
 #include <cmath>
 #include <numeric>
 #include <string>
-#include <cstring>
 #include <vector>
 
 #include "xs_engine.h"
@@ -50,15 +49,6 @@ struct DevGuard {
 // it (VoigtProfile.cpp:30-36) stay moderate.
 constexpr size_t kGpuNtransCap = size_t(1) << 26;
 
-// Line lists of up to this many bytes cross to the device in one copy of one
-// block: a copy of pageable memory costs about 10 us however small it is, packing
-// 256 KB about as much.  (2000 lines: six copies 72 us, one 34.  The grid's two
-// arrays stay two copies: below 64 KB each those take the driver's short path,
-// and one of both was slower, 39 against 22 us.)
-constexpr size_t kPackBytes = size_t(256) << 10;
-
-size_t al256(size_t v) { return (v + 255) / 256 * 256; }
-
 }  // namespace
 
 struct xs_manager {
@@ -78,8 +68,6 @@ struct xs_manager {
     double *d_nu = nullptr, *d_e = nullptr, *d_aif = nullptr, *d_gamma = nullptr, *d_n = nullptr;
     int* d_gns = nullptr;
     size_t cap = 0, nlines = 0;
-    bool one_block = false;   // the line arrays lie behind d_nu in one allocation
-    std::vector<char> pack;   //   and cross in one copy, packed here
     bool have_gamma = false;
 
     bool have_consts = false;
@@ -89,14 +77,11 @@ struct xs_manager {
 
     void free_lines() {
         cudaFree(d_nu);
-        if (!one_block) {
-            cudaFree(d_e);
-            cudaFree(d_aif);
-            cudaFree(d_gamma);
-            cudaFree(d_n);
-            cudaFree(d_gns);
-        }
-        one_block = false;
+        cudaFree(d_e);
+        cudaFree(d_aif);
+        cudaFree(d_gamma);
+        cudaFree(d_n);
+        cudaFree(d_gns);
         d_nu = d_e = d_aif = d_gamma = d_n = nullptr;
         d_gns = nullptr;
         cap = nlines = 0;
@@ -139,7 +124,6 @@ int xs_manager_cleanup(xs_manager* m) {
     m->d_freq = m->d_intens = nullptr;
     m->npoints = 0;
     m->free_lines();
-    std::vector<char>().swap(m->pack);
     return XS_OK;
 }
 
@@ -233,30 +217,13 @@ int xs_manager_transfer_vectors(xs_manager* m, size_t Nener, const double* h_ene
     if (Nener > m->cap || (with_gamma && !m->d_gamma)) {
         m->free_lines();
         const size_t c = std::max<size_t>(Nener, 1);
-        const bool wings = with_gamma || m->profile == XS_VOIGT;
-        const size_t d8 = al256(c * sizeof(double)), d4 = al256(c * sizeof(int));
-        const size_t block = (wings ? 5 : 3) * d8 + d4;
-        m->one_block = block <= kPackBytes;
-        if (m->one_block) {
-            char* base = nullptr;
-            XM_CU(cudaMalloc(&base, block));
-            m->d_nu = reinterpret_cast<double*>(base);
-            m->d_e = reinterpret_cast<double*>(base + d8);
-            m->d_aif = reinterpret_cast<double*>(base + 2 * d8);
-            m->d_gns = reinterpret_cast<int*>(base + 3 * d8);
-            if (wings) {
-                m->d_gamma = reinterpret_cast<double*>(base + 3 * d8 + d4);
-                m->d_n = reinterpret_cast<double*>(base + 4 * d8 + d4);
-            }
-        } else {
-            XM_CU(cudaMalloc(&m->d_nu, c * sizeof(double)));
-            XM_CU(cudaMalloc(&m->d_e, c * sizeof(double)));
-            XM_CU(cudaMalloc(&m->d_aif, c * sizeof(double)));
-            XM_CU(cudaMalloc(&m->d_gns, c * sizeof(int)));
-            if (wings) {
-                XM_CU(cudaMalloc(&m->d_gamma, c * sizeof(double)));
-                XM_CU(cudaMalloc(&m->d_n, c * sizeof(double)));
-            }
+        XM_CU(cudaMalloc(&m->d_nu, c * sizeof(double)));
+        XM_CU(cudaMalloc(&m->d_e, c * sizeof(double)));
+        XM_CU(cudaMalloc(&m->d_aif, c * sizeof(double)));
+        XM_CU(cudaMalloc(&m->d_gns, c * sizeof(int)));
+        if (with_gamma || m->profile == XS_VOIGT) {
+            XM_CU(cudaMalloc(&m->d_gamma, c * sizeof(double)));
+            XM_CU(cudaMalloc(&m->d_n, c * sizeof(double)));
         }
         m->cap = c;
     }
@@ -279,26 +246,7 @@ int xs_manager_transfer_vectors(xs_manager* m, size_t Nener, const double* h_ene
         std::stable_sort(order.begin(), order.end(),
                          [&](size_t a, size_t b) { return h_nu[a] < h_nu[b]; });
     }
-    if (Nener > 0 && sorted && m->one_block) {
-        // a small list in one copy, laid out as the device block is
-        const char* base = reinterpret_cast<const char*>(m->d_nu);
-        const char* last = with_gamma ? reinterpret_cast<const char*>(m->d_n + Nener)
-                                      : reinterpret_cast<const char*>(m->d_gns + Nener);
-        const size_t span = size_t(last - base);
-        m->pack.resize(span);
-        auto put = [&](const void* dst, const void* src, size_t bytes) {
-            std::memcpy(m->pack.data() + (static_cast<const char*>(dst) - base), src, bytes);
-        };
-        put(m->d_nu, h_nu, Nener * sizeof(double));
-        put(m->d_e, h_energies, Nener * sizeof(double));
-        put(m->d_aif, h_aif, Nener * sizeof(double));
-        put(m->d_gns, h_gns, Nener * sizeof(int));
-        if (with_gamma) {
-            put(m->d_gamma, h_gamma, Nener * sizeof(double));
-            put(m->d_n, h_n, Nener * sizeof(double));
-        }
-        XM_CU(cudaMemcpy(m->d_nu, m->pack.data(), span, cudaMemcpyHostToDevice));
-    } else if (Nener > 0) {
+    if (Nener > 0) {
         XM_CU(put_d(m->d_nu, h_nu));
         XM_CU(put_d(m->d_e, h_energies));
         XM_CU(put_d(m->d_aif, h_aif));

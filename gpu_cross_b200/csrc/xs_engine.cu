@@ -81,6 +81,8 @@ struct xs_engine {
     bool timed = false;
     // host line lists (xs_engine_execute_host): a copy stream and an event
     // per slice, made on first use
+    std::shared_ptr<void> stream_ws;  // xs_stream_execute's buffers
+    std::mutex stream_mu;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t pev[kMaxPieces + 1] = {};
     // error statement of the last execute: the a-priori bound and, with
@@ -307,6 +309,7 @@ int xs_engine_destroy(xs_engine* e) {
         DeviceGuard g(e->device);
         if (e->stream) cudaStreamSynchronize(e->stream);
         else cudaDeviceSynchronize();
+        e->stream_ws.reset();
         for (auto& ev : e->ev)
             if (ev) cudaEventDestroy(ev);
         for (auto& ev : e->pev)
@@ -1028,6 +1031,9 @@ int engine_reserve(xs_engine* e, size_t bytes) {
     e->scratch_cap = bytes;
     return XS_OK;
 }
+
+std::shared_ptr<void>& engine_stream_workspace(xs_engine* e) { return e->stream_ws; }
+std::mutex& engine_stream_mutex(xs_engine* e) { return e->stream_mu; }
 
 int engine_device(const xs_engine* e) { return e ? e->device : -1; }
 void* engine_stream(const xs_engine* e) { return e ? static_cast<void*>(e->stream) : nullptr; }

@@ -3,6 +3,8 @@
 #pragma once
 
 #include <cstddef>
+#include <memory>
+#include <mutex>
 
 #include "xsec_b200.h"
 
@@ -40,6 +42,10 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
 // Grows the engine's scratch to at least `bytes` (synchronises the engine's
 // stream when it has to reallocate).
 int engine_reserve(xs_engine* e, size_t bytes);
+// What xs_stream_execute keeps between calls (freed with the engine, its device
+// current) and the lock a call holds meanwhile.
+std::shared_ptr<void>& engine_stream_workspace(xs_engine* e);
+std::mutex& engine_stream_mutex(xs_engine* e);
 // The engine's device and stream.
 int engine_device(const xs_engine* e);
 void* engine_stream(const xs_engine* e);

@@ -48,8 +48,10 @@ int cuda_fail(cudaError_t e, const char* what) {
 // Most slices of a host line list (xs_engine_execute_host).
 constexpr int kMaxPieces = 16;
 
-// Least lines in a window, width of the window in tiles, and pairs of the call
-// from which the far wings are taken by cells.  (Below 1.2e7 pairs, some 10 us
+// Least lines in a window (half of it for batches: 70000 lines, 684 per window, 24
+// conditions 443 us with cells and 460 before; a single condition with 741 per
+// window 158 with and 152 without), width of the window in tiles, and pairs of the
+// call from which the far wings are taken by cells.  (Below 1.2e7 pairs, some 10 us
 // of step two, the GPU is not full either way and the series' launch and the
 // search for far cells cost what they save: 2000 lines on 4001 points, 7e6
 // pairs, 26 us without and 69 us with cells.)
@@ -98,21 +100,22 @@ namespace xs {
 int set_error(int code, const char* msg) { return fail(code, msg); }
 
 // Default launch shapes, from measurements on a B200 (the autotuner's table
-// takes precedence).  Voigt tiles of 32 P points: wide where a line's window
-// spans thousands of points (fewer partial lines per tile, record loads
-// shared by more points), narrow on coarse grids, where a 128-point tile
-// would hold mostly partial and core lines.  4 warps per block (the mixed
-// kernels then fit 28 warps per SM).
+// takes precedence).  Voigt tiles of 32 P points: two per lane where a line's
+// window spans many tiles (fewer partial lines per tile, record loads shared by
+// more points; 12000 lines on 700000 points: 109 us per call at P = 2 and 4, 131
+// at 1; 30000 on 200000: 103 at 2, 110 at 4), one on coarse grids, where a wider
+// tile would hold mostly partial and core lines.  4 warps per block.
 // With the far wings taken by cells, what is left line by line is the lines
-// near the tile and those whose windows end in it, so narrow tiles win: FP64
-// single point (1e7 lines, 7.5e5 points) 10.3 ms of step two at P = 4, 7.6 at
-// 2, 7.1 at 1; mixed 6.6, 4.7 (8 warps), 4.9.
-void default_shape(int kind, bool mixed, bool cells, double window_points, int* P, int* warps) {
+// near the tile and those whose windows end in it, so narrow tiles win (FP64
+// single point, 1e7 lines, 7.5e5 points, one kernel at three shapes: 10.3 ms of
+// step two at P = 4, 7.6 at 2, 7.1 at 1): P = 1, which single conditions take with
+// a lane per line (k_steptwo_near, k_steptwo_near64).
+void default_shape(int kind, bool cells, double window_points, int* P, int* warps) {
     if (kind == kVoigt && cells) {
-        *P = mixed ? 2 : 1;
-        *warps = mixed ? 8 : 4;
+        *P = 1;
+        *warps = 4;
     } else if (kind == kVoigt) {
-        *P = window_points >= 2048.0 ? 4 : (window_points >= 512.0 ? 2 : 1);
+        *P = window_points >= 512.0 ? 2 : 1;
         *warps = 4;
     } else {
         *P = 1;
@@ -197,7 +200,7 @@ int cell_shift(const xs_options& o, const xs_condition* conds, int ncond, long n
     const double win = 2.0 * cutmax, span = double(grid.points) * o.dfreq;
     const double lines = double(n) * win / (span + win);
     const double pairs = lines * double(grid.points) * double(ncond);
-    if (!(lines >= kCellMinLines) || !(win >= kCellMinTiles * double(tile_pts) * o.dfreq) ||
+    if (!(lines >= (ncond > 1 ? 0.5 : 1.0) * kCellMinLines) || !(win >= kCellMinTiles * double(tile_pts) * o.dfreq) ||
         !(pairs >= kCellMinPairs))
         return 0;
     int sh = int(std::lround(0.5 * std::log2(lines)));
@@ -522,7 +525,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         int dP, dW;
         double cutmax = 0.0;
         for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
-        default_shape(kind, mixed, cells, 2.0 * cutmax / opt->dfreq, &dP, &dW);
+        default_shape(kind, cells, 2.0 * cutmax / opt->dfreq, &dP, &dW);
         // Calls with fewer tiles than the GPU holds warps take narrower tiles:
         // a line split needs a buffer and a reduction, a narrow tile neither.
         // (3000 lines, 12000 points, 5000-point windows: step two 71 us with
@@ -630,11 +633,13 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // walks a long line list, and with a few items per warp the last items
     // leave a tail.  Each tile's lines are then split into parts taken by
     // different warps -- enough for about 16 items per resident warp, at
-    // least ~128 lines per part, the parts' buffer within kMaxPartBytes.
+    // least 128 or 256 lines per part, the parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
     const int tile_pts = (CG || near64) ? row : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
-    const int cshift = (ov && ov->scratch) ? 0 : cell_shift(*opt, conds, ncond, n, *grid, tile_pts);
+    // (tiles wider than 32 points, asked for by the caller, go line by line)
+    int cshift = near || near64 || C > 1 ? cell_shift(*opt, conds, ncond, n, *grid, tile_pts) : 0;
+    if (ov && ov->scratch) cshift = 0;
     int S = opt->line_splits;
     if (ov && ov->scratch) S = 1;  // a fixed caller scratch holds no parts
     if (S == 0) {
@@ -657,7 +662,11 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             if (cshift)
                 lpt = std::min(lpt, double(n) * 3.0 * double(tile_pts) * opt->dfreq / span + double(8L << cshift));
             long want = (waves * warps + items - 1) / items;
-            want = std::min<long>(want, long(lpt / (cshift ? 64.0 : kind == XS_VOIGT ? 128.0 : 256.0)));
+            // (128 lines per part where there are few tiles, 256 from a third of
+            // a tile per resident warp on: 30000 lines on 200000 points, 1562
+            // tiles, 112 us per call in 1 part and 127 in 2)
+            const double least = cshift ? 64.0 : kind == XS_VOIGT && 3 * items < warps ? 128.0 : 256.0;
+            want = std::min<long>(want, long(lpt / least));
             // (one condition: cells and parts together stay within kMaxPartBytes,
             // what the server and the streamed lists reserve beside the records)
             const size_t cell_b = cshift && ncond == 1 ? cell_bytes(mixed, n, group, CG, cshift) : 0;
@@ -666,23 +675,29 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             if (want > 1) S = int(want);
         }
     }
-    // Scratch after the records: cell heads and moments, then the split parts.
-    const int ncell = cshift ? int((n + (1L << cshift) - 1) >> cshift) : 0;
-    const size_t head_off = (plan.need + 255) & ~size_t(255);
-    const size_t mom_off = head_off + sizeof(CellHead) * size_t(ncell) * size_t(CG ? group / CG : group);
-    const size_t cell_end = cshift ? head_off + cell_bytes(mixed, n, group, CG, cshift) : plan.need;
-    const size_t part_off = (cell_end + 255) & ~size_t(255);
-    const size_t part_end = S > 1 ? part_off + sizeof(double) * size_t(S) * size_t(group) * size_t(grid->points)
-                                  : cell_end;
     // sampled FP64 check (mixed Voigt): before/ref values and statistics
     const bool streamed_call = ov && ov->s32;
     const int tiles32 = (grid->points + 31) / 32;
     const int nchk = (mixed && kind == XS_VOIGT && !streamed_call && opt->check_rows > 0)
                          ? std::min(std::min(opt->check_rows, kMaxCheckRows), tiles32)
                          : 0;
-    const size_t chk_off = (part_end + 255) & ~size_t(255);
-    const size_t chk_bytes = nchk ? sizeof(double) * (size_t(2 * 32 * nchk) + 4) * size_t(ncond) : 0;
-    const size_t need = nchk ? chk_off + chk_bytes : part_end;
+    // Scratch after the records: cell heads and moments, then the split parts,
+    // then the check's values.
+    int ncell = 0;
+    size_t head_off = 0, mom_off = 0, part_off = 0, chk_off = 0, need = 0;
+    auto layout = [&]() {
+        auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
+        ncell = cshift ? int((n + (1L << cshift) - 1) >> cshift) : 0;
+        head_off = al(plan.need);
+        mom_off = al(head_off + sizeof(CellHead) * size_t(ncell) * size_t(CG ? group / CG : group));
+        const size_t cell_end = cshift ? head_off + cell_bytes(mixed, n, group, CG, cshift) : plan.need;
+        part_off = al(cell_end);
+        const size_t part_end =
+            S > 1 ? part_off + sizeof(double) * size_t(S) * size_t(group) * size_t(grid->points) : cell_end;
+        chk_off = al(part_end);
+        need = nchk ? chk_off + sizeof(double) * (size_t(2 * 32 * nchk) + 4) * size_t(ncond) : part_end;
+    };
+    layout();
 
     void* scratch = nullptr;
     unsigned* words = e->d_words;
@@ -698,6 +713,20 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             e->scratch = nullptr;
             e->scratch_cap = 0;
             cudaError_t err = cudaMalloc(&e->scratch, need);
+            if (err == cudaErrorMemoryAllocation && !streamed_call && e->stream_mu.try_lock()) {
+                // what an earlier streamed call left
+                cudaGetLastError();
+                e->stream_ws.reset();
+                e->stream_mu.unlock();
+                err = cudaMalloc(&e->scratch, need);
+            }
+            if (err == cudaErrorMemoryAllocation && cshift) {
+                // without the cells: slower, but the records may still fit
+                cudaGetLastError();
+                cshift = 0;
+                layout();
+                err = cudaMalloc(&e->scratch, need);
+            }
             if (err != cudaSuccess) {
                 cudaGetLastError();
                 return cuda_fail(err, "cudaMalloc(scratch)");
@@ -870,7 +899,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             la.ncell = ncell;
             la.df = G.df;
             la.head = reinterpret_cast<CellHead*>(base + head_off);
-            la.mom = reinterpret_cast<double*>(base + ((mom_off + 255) & ~size_t(255)));
+            la.mom = reinterpret_cast<double*>(base + mom_off);
             for (int c = 0; c < nc; ++c) la.dpw[c] = pa.cond[c].dpw;
             err = launch_cells(mixed, la, st);
             if (err != cudaSuccess) return cuda_fail(err, "cell moments launch");
@@ -898,7 +927,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         sa.part_stride = size_t(grid->points);
         if (cshift) {
             sa.chead = reinterpret_cast<const CellHead*>(base + head_off);
-            sa.cmom = reinterpret_cast<const double*>(base + ((mom_off + 255) & ~size_t(255)));
+            sa.cmom = reinterpret_cast<const double*>(base + mom_off);
             sa.ncell = ncell;
             sa.cshift = cshift;
         }

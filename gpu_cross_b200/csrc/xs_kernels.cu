@@ -1308,9 +1308,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
         const long E = warp_lower_bound(fs, fe, lane, [&](long i) { return mi[i] >= t0 - kc; });
         const long Fc = warp_lower_bound(E, fe, lane, [&](long i) { return mi[i] > tl + kc; });
         const REC* recs = recs_all + cbase;
-        const LineRuns runs = line_runs(a.chead + size_t(w.c) * size_t(a.ncell), a.ncell, a.cshift, a.n, La, Lb, fs,
-                                        fe, F[t0], F[tl], lane);
-
         int jj[P];
         float jf[P];
         double fj[P];
@@ -1520,17 +1517,16 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             }
         };
 
-        // this item's groups of 32 lines
-        const int ngroups = runs.groups_of(a.splits, w.s);
-        auto gstart = [&](int gi, long& end) { return runs.start(w.s + gi * a.splits, end); };
+        // this item's groups of 32 lines: gi-th starts at La + 32 (s + gi S)
+        const int ngroups = split_groups(Lb - La, a.splits, w.s);
+        auto gstart = [&](int gi) { return La + 32L * (w.s + long(gi) * a.splits); };
         // kStages-deep cp.async pipeline: groups gi+1 .. gi+kStages-1 are in
         // flight while group gi is evaluated (one commit per step, empty
         // commits past the end keep the group count uniform).
         auto issue = [&](int g) {
             if (g < ngroups) {
-                long end;
-                const long b = gstart(g, end);
-                const long rem = end - b;
+                const long b = gstart(g);
+                const long rem = Lb - b;
                 stage_rec<kRec, int(sizeof(REC))>(mine + (g % kStages) * 32 * kRec, recs + b, int(rem < 32 ? rem : 32),
                                                   lane);
             }
@@ -1544,9 +1540,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
             __syncwarp();
             const unsigned char* R0 = mine + (gi % kStages) * 32 * kRec;
             auto R = [&](int t) { return R0 + t * kRec; };
-            long end;
-            const long gb = gstart(gi, end);
-            const long ge = end - gb < 32 ? end : gb + 32;
+            const long gb = gstart(gi);
+            const long ge = Lb - gb < 32 ? Lb : gb + 32;
             auto lo_of = [&](long v) { return int((v < gb ? gb : (v > ge ? ge : v)) - gb); };
             const int a0 = lo_of(La), a1 = lo_of(fs);
             const int b1 = lo_of(E), c1 = lo_of(Fc), d1 = lo_of(fe), e1 = lo_of(Lb);
@@ -1592,15 +1587,6 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
         double v[P];
 #pragma unroll
         for (int p = 0; p < P; ++p) v[p] = MIXED ? double(sumf[p]) - double(cmpf[p]) : accd[p];
-        if (runs.fa < runs.fb || runs.fc < runs.fd) {
-            constexpr int PM = cell_moments(MIXED);
-            const size_t cell0 = size_t(w.c) * size_t(a.ncell);
-            double f[P];
-#pragma unroll
-            for (int p = 0; p < P; ++p) f[p] = F[jj[p] < t1 ? jj[p] : tl];
-            add_far_cells<P, PM>(a.chead + cell0, a.cmom + cell0 * PM, runs, a.splits, w.s,
-                                 MIXED ? kCellBitsMixed : kCellBits64, F[t0], F[tl], f, v, lane);
-        }
         if constexpr (!MIXED) {
             // W4 regions II-IV
             double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine);

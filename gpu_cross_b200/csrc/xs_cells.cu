@@ -2,9 +2,6 @@
 // series (CellHead in xs_internal.cuh has the formulas).
 #include <cuda_runtime.h>
 
-#include <cfloat>
-#include <type_traits>
-
 #include "xs_internal.cuh"
 
 namespace xs {
@@ -27,12 +24,13 @@ __device__ __forceinline__ void transpose_sum(double (&v)[32], int lane) {
     }
 }
 
-// One warp per (cell, group of conditions), lanes over the cell's lines.
-// Step one's records give y and pref of each (line, condition):
-//   GROUPED false: RecV64 / RecV32;  true: CondRec64 (FP64).
-template <bool MIXED, bool GROUPED, int C>
+// FP64: one warp per (cell, group of conditions), lanes over the cell's lines;
+// y and pref of each (line, condition) from step one's RecV64 or, GROUPED,
+// CondRec64.  Bound by the FP64 pipe: 30 terms x 6 operations per (line,
+// condition); 1e7 lines 0.23 ms.
+template <bool GROUPED, int C>
 __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
-    constexpr int PM = cell_moments(MIXED);
+    constexpr int PM = kCellTerms64;
     const int lane = threadIdx.x & 31;
     const int cell = int(blockIdx.x) * kCellWarps + int(threadIdx.x >> 5);
     if (cell >= a.ncell) return;
@@ -47,10 +45,6 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
             const CondRec64& r = static_cast<const CondRec64*>(a.rec)[(size_t(g) * size_t(a.n) + size_t(i)) * C + k];
             y = r.y;
             pref = r.pref;
-        } else if constexpr (MIXED) {
-            const RecV32& r = static_cast<const RecV32*>(a.rec)[c * size_t(a.n) + size_t(i)];
-            y = double(r.y);
-            pref = double(r.pref);
         } else {
             const RecV64& r = static_cast<const RecV64*>(a.rec)[c * size_t(a.n) + size_t(i)];
             y = r.y;
@@ -76,7 +70,7 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
             const float z = __double2float_ru(sqrt(fma(re, re, gam * gam)));
             const float h = __double2float_ru(d + (y < 15.0 ? (15.0 - y) * w : 0.0));
             // (a NaN fails the comparisons)
-            good = good && w > 0.0 && z < 1.0e30f && h < 1.0e30f && fabs(pref) < (MIXED ? double(FLT_MAX) : 1.0e280);
+            good = good && w > 0.0 && z < 1.0e30f && h < 1.0e30f && fabs(pref) < 1.0e280;
             q = fmaxf(q, z);
             reach = fmaxf(reach, h);
         }
@@ -253,31 +247,24 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
     }
 }
 
-template <bool MIXED>
-cudaError_t run_cells(const CellArgs& a, cudaStream_t st) {
-    const dim3 grid(unsigned((a.ncell + kCellWarps - 1) / kCellWarps),
-                    unsigned(a.group > 1 ? a.ncond / a.group : a.ncond));
-    auto go = [&](auto c) {
-        constexpr int C = decltype(c)::value;
-        if constexpr (MIXED) k_cells_f32<C><<<grid, kCellWarps * 32, 0, st>>>(a);
-        else k_cells<false, true, C><<<grid, kCellWarps * 32, 0, st>>>(a);
-    };
-    switch (a.group) {
-        case 0: k_cells<MIXED, false, 1><<<grid, kCellWarps * 32, 0, st>>>(a); break;
-        case 1: go(std::integral_constant<int, 1>()); break;
-        case 2: go(std::integral_constant<int, 2>()); break;
-        case 4: go(std::integral_constant<int, 4>()); break;
-        case 8: go(std::integral_constant<int, 8>()); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
-}
-
 }  // namespace
 
 cudaError_t launch_cells(bool mixed, const CellArgs& a, cudaStream_t stream) {
     if (a.ncell <= 0 || a.ncond <= 0) return cudaSuccess;
-    return mixed ? run_cells<true>(a, stream) : run_cells<false>(a, stream);
+    const dim3 grid(unsigned((a.ncell + kCellWarps - 1) / kCellWarps),
+                    unsigned(a.group > 1 ? a.ncond / a.group : a.ncond));
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kCellWarps * 32, 0, stream>>>(a);
+        return cudaGetLastError();
+    };
+    switch (a.group) {
+        case 0: return mixed ? cudaErrorInvalidValue : go(k_cells<false, 1>);
+        case 1: return mixed ? go(k_cells_f32<1>) : cudaErrorInvalidValue;
+        case 2: return mixed ? go(k_cells_f32<2>) : go(k_cells<true, 2>);
+        case 4: return mixed ? go(k_cells_f32<4>) : go(k_cells<true, 4>);
+        case 8: return mixed ? go(k_cells_f32<8>) : go(k_cells<true, 8>);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 }  // namespace xs

@@ -310,8 +310,8 @@ struct CellArgs {
     const double* nu;   // line centres
     long n;             // lines per condition
     int ncond;
-    int group;          // conditions per group (0: single-condition layout)
-    const void* rec;    // RecV64 / RecV32, or CondRec64 (FP64 groups)
+    int group;          // conditions per group (0: RecV64)
+    const void* rec;    // RecV64, or CondRec64 (FP64 groups)
     const float2* cyp;  // mixed groups: (y, c pref), c = kW4C
     int cshift, ncell;
     double df;

@@ -4,13 +4,16 @@
 //  k_prep         "step one" per (line, condition): intensity S(T), Lorentz
 //                 width, Doppler width, the exact window of grid indices each
 //                 line reaches, and a packed record for step two.
+//  k_cells        (xs_cells.cu) per cell of consecutive lines, the moments that
+//                 stand for the lines' far wings.
 //  k_steptwo_*    "step two": a persistent grid of warps takes work items
-//                 (condition, tile of 32*P grid points) from an atomic
-//                 counter.  A warp finds the lines whose windows meet its tile
-//                 with a 32-way ballot search over the window arrays, streams
-//                 their records through a per-warp double-buffered shared
-//                 memory stage (cp.async), and accumulates its 32*P grid
-//                 points in registers, line by line in ascending order: a
+//                 (condition or group of conditions, tile of grid points) from
+//                 an atomic counter.  A warp finds the lines whose windows meet
+//                 its tile with a 32-way ballot search over the window arrays,
+//                 streams the records of those that are too near the tile for
+//                 their cells through a per-warp shared memory stage
+//                 (cp.async), accumulates the tile in registers -- a lane per
+//                 point or a lane per line -- and adds the far cells' series: a
 //                 fixed summation order, no atomics on the result.
 //
 // The reference computes the same sums with one CTA per grid point that scans
@@ -909,15 +912,16 @@ __device__ __forceinline__ double rcp_newton2_f64(double x) {
     return fma(r, fma(-x, r, 1.0), r);
 }
 
-// Adds the far cells of split s of S to the sums v of this lane's P points
-// f[] (one condition).  The heads of 32 cells are read at once, a cell per lane,
-// and handed round; two cells are summed side by side, so that the latency of
-// their moments' loads and of the chain is shared.  The warp's LS lane subsets
-// (sub = this lane's) take every LS-th cell; their sums are left apart.
-template <int P, int PM, int LS = 1>
+// Adds the far cells of split s of S to the sum v of this lane's point f (one
+// condition).  The heads of 32 cells are read at once, a cell per lane, and handed
+// round; two cells are summed side by side, so that the latency of their moments'
+// loads and of the chain is shared (one head and one chain at a time: 7.1 ms of
+// step two for the FP64 single point, 5.1 so).  The SUB neighbouring lanes of a
+// point take every SUB-th cell each (sub = this lane's); their sums are left apart.
+template <int PM, int SUB>
 __device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M, const LineRuns& r, int S, int s,
-                                              float bits, double ftlo, double fthi, const double (&f)[P],
-                                              double (&v)[P], int lane, int sub = 0) {
+                                              float bits, double ftlo, double fthi, double f, double& v, int lane,
+                                              int sub) {
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         const int c1 = h ? r.fd : r.fb;
@@ -927,42 +931,30 @@ __device__ __forceinline__ void add_far_cells(const CellHead* H, const double* M
             const CellHead hd = H[min(b + lane * S, c1 - 1)];
             const int terms = cell_terms<PM>(bits, fmax(ftlo - hd.c0, hd.c0 - fthi), hd.q);
 #pragma unroll 1
-            for (int k = 0; k < cnt; k += 2 * LS) {
-                double t[2][P], a[2][P];
+            for (int k = 0; k < cnt; k += 2 * SUB) {
+                double t[2], a[2] = {0.0, 0.0};
                 const double2* m[2];
                 int np = 0;
 #pragma unroll
                 for (int w = 0; w < 2; ++w) {
-                    const int kk = k + w * LS + sub;
+                    const int kk = k + w * SUB + sub;
                     const bool ok = kk < cnt;
                     const int at = ok ? kk : cnt - 1;
                     const double cc = __shfl_sync(0xffffffffu, hd.c0, at);
                     const float q = __shfl_sync(0xffffffffu, hd.q, at);
-                    const int n = __shfl_sync(0xffffffffu, terms, at);
-                    np = max(np, n);
+                    np = max(np, __shfl_sync(0xffffffffu, terms, at));
                     m[w] = reinterpret_cast<const double2*>(M + size_t(b + at * S) * PM);
-#pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        // (a cell past the end adds 0: t = 0)
-                        t[w][p] = ok ? double(q) * rcp_newton2_f64(f[p] - cc) : 0.0;
-                        a[w][p] = 0.0;
-                    }
+                    t[w] = ok ? double(q) * rcp_newton2_f64(f - cc) : 0.0;  // (past the end: adds 0)
                 }
-                if constexpr (LS > 1) np = __reduce_max_sync(0xffffffffu, np);
+                if constexpr (SUB > 1) np = __reduce_max_sync(0xffffffffu, np);
 #pragma unroll 2
                 for (int i = np / 2 - 1; i >= 0; --i) {
                     const double2 m0 = __ldg(m[0] + i), m1 = __ldg(m[1] + i);
-#pragma unroll
-                    for (int p = 0; p < P; ++p) {
-                        a[0][p] = fma(fma(a[0][p], t[0][p], m0.y), t[0][p], m0.x);
-                        a[1][p] = fma(fma(a[1][p], t[1][p], m1.y), t[1][p], m1.x);
-                    }
+                    a[0] = fma(fma(a[0], t[0], m0.y), t[0], m0.x);
+                    a[1] = fma(fma(a[1], t[1], m1.y), t[1], m1.x);
                 }
-#pragma unroll
-                for (int p = 0; p < P; ++p) {
-                    v[p] = fma(a[0][p] * t[0][p], t[0][p], v[p]);
-                    v[p] = fma(a[1][p] * t[1][p], t[1][p], v[p]);
-                }
+                v = fma(a[0] * t[0], t[0], v);
+                v = fma(a[1] * t[1], t[1], v);
             }
         }
     }
@@ -1871,11 +1863,11 @@ constexpr size_t mcx_warp_smem() {
 }
 
 // Sums w[0..V) over the lane bits 16 .. LP by halving exchanges: a lane ends
-// with the values base .. base + n - 1 of `kept` (fewer values than lanes: every
+// with kept() values from base() on (fewer values than lanes: every
 // lane of the remaining bits holds the same one).
 template <int V, int LP, class R = float>
 struct Halving {
-    static constexpr int kKept = V * LP / 32 > 1 ? V * LP / 32 : 1;
+    static constexpr int kept() { return V * LP / 32 > 1 ? V * LP / 32 : 1; }
     __device__ static __forceinline__ void sum(R (&w)[V], int lane) {
         int n = V;
 #pragma unroll
@@ -1918,7 +1910,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
     constexpr int NP = C / 2;
     constexpr int LP = 32 / LS, PT = 2 * LP;  // lane points, points of a row
     using Sum = Halving<2 * C, LP>;
-    constexpr int VF = Sum::kKept;
+    constexpr int VF = Sum::kept();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -2688,11 +2680,10 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
 
         const int jj = t0 + lane / SUB;
         if (runs.fa < runs.fb || runs.fc < runs.fd) {
-            const double f[1] = {F[min(jj, tl)]};
-            double far[1] = {0.0};
-            add_far_cells<1, kCellTermsMixed, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits,
-                                                   split, kCellBitsMixed, F[t0], F[tl], f, far, lane, lane % SUB);
-            sum += sum_neighbours<SUB>(far[0]);
+            double far = 0.0;
+            add_far_cells<kCellTermsMixed, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTermsMixed, runs, a.splits, split,
+                                                kCellBitsMixed, F[t0], F[tl], F[min(jj, tl)], far, lane, lane % SUB);
+            sum += sum_neighbours<SUB>(far);
         }
         if (lane % SUB == 0 && jj < t1) put_result(a, cond, split, jj, sum);
         __syncwarp();
@@ -2713,9 +2704,10 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
 // grids over dense lists, where a 32-point tile is wider than the near zone.
 //
 // Bound by the FP64 pipe and the instructions around it: 8 FP64 operations and
-// about 4 others per region-I pair.  B200, 1e7 lines, 7.5e5 points with cells:
-// the point-parallel kernel needed 7.0 ms, 26 % of the FP64 pipe and three other
-// instructions for each FP64 one.
+// about 4 others per region-I pair.  B200, 1e7 lines, 7.5e5 points with cells: 4.0
+// ms, with 32-point tiles 5.1 (64 more registers); the point-parallel kernel needed
+// 7.0, 26 % of the FP64 pipe and three other instructions for each FP64 one.  16
+// warps per SM (128 registers): 20 spill and take 4.15 ms.
 // ---------------------------------------------------------------------------
 template <int PT>
 constexpr size_t near64_warp_smem() {
@@ -2887,11 +2879,10 @@ __global__ void __launch_bounds__(kNearWarps * 32, 4) k_steptwo_near64(StepArgs 
         }
         const int jj = t0 + lane / SUB;
         if (runs.fa < runs.fb || runs.fc < runs.fd) {
-            const double f[1] = {F[min(jj, tl)]};
-            double far[1] = {0.0};
-            add_far_cells<1, kCellTerms64, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTerms64, runs, a.splits, split,
-                                                kCellBits64, F[t0], F[tl], f, far, lane, lane % SUB);
-            sum += sum_neighbours<SUB>(far[0]);
+            double far = 0.0;
+            add_far_cells<kCellTerms64, SUB>(a.chead + cell0, a.cmom + cell0 * kCellTerms64, runs, a.splits, split,
+                                             kCellBits64, F[t0], F[tl], F[min(jj, tl)], far, lane, lane % SUB);
+            sum += sum_neighbours<SUB>(far);
         }
         if (lane % SUB == 0 && jj < t1) put_result(a, c, split, jj, sum);
         __syncwarp();

@@ -219,14 +219,15 @@ int xs_engine_execute_host(xs_engine* e, const xs_options* opt, const xs_conditi
  *     the result, and so of the band integral (every pair's true value is
  *     positive for non-negative intensities).  Mixed Voigt: 1024 * 2^-24 =
  *     6.1e-5, above the rounding-error analysis of the FP32 steps (region I:
- *     offset, u, u^2 + 2y^2, the shared reciprocal, 32-line FP32 partial sums
- *     folded with compensation, 76 * 2^-24; regions II-IV: the FP32 x and y
+ *     offset, u, u^2 + 2y^2, the shared reciprocal, FP32 partial sums at most 32
+ *     deep, 76 * 2^-24; far wings summed by cells: less; regions II-IV: the FP32 x and y
  *     through the profile's sensitivity, at most 2 x^2 = 60.5, the FP32 W4
  *     forms and, for several conditions at once, the region-I value that
  *     step two adds there and the core pass takes back, at most 1.21 W4 --
  *     about 690 * 2^-24).
- *     FP64 (every FP64 result, Doppler and Gaussian included): 1e-12,
- *     summation order only.
+ *     FP64 (every FP64 result, Doppler and Gaussian included): 1e-12
+ *     (summation order, reciprocals, and the far wings' series, which leaves off
+ *     at most 3e-15 of a line's value).
  *   sampled_*: with xs_options.check_rows > 0 (mixed Voigt), measured on
  *     the sampled rows of every condition -- the largest relative error on
  *     points above 1e-6 of the rows' FP64 peak, and the relative error of

@@ -127,3 +127,21 @@ def test_cells_low_wavenumbers(engine, cuda, C):
         ref = reference(capi.CONV_GPU, fr, lines, c, grid.dfreq, c["gamma_scale"])
         assert_fp64_parity(f64[k], ref)
         assert_mixed_parity(mix[k], ref)
+
+
+@pytest.mark.parametrize("convention", [capi.CONV_GPU, capi.CONV_CPU])
+@pytest.mark.parametrize("n, df, make", [(60001, 0.1, "even"), (60001, 0.1, "uneven"), (16385, 0.04, "uneven")])
+def test_cells_single_condition_tiles(engine, cuda, convention, n, df, make):
+    """Single conditions at the default shape on 8-point tiles (a coarse grid over a dense list: a 32-point row
+    holds more lines than four cells) and on 16-point ones, both above the 1.2e7 pairs from which cells are used."""
+    lines = uneven(n, 51) if make == "uneven" else synth.random_lines(n, 1000.0, 1100.0, 2500.0, 1e-6, 1e2, seed=50)
+    grid = synth.Grid(985.0, 1117.0, int(132.0 / df))
+    fr = grid.freq()
+    for t, p in ((296.0, 1e-3), (1500.0, 10.0)):
+        cond = dict(temperature=t, partition=synth.partition_poly(t), mean_mass=17.03, pressure=1.0,
+                    ref_temp=296.0, cut=CUT)
+        ref = reference(convention, fr, lines, cond, grid.dfreq, p)
+        run = dict(conds=[dict(cond, gamma_scale=p)], convention=convention)
+        assert_fp64_parity(run_engine(engine, capi.VOIGT, lines, fr, cond, grid.dfreq, cuda, **run)[0], ref)
+        assert_mixed_parity(run_engine(engine, capi.VOIGT, lines, fr, cond, grid.dfreq, cuda,
+                                       precision=capi.MIXED, **run)[0], ref)

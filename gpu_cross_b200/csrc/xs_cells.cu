@@ -131,9 +131,11 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
 
 // Mixed precision, from the (y, c pref) pairs of the group layouts: the same in
 // FP32, the two poles as one packed FP32x2 operand, the sums over the lanes in
-// FP64.  The amplitudes are taken relative to the cell's largest, so their
-// range does not matter; a moment is off by about 1e-7 of itself, as one FP32
-// evaluation of the line is.
+// FP64.  The amplitudes c pref w are formed from c pref times a power of two that
+// brings the cell's largest to [1, 2), so that they are normal numbers however
+// weak the lines are (S below 1e-38 leaves c pref w, and its reciprocal, outside
+// the FP32 range); a moment is off by about 1e-7 of itself, as one FP32 evaluation
+// of the line is.
 // Bound by the FP32 pipe: 16 terms x 3 packed operations per (line, condition);
 // 40 conditions x 1e7 lines 4.77 ms in FP64, 2.1 in FP32.
 template <int C>
@@ -150,8 +152,8 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
     const float2* yp = a.cyp + size_t(g) * C * size_t(a.n);
     const float s2 = 0.70710678f;
 
-    // scale, reach and the largest amplitudes (all widened by 1e-6, far more
-    // than their FP32 rounding)
+    // scale and reach (widened by 1e-6, far more than their FP32 rounding) and
+    // the largest |c pref|
     float z2 = 0.0f, reach = 0.0f, big[C];
     bool good = true;
 #pragma unroll
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
             good = good && w > 0.0f && z < 1.0e30f && h < 1.0e30f && A < 1.0e37f;
             z2 = fmaxf(z2, z);
             reach = fmaxf(reach, h);
-            big[k] = fmaxf(big[k], A);
+            big[k] = fmaxf(big[k], fabsf(v.y));
         }
     }
     // non-negative floats order as their bit patterns
@@ -201,7 +203,9 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
 #pragma unroll
         for (int j = 0; j < C; ++j) bk = j == k ? big[j] : bk;
         bk = warp_max(bk);
-        const float rb = bk > 0.0f ? 1.0f / bk : 0.0f;
+        // 2^(127 - e), e the biased exponent of bk (0: zero or subnormal)
+        const int e = int(__float_as_uint(bk) >> 23);
+        const float sv = __uint_as_float(unsigned(max(254 - e, 1)) << 23);
         const double wq = a.dpw[g * C + k] * rq;
         float2 m[PM];
 #pragma unroll
@@ -211,8 +215,8 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
             const float2 v = yp[size_t(k) * size_t(a.n) + size_t(i)];
             const double nu = a.nu[i];
             const float w = float(nu * wq), d = float((nu - c0) * rq);  // in units of q
-            // |c pref| w / big <= 1, through nu dpw as above
-            const float A = v.y * (float(nu) * float(a.dpw[g * C + k])) * rb;
+            // c pref sv w, |c pref| sv < 2, through nu dpw as above
+            const float A = (v.y * sv) * (float(nu) * float(a.dpw[g * C + k]));
             const float s = s2 * w, gam = v.x * w, g2 = gam * gam;
             // I_k = A Im(zeta^k) of both poles by
             // I_{k+1} = 2 Re(zeta) I_k - |zeta|^2 I_{k-1}
@@ -242,8 +246,8 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
             }
         }
         t[0] += __shfl_xor_sync(0xffffffffu, t[0], 16);
-        // A stands for c pref w / big; the series wants c pref w / (2 q)
-        if (lane < PM) M[size_t(lane) * C + k] = t[0] * (0.5 * double(bk) * rq);
+        // A stands for c pref w sv; the series wants c pref w / (2 q)
+        if (lane < PM) M[size_t(lane) * C + k] = t[0] * (0.5 / double(sv) * rq);
     }
 }
 

@@ -387,12 +387,11 @@ __device__ __forceinline__ int prep_line(const PrepArgs& a, long i, int c, int* 
             // one condition per group of the line-parallel step two: offsets
             // scaled by g, x = (m - j) dfn + rn
             LineShX ls;
-            const bool far_m = !(fabs(m) < 16000000.0);
             const double xw = (cut + double(a.mixed_tile_span + 4) * df) * g;
-            ls.m = float(far_m ? 0.0 : m);
+            ls.m = float(fabs(m) < 16000000.0 ? m : 0.0);
             ls.dfn = float(df * g);
             ls.rn = float(((nu_p - f0) - m * df) * g);
-            ls.flags = (far_m ? kLineWhole : 0) |
+            ls.flags = (whole ? kLineWhole : 0) |
                        (!(xw * xw + y2 < kPairUMax) || !(fabs(Pc) < kPairPcMax) ? kLineWide : 0);
             ls.lo = lo;
             ls.hi = hi;
@@ -2577,6 +2576,9 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
             for (int j = jlo; j <= jhi; ++j) {
                 const float ax =
                     fabsf(whole ? float((nu - F[j]) / nu) * a.kx[cond] : fmaf(s.x - float(j), s.y, s.z));
+                // (a line at nu = 0 in the GPU convention has infinite or NaN x, y
+                // and pref: the pair is left out, not multiplied by 0)
+                if (!(ax < 1.0e18f)) continue;
                 float wf;
                 if (!all || (j >= iv.lo55 && j <= iv.hi55)) {
                     wf = float(1.0 / kW4C) *
@@ -2589,7 +2591,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
                     const float u = fmaf(ax, ax, region1_cy(y));
                     const float rat = u > 1.0e12f ? rcp_approx_f32(u)
                                                   : (u + 1.0f) * rcp_approx_f32(fmaf(u, u, 2.0f * y * y));
-                    wf = ax < 1.0e18f ? y * rat : 0.0f;
+                    wf = y * rat;
                 }
                 T[j - t0][lane] += v.y * wf;
             }

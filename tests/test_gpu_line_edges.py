@@ -1,0 +1,46 @@
+"""Voigt lines at the edges of what a list or a condition may hold, single
+conditions and batches, on calls below and above the pair count from which far
+wings go by cells."""
+import numpy as np
+import pytest
+
+from gpu_cross_b200 import capi, synth
+
+from helpers import assert_mixed_parity, run_engine
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def engine(cuda):
+    e = capi.Engine(0)
+    yield e
+    e.close()
+
+
+def conditions(count, **kw):
+    base = dict(temperature=300.0, partition=synth.partition_poly(300.0), mean_mass=17.03, pressure=1.0, ref_temp=296.0,
+                cut=25.0)
+    return [dict(base, gamma_scale=p, **kw) for p in (0.1, 1.0)[:count]]
+
+
+@pytest.mark.parametrize("convention", [capi.CONV_GPU, capi.CONV_CPU])
+@pytest.mark.parametrize("n, points", [(300, 4001), (20000, 7000)])
+@pytest.mark.parametrize("C", [1, 2])
+def test_line_at_zero_wavenumber(engine, cuda, convention, n, points, C):
+    """A centre of 0 in reach of the grid.  GPU convention: its Doppler width is
+    0, x infinite, and a mixed call leaves it out (FP64 gives the reference's NaN
+    there), so the FP64 spectrum of the other lines is the reference; the CPU
+    convention takes the centre as 1e-6."""
+    lines = synth.random_lines(n, 1.0, 60.0, 2500.0, 1e-6, 1e2, seed=71)
+    lines.nu[0] = 0.0
+    grid = synth.Grid(0.5, 0.5 + points * 0.01, points)
+    conds = conditions(C)
+    args = (grid.freq(), conds[0], grid.dfreq, cuda)
+    run = dict(conds=conds, C=C, convention=convention)
+    rest = lines.slice(1, n) if convention == capi.CONV_GPU else lines
+    ref = run_engine(engine, capi.VOIGT, rest, *args, **dict(run, C=0))
+    got = run_engine(engine, capi.VOIGT, lines, *args, precision=capi.MIXED, **run)
+    assert np.isfinite(got).all()
+    for k in range(C):
+        assert_mixed_parity(got[k], ref[k])

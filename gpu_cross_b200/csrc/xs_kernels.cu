@@ -303,6 +303,9 @@ __device__ __forceinline__ int prep_line(const PrepArgs& a, long i, int c, int* 
 
     if (tc_write) a.L.tc_s[i] = S;
     if (KIND == kVoigt) {
+        // an empty window has length 0 (a negative cut, from a negative pressure,
+        // puts hi below lo; step two takes hi - lo as unsigned)
+        if (hi < lo) hi = lo;
         double pw = 0.0;
         if (!streamed) {
             pw = tc_read ? a.L.tc_pw[i] : pow(C.tratio, a.L.nexp[i]);

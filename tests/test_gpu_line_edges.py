@@ -44,3 +44,19 @@ def test_line_at_zero_wavenumber(engine, cuda, convention, n, points, C):
     assert np.isfinite(got).all()
     for k in range(C):
         assert_mixed_parity(got[k], ref[k])
+
+
+@pytest.mark.parametrize("convention", [capi.CONV_GPU, capi.CONV_CPU])
+@pytest.mark.parametrize("precision", [capi.FP64, capi.MIXED])
+@pytest.mark.parametrize("C, P", [(1, 0), (1, 1), (1, 2), (2, 0)])
+def test_negative_cut_reaches_nothing(engine, cuda, convention, precision, C, P):
+    """The cut rule gives 25 P: a negative pressure leaves every window empty."""
+    lines = synth.random_lines(400, 1000.0, 1040.0, 2500.0, 1e-6, 1e2, seed=73)
+    grid = synth.Grid(995.0, 1045.0, 5000)
+    for pressure in (-1e-4, -0.02, -1.0):
+        conds = conditions(C, cut=-1.0)
+        for c in conds:
+            c["pressure"] = pressure
+        got = run_engine(engine, capi.VOIGT, lines, grid.freq(), conds[0], grid.dfreq, cuda, conds=conds, C=C, P=P,
+                         convention=convention, precision=precision)
+        assert not got.any()

@@ -3315,7 +3315,9 @@ cudaError_t launch_prep(int kind, int conv, bool mixed, const PrepArgs& a, cudaS
         const int ncache = a.nclass <= kMaxClassCache ? a.nclass : 0;
         const size_t smem = sizeof(double) * 3 * size_t(ncache) * 256;
         auto go = [&](auto kernel) {
-            if (smem > 48 * 1024 &&
+            // (the kernel's static arrays count against the 48 KB that need no
+            // attribute: 8 classes are exactly 48 KB without them)
+            if (smem + sizeof(int) * 2 * kMaxCond * 8 > 48 * 1024 &&
                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
                 return cudaGetLastError();
             kernel<<<nblk, 256, smem, stream>>>(a);

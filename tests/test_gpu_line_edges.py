@@ -60,3 +60,18 @@ def test_negative_cut_reaches_nothing(engine, cuda, convention, precision, C, P)
         got = run_engine(engine, capi.VOIGT, lines, grid.freq(), conds[0], grid.dfreq, cuda, conds=conds, C=C, P=P,
                          convention=convention, precision=precision)
         assert not got.any()
+
+
+@pytest.mark.parametrize("temperatures", [1, 7, 8, 9, 16])
+def test_batches_of_distinct_temperatures(engine, cuda, temperatures):
+    """Step one keeps the values of up to 16 temperatures per line in shared
+    memory, 6 KB each beside its own 4 KB: 8 of them cross 48 KB."""
+    lines = synth.random_lines(3000, 1000.0, 1040.0, 2500.0, 1e-6, 1e2, seed=75)
+    grid = synth.Grid(995.0, 1045.0, 500)
+    conds = [dict(c, temperature=t, partition=synth.partition_poly(t))
+             for t in np.linspace(250.0, 2500.0, temperatures) for c in conditions(2)]
+    args = (grid.freq(), conds[0], grid.dfreq, cuda)
+    ref = run_engine(engine, capi.VOIGT, lines, *args, conds=conds)
+    got = run_engine(engine, capi.VOIGT, lines, *args, conds=conds, C=2, precision=capi.MIXED)
+    for k in range(len(conds)):
+        assert_mixed_parity(got[k], ref[k])

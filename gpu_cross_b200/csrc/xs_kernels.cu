@@ -1830,9 +1830,11 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
 // 8-point one 1.6 and 0.8).  What bounds it is shared memory: a lane needs 24 +
 // 8 C bytes of every line it takes, 128 bytes a wavefront for the warp, so two
 // points per lane halve it, and 2 y^2 comes from Cy = y^2 - 1/2 instead of a
-// third array.  Every LS groups of 32 lines the FP32 sums (16 deep) are added
-// up over the lane subsets by halving exchanges, each lane keeping 2 C / LS of
-// them in FP64.
+// third array.  After each group of 32 lines the FP32 sums (32 / LS lines deep)
+// are added up over the lane subsets by halving exchanges, each lane keeping
+// 2 C / LS of them in FP64.  (Every LS groups only, 0.5 of 24.1 ms less for the
+// 40-condition sweep, the error at 10 atm is 0.23e-7 instead of 0.18e-7, and
+// 0.57e-7 instead of 0.43e-7 for a tenth of the lines.)
 // ---------------------------------------------------------------------------
 // Resident blocks per SM the mixed multi-condition kernel asks the compiler
 // to fit (register budget): 20 warps per SM at 8 conditions and 4 warps per
@@ -2179,7 +2181,7 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                     line_step(true, X1, r, p, in1, acc[1][p]);
                 }
             }
-            if ((gi & (LS - 1)) == LS - 1 || gi + 1 == ngroups) {
+            {
                 float w[2 * C];
 #pragma unroll
                 for (int v = 0; v < C; ++v) {
@@ -2398,12 +2400,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // point of the tile into PT accumulators.  The line's constants are read once
 // per lane (a broadcast to every lane costs a shared-memory wavefront per 4
 // bytes), and the lines of a group, being neighbours, are in the same W4 region
-// at the same point.  Every 8 groups of lines the accumulators are summed over
-// the lanes by halving exchanges and added in FP64 (sums 8 + 5 deep: 4.5e-8 of
-// the result in the 2-norm, 7.0e-8 with 32 groups; the point-parallel kernel
-// 5.3e-8).  Tiles of 16 points (32: 2.72 against 2.50 ms at the sizes below), of
-// 8 on coarse grids over dense lists, where 16 points are wider than the near
-// zone.
+// at the same point.  Every 4 groups of lines the accumulators are summed over
+// the lanes by halving exchanges and added in FP64 (sums 4 + 5 deep; 3e5 lines on
+// 5e4 points at 10 atm: 1.66e-8 of the result in the 2-norm, 1.93e-8 and 2 % less
+// time with 8 groups; a lane per point 2.25e-8).  Tiles of 16 points (32: 2.72 against
+// 2.50 ms at the sizes below), of 8 on coarse grids over dense lists, where 16
+// points are wider than the near zone.
 //
 // Two evaluations share one reciprocal, 1/dA = dB / (dA dB) (narrow lines,
 // kPairUMax).  Groups with lines of the core reach choose region I or II per
@@ -2678,7 +2680,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a)
             } else {
                 plain_group(std::true_type(), s, win, v);
             }
-            if ((gi & 7) == 7) fold();
+            if ((gi & 3) == 3) fold();
         }
         cp_async_wait<0>();
         fold();

@@ -120,6 +120,7 @@ _SIGS = {
     "xs_engine_set_stream": (_I, [_VP, _VP]),
     "xs_engine_sync": (_I, [_VP]),
     "xs_engine_scratch_bytes": (_I, [_VP, ctypes.POINTER(_SZ)]),
+    "xs_engine_limit_scratch": (_I, [_VP, _SZ]),
     "xs_scratch_bytes_needed": (_SZ, [ctypes.POINTER(Options), _I, _SZ]),
     "xs_engine_execute": (_I, [_VP, ctypes.POINTER(Options), ctypes.POINTER(Condition), _I,
                                ctypes.POINTER(Lines), ctypes.POINTER(GridC), _VP, _SZ]),
@@ -250,6 +251,10 @@ class Engine:
         v = ctypes.c_size_t()
         check(lib().xs_engine_scratch_bytes(self.h, ctypes.byref(v)))
         return int(v.value)
+
+    def limit_scratch(self, nbytes: int) -> None:
+        """xs_engine_limit_scratch: most bytes the scratch may grow to (0: no limit)."""
+        check(lib().xs_engine_limit_scratch(self.h, nbytes))
 
     def execute(self, opts: Options, conds: list[Condition], lines: Lines, grid: GridC, out_ptr: int,
                 out_stride: int = 0) -> None:

@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -78,13 +79,15 @@ struct xs_engine {
     int num_sms = 0;
     void* scratch = nullptr;
     size_t scratch_cap = 0;
+    size_t scratch_limit = SIZE_MAX;  // xs_engine_limit_scratch
+    size_t no_room = SIZE_MAX;        // least scratch with cells that did not fit
     unsigned* d_words = nullptr;  // [0] error bits, [1] work counter
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     bool timed = false;
-    // host line lists (xs_engine_execute_host): a copy stream and an event
-    // per slice, made on first use
     std::shared_ptr<void> stream_ws;  // xs_stream_execute's buffers
     std::mutex stream_mu;
+    // host line lists (xs_engine_execute_host): a copy stream and an event
+    // per slice, made on first use
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t pev[kMaxPieces + 1] = {};
     // error statement of the last execute: the a-priori bound and, with
@@ -177,6 +180,23 @@ CondDev make_cond(const xs_options& o, const xs_condition& c) {
         d.cut = o.half_width * 10.0;
     }
     return d;
+}
+
+// Device memory for the engine's scratch (a limit counts as a full card).
+cudaError_t alloc_scratch(xs_engine* e, size_t bytes) {
+    if (bytes > e->scratch_limit) return cudaErrorMemoryAllocation;
+    return cudaMalloc(&e->scratch, bytes);
+}
+
+// Whether `bytes` would fit in the present scratch's place.
+bool room_for(const xs_engine* e, size_t bytes) {
+    size_t fr = 0, tot = 0;
+    if (bytes > e->scratch_limit) return false;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes <= fr + e->scratch_cap;
 }
 
 // Bytes of the cell heads and moments (both multiples of 16) of one launch.
@@ -357,6 +377,13 @@ int xs_engine_sync(xs_engine* e) {
 int xs_engine_scratch_bytes(xs_engine* e, size_t* bytes) {
     if (!e || !bytes) return fail(XS_ERR_INVALID, "xs_engine_scratch_bytes: NULL argument");
     *bytes = e->scratch_cap;
+    return XS_OK;
+}
+
+int xs_engine_limit_scratch(xs_engine* e, size_t bytes) {
+    if (!e) return fail(XS_ERR_INVALID, "xs_engine_limit_scratch: NULL engine");
+    std::lock_guard<std::mutex> lk(e->mu);
+    e->scratch_limit = bytes ? bytes : SIZE_MAX;
     return XS_OK;
 }
 
@@ -707,25 +734,38 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         scratch = ov->scratch;
         if (ov->words) words = ov->words;
     } else {
+        // no allocation and no wait inside a stream capture
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (need > e->scratch_cap && cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess) cudaGetLastError();
+        const bool capturing = cap == cudaStreamCaptureStatusActive;
+        if (need > e->scratch_cap && cshift && need >= e->no_room && (capturing || !room_for(e, need))) {
+            // a call of this size had no room for its cells before
+            cshift = 0;
+            layout();
+        }
         if (need > e->scratch_cap) {
+            if (capturing)
+                return fail(XS_ERR_STATE, "the engine's scratch is too small for this call and cannot grow inside a "
+                                          "stream capture: execute it once before");
             XS_CU(cudaStreamSynchronize(e->stream));
             cudaFree(e->scratch);
             e->scratch = nullptr;
             e->scratch_cap = 0;
-            cudaError_t err = cudaMalloc(&e->scratch, need);
+            cudaError_t err = alloc_scratch(e, need);
             if (err == cudaErrorMemoryAllocation && !streamed_call && e->stream_mu.try_lock()) {
                 // what an earlier streamed call left
                 cudaGetLastError();
                 e->stream_ws.reset();
                 e->stream_mu.unlock();
-                err = cudaMalloc(&e->scratch, need);
+                err = alloc_scratch(e, need);
             }
             if (err == cudaErrorMemoryAllocation && cshift) {
                 // without the cells: slower, but the records may still fit
                 cudaGetLastError();
+                e->no_room = std::min(e->no_room, need);
                 cshift = 0;
                 layout();
-                err = cudaMalloc(&e->scratch, need);
+                err = alloc_scratch(e, need);
             }
             if (err != cudaSuccess) {
                 cudaGetLastError();
@@ -1052,7 +1092,7 @@ int engine_reserve(xs_engine* e, size_t bytes) {
     cudaFree(e->scratch);
     e->scratch = nullptr;
     e->scratch_cap = 0;
-    cudaError_t err = cudaMalloc(&e->scratch, bytes);
+    cudaError_t err = alloc_scratch(e, bytes);
     if (err != cudaSuccess) {
         cudaGetLastError();
         return cuda_fail(err, "cudaMalloc(scratch)");

@@ -185,7 +185,16 @@ int xs_engine_set_stream(xs_engine* e, void* stream);
 int xs_engine_sync(xs_engine* e);
 /* Device bytes held by the engine's scratch (records, windows, counters). */
 int xs_engine_scratch_bytes(xs_engine* e, size_t* bytes);
-/* Upper bound on scratch bytes xs_engine_execute needs for this shape. */
+/* Most device bytes the engine's scratch may grow to from now on (0: whatever
+ * the device has).  A call whose far-wing cells do not fit goes without them,
+ * line by line and slower; one whose records do not fit fails with
+ * XS_ERR_NOMEM. */
+int xs_engine_limit_scratch(xs_engine* e, size_t bytes);
+/* Scratch bytes of step one's records and windows, at most, for this shape.  A
+ * call adds, where it uses them: far-wing cells (up to 8 bytes per line and
+ * condition), line-split parts (8 bytes per part, condition and grid point;
+ * with automatic splits up to 64 MiB, one condition's cells included) and the
+ * values of check_rows. */
 size_t xs_scratch_bytes_needed(const xs_options* opt, int ncond, size_t n_lines);
 
 /* For each condition c: out[c*out_stride + j] += sigma_c(f_j) for j in

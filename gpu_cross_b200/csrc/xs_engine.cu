@@ -136,6 +136,10 @@ struct Shape {
 std::mutex g_tune_mu;
 std::map<std::string, Shape> g_tune;
 
+// First part of every key: entries of tables measured on earlier kernels, whose
+// shapes mean something else now, are left out by xs_tune_load.
+constexpr char kTuneVersion[] = "k2.";
+
 std::string shape_key(const xs_options& o, const xs_condition* conds, int ncond, long n, int points) {
     double cutmax = 0.0;
     for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(o, conds[c]).cut);
@@ -143,7 +147,7 @@ std::string shape_key(const xs_options& o, const xs_condition* conds, int ncond,
     const double density = double(n) * win / (double(points) + win);
     auto lg = [](double v) { return v < 1.0 ? 0 : int(std::floor(std::log2(v))); };
     char buf[96];
-    std::snprintf(buf, sizeof(buf), "p%d.v%d.x%d.c%d.g%d.d%d", o.profile, o.convention, o.precision,
+    std::snprintf(buf, sizeof(buf), "%sp%d.v%d.x%d.c%d.g%d.d%d", kTuneVersion, o.profile, o.convention, o.precision,
                   ncond < kMaxCond ? ncond : kMaxCond, lg(double(points)), lg(density));
     return buf;
 }
@@ -1285,7 +1289,8 @@ int xs_tune_load(const char* path) {
     Shape sh{};
     std::lock_guard<std::mutex> lk(g_tune_mu);
     while (std::fscanf(f, "%95s %d %d %d %lf", key, &sh.P, &sh.W, &sh.C, &sh.ms) == 5) {
-        const bool ok = (sh.P == 1 || sh.P == 2 || sh.P == 4 || sh.P == 8) && (sh.W == 4 || sh.W == 8) &&
+        const bool ok = std::strncmp(key, kTuneVersion, sizeof(kTuneVersion) - 1) == 0 &&
+                        (sh.P == 1 || sh.P == 2 || sh.P == 4 || sh.P == 8) && (sh.W == 4 || sh.W == 8) &&
                         (sh.C == 0 || sh.C == 1 || sh.C == 2 || sh.C == 4 || sh.C == 8);
         if (ok) g_tune[key] = sh;
     }

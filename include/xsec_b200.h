@@ -286,7 +286,8 @@ int xs_measure_peaks(int device, double* fp32_tflops, double* fp64_tflops, doubl
  * grid points and of the lines per point), and reports it.  Later calls with
  * points_per_thread = warps_per_block = conditions_per_warp = 0 use it.  `out`
  * is accumulated into many times: clear it afterwards.  The table lives in
- * the process; xs_tune_save / xs_tune_load keep it in a text file. */
+ * the process; xs_tune_save / xs_tune_load keep it in a text file (entries that
+ * an earlier version of the kernels was measured with are left out on loading). */
 typedef struct {
     int points_per_thread, warps_per_block, conditions_per_warp;
     double ms;       /* step one + step two of the chosen shape */

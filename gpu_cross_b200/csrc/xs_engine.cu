@@ -646,9 +646,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Scratch layout for one group of conditions.
     const int group = ncond < kMaxCond ? ncond : kMaxCond;
     const ScratchPlan plan = plan_scratch(kind, mixed, size_t(n), group, 0, CG);
-    if (near || near64) W = 4;
-    int occ = near ? steptwo_near_blocks_per_sm(row)
-              : near64 ? steptwo_near64_blocks_per_sm(row)
+    int occ = near || near64 ? steptwo_near_blocks_per_sm(mixed, row, W)
               : CG ? steptwo_mc_blocks_per_sm(mixed, CG, W, row)
                    : steptwo_blocks_per_sm(kind, opt->convention, mixed, P, W);
     if (occ < 1) {
@@ -663,8 +661,9 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // or coarse grids over many lines) most of the GPU idles while each warp
     // walks a long line list, and with a few items per warp the last items
     // leave a tail.  Each tile's lines are then split into parts taken by
-    // different warps -- enough for about 16 items per resident warp, at
-    // least 128 or 256 lines per part, the parts' buffer within kMaxPartBytes.
+    // different warps -- enough for 16 items per resident warp (6 with cells, 4
+    // for erf profiles), at least 128 or 256 lines per part (64 with cells), the
+    // parts' buffer within kMaxPartBytes.
     // The count depends only on the call's sizes and the SM count.
     const int tile_pts = (CG || near64) ? row : 32 * P;
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
@@ -1027,8 +1026,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
         const long want = (long(sa.n_items) + W - 1) / W;
         const int blocks = int(std::min<long>(want, long(occ) * e->num_sms));
-        err = near ? launch_steptwo_near(row, blocks, sa, st)
-              : near64 ? launch_steptwo_near64(row, blocks, sa, st)
+        err = near || near64 ? launch_steptwo_near(mixed, row, W, blocks, sa, st)
               : CG ? launch_steptwo_mc(mixed, CG, W, row, blocks, sa, st)
                 : launch_steptwo(kind, opt->convention, mixed, P, W, blocks, sa, st);
         if (err != cudaSuccess) return cuda_fail(err, "step two launch");

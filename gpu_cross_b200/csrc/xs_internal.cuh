@@ -403,14 +403,11 @@ cudaError_t launch_check_snapshot(const CheckArgs& a, cudaStream_t stream);
 // (launched after the call's last kernel).
 cudaError_t launch_check_rows(const CheckArgs& a, cudaStream_t stream);
 
-// Mixed single-condition step two with cells, lane = line (LineShX, civ, cyp
-// records, groups of one condition), W4 regions II-IV included; 4 warps a block.
-// Tiles of `row` = 8, 16 or 32 points.
-cudaError_t launch_steptwo_near(int row, int blocks, const StepArgs& a, cudaStream_t stream);
-int steptwo_near_blocks_per_sm(int row);
-// FP64 single-condition step two on tiles of `row` = 16 or 8 points, lane = line.
-cudaError_t launch_steptwo_near64(int row, int blocks, const StepArgs& a, cudaStream_t stream);
-int steptwo_near64_blocks_per_sm(int row);
+// Single-condition step two on tiles of `row` = 16 or 8 points, lane = line, 4 or 8
+// warps a block.  Mixed: LineShX, civ, cyp records, groups of one condition, W4
+// regions II-IV included; FP64: RecV64.
+cudaError_t launch_steptwo_near(bool mixed, int row, int warps, int blocks, const StepArgs& a, cudaStream_t stream);
+int steptwo_near_blocks_per_sm(bool mixed, int row, int warps);
 
 // Multi-condition step two (Voigt): C conditions per warp.
 // Rows of `row` = 32 or 8 points.

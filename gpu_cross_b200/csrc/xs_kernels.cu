@@ -2421,7 +2421,6 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // coarse sweep (20.7 against 12.6 ms).
 // ---------------------------------------------------------------------------
 constexpr int kNearRow = 33;
-constexpr int kNearWarps = 4;
 // Two stages of offsets and flags, windows and (y, pref), and the table.
 template <int PT>
 constexpr size_t near_warp_smem() {
@@ -2435,8 +2434,8 @@ __device__ __forceinline__ double sum_neighbours(double v) {
     return v;
 }
 
-template <int PT>
-__global__ void __launch_bounds__(kNearWarps * 32, 5) k_steptwo_near(StepArgs a) {
+template <int PT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     constexpr int SUB = 32 / PT;  // lanes to a point where lanes stand for points
@@ -2721,8 +2720,8 @@ constexpr size_t near64_warp_smem() {
     return 64 * sizeof(RecV64) + sizeof(double) * PT * kCoreRow64 + sizeof(double) * PT;
 }
 
-template <int PT>
-__global__ void __launch_bounds__(kNearWarps * 32, 4) k_steptwo_near64(StepArgs a) {
+template <int PT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) k_steptwo_near64(StepArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     constexpr int SUB = 32 / PT;        // lanes to a point where lanes stand for points
@@ -3389,47 +3388,36 @@ cudaError_t launch_steptwo_mc(bool mixed, int C, int warps, int row, int blocks,
     return dispatch_mc(mixed, C, warps, row, blocks, a, stream, nullptr);
 }
 
-static cudaError_t dispatch_near(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
+template <int WARPS>
+static cudaError_t dispatch_near_w(bool mixed, int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
     auto go = [&](auto kernel, size_t smem) {
-        return run_group_kernel(kernel, kNearWarps * 32, kNearWarps * smem, blocks, a, st, occ);
+        return run_group_kernel(kernel, WARPS * 32, WARPS * smem, blocks, a, st, occ);
     };
-    switch (row) {
-        case 8: return go(k_steptwo_near<8>, near_warp_smem<8>());
-        case 16: return go(k_steptwo_near<16>, near_warp_smem<16>());
-        default: return cudaErrorInvalidValue;
-    }
-}
-
-cudaError_t launch_steptwo_near(int row, int blocks, const StepArgs& a, cudaStream_t stream) {
-    if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
-    return dispatch_near(row, blocks, a, stream, nullptr);
-}
-
-int steptwo_near_blocks_per_sm(int row) {
-    StepArgs dummy{};
-    int occ = 0;
-    return dispatch_near(row, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
-}
-
-static cudaError_t dispatch_near64(int row, int blocks, const StepArgs& a, cudaStream_t st, int* occ) {
     if (row == 16)
-        return run_group_kernel(k_steptwo_near64<16>, kNearWarps * 32, kNearWarps * near64_warp_smem<16>(), blocks, a, st,
-                                occ);
+        return mixed ? go(k_steptwo_near<16, WARPS>, near_warp_smem<16>())
+                     : go(k_steptwo_near64<16, WARPS>, near64_warp_smem<16>());
     if (row == 8)
-        return run_group_kernel(k_steptwo_near64<8>, kNearWarps * 32, kNearWarps * near64_warp_smem<8>(), blocks, a, st,
-                                occ);
+        return mixed ? go(k_steptwo_near<8, WARPS>, near_warp_smem<8>())
+                     : go(k_steptwo_near64<8, WARPS>, near64_warp_smem<8>());
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_steptwo_near64(int row, int blocks, const StepArgs& a, cudaStream_t stream) {
-    if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
-    return dispatch_near64(row, blocks, a, stream, nullptr);
+static cudaError_t dispatch_near(bool mixed, int row, int warps, int blocks, const StepArgs& a, cudaStream_t st,
+                                 int* occ) {
+    if (warps == 4) return dispatch_near_w<4>(mixed, row, blocks, a, st, occ);
+    if (warps == 8) return dispatch_near_w<8>(mixed, row, blocks, a, st, occ);
+    return cudaErrorInvalidValue;
 }
 
-int steptwo_near64_blocks_per_sm(int row) {
+cudaError_t launch_steptwo_near(bool mixed, int row, int warps, int blocks, const StepArgs& a, cudaStream_t stream) {
+    if (blocks <= 0 || a.n_items <= 0) return cudaSuccess;
+    return dispatch_near(mixed, row, warps, blocks, a, stream, nullptr);
+}
+
+int steptwo_near_blocks_per_sm(bool mixed, int row, int warps) {
     StepArgs dummy{};
     int occ = 0;
-    return dispatch_near64(row, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
+    return dispatch_near(mixed, row, warps, 0, dummy, nullptr, &occ) == cudaSuccess ? occ : 0;
 }
 
 int steptwo_mc_blocks_per_sm(bool mixed, int C, int warps, int row) {

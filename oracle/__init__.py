@@ -48,10 +48,16 @@ def build(ref: bool = True) -> None:
 _libs: dict[str, ctypes.CDLL] = {}
 
 
+class ReferenceMissing(FileNotFoundError):
+    """A checker built from the reference's sources is not there (no reference
+    tree was at hand when oracle/ was built)."""
+
+
 def _load(path: str) -> ctypes.CDLL:
     if path not in _libs:
         if not os.path.exists(path):
-            raise FileNotFoundError(f"{path} is not built (run make -C oracle)")
+            missing = FileNotFoundError if path == LIB_ORACLE else ReferenceMissing
+            raise missing(f"{path} is not built (run make -C oracle)")
         _libs[path] = ctypes.CDLL(path)
     return _libs[path]
 

@@ -547,9 +547,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         }
     }
     // whether the call's far wings can go by cells on tiles of `pts` points
-    auto cells_at = [&](int pts) {
-        return !(ov && ov->scratch) && cell_shift(*opt, conds, ncond, n, *grid, pts) > 0;
-    };
+    auto cells_at = [&](int pts) { return cell_shift(*opt, conds, ncond, n, *grid, pts) > 0; };
     const bool cells = cells_at(32);
     const bool narrow_tiles = P <= 1;  // the caller did not ask for wide ones
     {
@@ -632,9 +630,8 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Tiles and rows of 8 points where a 32-point one is wider than what has to be
     // taken line by line beside it (about 6 cells).
     const bool wide_row = cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid);
-    const bool near =
-        mixed && C == 1 && !(ov && ov->scratch) && (P == 1 || (narrow_tiles && (cells || wide_row)));
-    const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1 && !(ov && ov->scratch);
+    const bool near = mixed && C == 1 && (P == 1 || (narrow_tiles && (cells || wide_row)));
+    const bool near64 = kind == XS_VOIGT && !mixed && C == 1 && P == 1;
     const int CG = near || C > 1 ? C : 0;
     const int row = C > 1 ? (wide_row ? 8 : 32) : wide_row ? 8 : 16;
     if (opt->line_splits < 0 || opt->line_splits > kMaxSplits)
@@ -669,9 +666,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     const int tiles = (grid->points + tile_pts - 1) / tile_pts;
     // (tiles wider than 32 points, asked for by the caller, go line by line)
     int cshift = near || near64 || C > 1 ? cell_shift(*opt, conds, ncond, n, *grid, tile_pts) : 0;
-    if (ov && ov->scratch) cshift = 0;
     int S = opt->line_splits;
-    if (ov && ov->scratch) S = 1;  // a fixed caller scratch holds no parts
     if (S == 0) {
         const long items = long(tiles) * (CG ? group / CG : group);
         const long warps = long(occ) * W * e->num_sms;
@@ -729,57 +724,51 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     };
     layout();
 
-    void* scratch = nullptr;
-    unsigned* words = e->d_words;
-    if (ov && ov->scratch) {
-        if (need > ov->scratch_bytes)
-            return fail(XS_ERR_NOMEM, "scratch larger than the caller-provided area");
-        scratch = ov->scratch;
-        if (ov->words) words = ov->words;
-    } else {
-        // no allocation and no wait inside a stream capture
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (need > e->scratch_cap && cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess) cudaGetLastError();
-        const bool capturing = cap == cudaStreamCaptureStatusActive;
-        if (need > e->scratch_cap && cshift && need >= e->no_room && (capturing || !room_for(e, need))) {
-            // a call of this size had no room for its cells before
+    // no allocation and no wait inside a stream capture
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(e->stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        cap = cudaStreamCaptureStatusNone;
+    }
+    const bool capturing = cap == cudaStreamCaptureStatusActive;
+    if (need > e->scratch_cap && cshift && need >= e->no_room && (capturing || !room_for(e, need))) {
+        // a call of this size had no room for its cells before
+        cshift = 0;
+        layout();
+    }
+    if (need > e->scratch_cap) {
+        if (capturing)
+            return fail(XS_ERR_STATE, "the engine's scratch is too small for this call and cannot grow inside a "
+                                      "stream capture: execute it once before");
+        XS_CU(cudaStreamSynchronize(e->stream));
+        cudaFree(e->scratch);
+        e->scratch = nullptr;
+        e->scratch_cap = 0;
+        cudaError_t err = alloc_scratch(e, need);
+        if (err == cudaErrorMemoryAllocation && !streamed_call && e->stream_mu.try_lock()) {
+            // what an earlier streamed call left
+            cudaGetLastError();
+            e->stream_ws.reset();
+            e->stream_mu.unlock();
+            err = alloc_scratch(e, need);
+        }
+        if (err == cudaErrorMemoryAllocation && cshift) {
+            // without the cells: slower, but the records may still fit
+            cudaGetLastError();
+            e->no_room = std::min(e->no_room, need);
             cshift = 0;
             layout();
+            err = alloc_scratch(e, need);
         }
-        if (need > e->scratch_cap) {
-            if (capturing)
-                return fail(XS_ERR_STATE, "the engine's scratch is too small for this call and cannot grow inside a "
-                                          "stream capture: execute it once before");
-            XS_CU(cudaStreamSynchronize(e->stream));
-            cudaFree(e->scratch);
-            e->scratch = nullptr;
-            e->scratch_cap = 0;
-            cudaError_t err = alloc_scratch(e, need);
-            if (err == cudaErrorMemoryAllocation && !streamed_call && e->stream_mu.try_lock()) {
-                // what an earlier streamed call left
-                cudaGetLastError();
-                e->stream_ws.reset();
-                e->stream_mu.unlock();
-                err = alloc_scratch(e, need);
-            }
-            if (err == cudaErrorMemoryAllocation && cshift) {
-                // without the cells: slower, but the records may still fit
-                cudaGetLastError();
-                e->no_room = std::min(e->no_room, need);
-                cshift = 0;
-                layout();
-                err = alloc_scratch(e, need);
-            }
-            if (err != cudaSuccess) {
-                cudaGetLastError();
-                return cuda_fail(err, "cudaMalloc(scratch)");
-            }
-            e->scratch_cap = need;
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            return cuda_fail(err, "cudaMalloc(scratch)");
         }
-        scratch = e->scratch;
+        e->scratch_cap = need;
     }
     if (ov && ov->alloc_only) return XS_OK;
-    char* base = static_cast<char*>(scratch);
+    char* base = static_cast<char*>(e->scratch);
+    unsigned* words = e->d_words;
     e->bound_rel = error_bound(kind, mixed);
     e->chk_rows = nchk;
     e->chk_ncond = ncond;
@@ -819,12 +808,7 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
     // Inside a stream capture the timing events must become event-record
     // nodes of the graph (cudaEventRecordExternal); outside one, a plain
     // record (the external flag is refused there).
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
-        cudaGetLastError();
-        cap = cudaStreamCaptureStatusNone;
-    }
-    const unsigned ev_flags = (cap == cudaStreamCaptureStatusActive) ? cudaEventRecordExternal : 0u;
+    const unsigned ev_flags = capturing ? cudaEventRecordExternal : 0u;
     cudaError_t err = launch_grid_check(G, words, reinterpret_cast<int*>(base + plan.off_kc), words + 1, st);
     if (err != cudaSuccess) return cuda_fail(err, "grid check launch");
     int launched = 1;

@@ -14,9 +14,6 @@ struct CondDev;
 
 // Optional knobs of one execute call.
 struct ExecOverride {
-    void* scratch = nullptr;      // caller-provided scratch area (device)
-    size_t scratch_bytes = 0;
-    unsigned* words = nullptr;    // caller-provided error word + counter (device)
     bool no_timing = false;       // skip the CUDA events
     bool alloc_only = false;      // only grow the engine scratch, launch nothing
     bool use_consts = false;      // take cmcoef and beta from below instead of

@@ -41,8 +41,6 @@ if ROOT not in sys.path:
 # rational's numerator and denominator, the scale and the accumulate, with the
 # per-line terms hoisted (the reciprocal runs on the XU pipe, not counted)
 FLOPS_PER_PAIR = 14
-# XU-pipe reciprocals per region-I pair: two pairs of line-evals share one
-RCP_PER_PAIR = 0.5
 
 
 def hbm_view(traffic_bytes, ms):
@@ -548,20 +546,21 @@ def run_ours(args, rank, world, dist):
                               "condition in the same call, worst over conditions")
 
     step2_ms = float(np.mean(step2))
-    achieved = pairs_step * FLOPS_PER_PAIR / (step2_ms * 1e-3) / 1e12
-    traffic = xu_pct = None
+    equivalent = pairs_step * FLOPS_PER_PAIR / (step2_ms * 1e-3) / 1e12
+    traffic = xu_pct = fma_pct = None
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
     if os.path.exists(tpath):
         try:
             tj = json.load(open(tpath))
             traffic = tj.get("steptwo_mixed_sweep_bytes_per_launch")
             xu_pct = tj.get("steptwo_mixed_sweep_xu_pipe_pct")
+            fma_pct = tj.get("steptwo_mixed_sweep_fma_pipe_pct")
         except (OSError, ValueError):
             traffic = None
     if args.workload != "sweep" or grid.npoints != 75_000:
-        traffic = xu_pct = None  # measured on the sweep's grid and conditions only
-    elif traffic:
-        traffic = traffic * lines.nu.size / 1e7  # step two's reads grow with the line count
+        traffic = xu_pct = fma_pct = None  # measured on the sweep's grid and conditions only
+    elif traffic and lines.nu.size != tj.get("steptwo_mixed_sweep_lines"):
+        traffic = None  # the reads do not grow in proportion to the list
     regions = region_histogram(lines, grid, conds, common) if args.workload == "sweep" else None
 
     # the reference's own GPU kernels (cross_kernal.cu built for sm_100a) on a
@@ -640,20 +639,20 @@ def run_ours(args, rank, world, dist):
         "speedup_mixed_vs_fp64": value / f64_value if f64_value else None,
         "kernel_ms": {"steptwo_mean": step2_ms, "prep_mean": float(np.mean(prep))},
         "roofline": {
-            "bound": "fp32", "achieved": achieved, "peak": peaks["fp32_tflops"],
-            "unit": "TFLOP/s", "frac": achieved / peaks["fp32_tflops"], "traffic": traffic,
+            "bound": "fp32", "peak": peaks["fp32_tflops"], "unit": "TFLOP/s",
+            "frac": fma_pct / 100.0 if fma_pct else None,
+            "frac_how": "FMA pipe cycles active of the sweep's step two in the committed capture "
+                        "(1e6 lines); null for other workloads",
+            "traffic": traffic,
             "peak_source": "measured (in-repo FP32 FMA probe, xs_measure_peaks, burst)",
+            "equivalent_tflops": equivalent,
+            "equivalent_over_peak": equivalent / peaks["fp32_tflops"],
+            "equivalent_how": "every pair of the windows counted at flops_per_pair; step two sums the far wings "
+                              "of many lines as one series, so this is not what the pipe does and can exceed 1",
             "flops_per_pair": FLOPS_PER_PAIR,
-            "note": "an equivalent rate, every pair of the windows counted: step two sums the far wings of "
-                    "many lines as one series, so frac is not the pipe's use and can exceed 1",
             "other_peaks": peaks,
             "region_share": regions,
-            "xu_pipe_pct_ncu": xu_pct if args.workload == "sweep" else None,
-            "mufu_view": {
-                "achieved_rcp_per_s": pairs_step * RCP_PER_PAIR / (step2_ms * 1e-3),
-                "peak_rcp_per_s": peaks.get("rcp32_tops", 0.0) * 1e12,
-                "rcp_per_pair": RCP_PER_PAIR,
-                "note": "one reciprocal per two region-I line-evals (shared), far wings counted line by line"},
+            "xu_pipe_pct_ncu": xu_pct,
             "hbm_view": hbm_view(traffic, step2_ms),
         },
         "cpu_baseline": cpu,
@@ -1017,7 +1016,7 @@ def run_extra_configs(args, rank, world, dist) -> dict:
                 "accuracy_vs_fp64", "error_statement", "kernel_ms", "e2e", "gpu_launches")}
             out["single"]["config"] = r["config"]["workload"]
             out["single"]["launch_shape"] = r["config"]["launch_shape"]
-            out["single"]["roofline_frac"] = r["roofline"]["frac"]
+            out["single"]["equivalent_over_fp32_peak"] = r["roofline"]["equivalent_over_peak"]
     except Exception as exc:
         out["single"] = {"error": f"{type(exc).__name__}: {exc}"}
     try:

@@ -26,8 +26,8 @@ __device__ __forceinline__ void transpose_sum(double (&v)[32], int lane) {
 
 // FP64: one warp per (cell, group of conditions), lanes over the cell's lines;
 // y and pref of each (line, condition) from step one's RecV64 or, GROUPED,
-// CondRec64.  Bound by the FP64 pipe: 30 terms x 6 operations per (line,
-// condition); 1e7 lines 0.23 ms.
+// CondRec64.  30 terms x 6 FP64 operations per (line, condition), the pipe busy 41 %
+// of the time at 14 warps per SM (116 registers; 1e6 lines); 1e7 lines 0.22 ms.
 template <bool GROUPED, int C>
 __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
     constexpr int PM = kCellTerms64;
@@ -136,8 +136,9 @@ __global__ void __launch_bounds__(kCellWarps * 32) k_cells(CellArgs a) {
 // weak the lines are (S below 1e-38 leaves c pref w, and its reciprocal, outside
 // the FP32 range); a moment is off by about 1e-7 of itself, as one FP32 evaluation
 // of the line is.
-// Bound by the FP32 pipe: 16 terms x 3 packed operations per (line, condition);
-// 40 conditions x 1e7 lines 4.77 ms in FP64, 2.1 in FP32.
+// 16 terms x 3 packed operations per (line, condition).  Issue slots 66 %, XU (the
+// conversions from FP64) 47 %, FMA pipe 36 % at 1e6 lines; 40 conditions x 1e7 lines
+// 4.77 ms in FP64, 2.45 in FP32.
 template <int C>
 __global__ void __launch_bounds__(kCellWarps * 32) k_cells_f32(CellArgs a) {
     constexpr int PM = kCellTermsMixed;

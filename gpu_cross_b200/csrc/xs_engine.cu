@@ -49,13 +49,16 @@ int cuda_fail(cudaError_t e, const char* what) {
 // Most slices of a host line list (xs_engine_execute_host).
 constexpr int kMaxPieces = 16;
 
-// Least lines in a window (half of it for batches: 70000 lines, 684 per window, 24
-// conditions 443 us with cells and 460 before; a single condition with 741 per
-// window 158 with and 152 without), width of the window in tiles, and pairs of the
-// call from which the far wings are taken by cells.  (Below 1.2e7 pairs, some 10 us
-// of step two, the GPU is not full either way and the series' launch and the
-// search for far cells cost what they save: 2000 lines on 4001 points, 7e6
-// pairs, 26 us without and 69 us with cells.)
+// Least lines in a window (half of it for batches), width of the window in tiles, and
+// pairs of the call from which the far wings are taken by cells.  Below them the
+// series' launch and the search for far cells cost what they save.  B200, graph
+// replays, FP64 / mixed, us without and with cells:
+//   2000 lines on 4001 points, 1111 per window, 4.5e6 pairs   37 -> 40 / 35 -> 38
+//   4000 on 8000, 1538 per window, 1.23e7 pairs               52 -> 43 / 47 -> 41
+//   10000 on 60000, 769 per window, 4.6e7 pairs               86 -> 92 / 74 -> 76
+//   5000 on 20000, 1000 per window, 2.0e7 pairs               56 -> 56 / 50 -> 47
+//   20000 on 20000, 4000 per window, 8.0e7 pairs              135 -> 84 / 109 -> 70
+//   24 conditions, 70000 lines, 684 per window                460 -> 443
 constexpr double kCellMinLines = 1024.0, kCellMinTiles = 4.0, kCellMinPairs = 1.2e7;
 
 // Restores the caller's current device on scope exit.

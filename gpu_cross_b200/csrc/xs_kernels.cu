@@ -1832,7 +1832,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_steptwo_voigt_mc(StepArgs a) {
 // points per lane halve it, and 2 y^2 comes from Cy = y^2 - 1/2 instead of a
 // third array.  After each group of 32 lines the FP32 sums (32 / LS lines deep)
 // are added up over the lane subsets by halving exchanges, each lane keeping
-// 2 C / LS of them in FP64.  (Every LS groups only, 0.5 of 24.1 ms less for the
+// 2 C / LS of them in FP64.  (Every LS groups only, 0.6 of 24.8 ms less for the
 // 40-condition sweep, the error at 10 atm is 0.23e-7 instead of 0.18e-7, and
 // 0.57e-7 instead of 0.43e-7 for a tenth of the lines.)
 // ---------------------------------------------------------------------------
@@ -2415,7 +2415,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // bodies: with every region unrolled a third of the time went to instruction
 // fetches.)
 //
-// B200, 1e7 lines, 7.5e5 points: 2.5 ms against 3.5 + 1.2 ms for the
+// B200, 1e7 lines, 7.5e5 points: 2.6 ms against 3.5 + 1.2 ms for the
 // point-parallel kernel with cells and its core pass.  The same kernel over
 // 32 / C points and C = 8 conditions was slower than k_steptwo_voigt_mcx on the
 // coarse sweep (20.7 against 12.6 ms).
@@ -2709,8 +2709,8 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArg
 // sums are added up by halving exchanges.  PT = 8: coarse
 // grids over dense lists, where a 32-point tile is wider than the near zone.
 //
-// Bound by the FP64 pipe and the instructions around it: 8 FP64 operations and
-// about 4 others per region-I pair.  B200, 1e7 lines, 7.5e5 points with cells: 4.0
+// Bound by issue slots and the FP64 pipe (50 and 34 % at 1e6 lines): 8 FP64
+// operations and about 4 others per region-I pair.  B200, 1e7 lines, 7.5e5 points with cells: 4.0
 // ms, with 32-point tiles 5.1 (64 more registers); the point-parallel kernel needed
 // 7.0, 26 % of the FP64 pipe and three other instructions for each FP64 one.  16
 // warps per SM (128 registers): 20 spill and take 4.15 ms.
@@ -2904,7 +2904,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS) k_steptwo_near64(StepA
 // tile) and taken 32 at a time, a pair per lane, each lane finding its line by a
 // search over the prefix sums.  Lanes l and l + 16 add to column l of a per-warp
 // table, one after the other; at the end each lane adds up its points' rows: a
-// fixed order.  Bound by erf (two per pair, about 40 FP64 operations each).
+// fixed order.  Bound by erf (two per pair, about 40 FP64 operations each; issue
+// slots 69 %, FP64 pipe 43 %).
 // B200, 1e6 lines on 1e6 points (12 pairs per line): 200 us, 421 with a lane per
 // point.
 // ---------------------------------------------------------------------------

@@ -229,11 +229,17 @@ int xs_engine_execute_host(xs_engine* e, const xs_options* opt, const xs_conditi
  *     positive for non-negative intensities).  Mixed Voigt: 1024 * 2^-24 =
  *     6.1e-5, above the rounding-error analysis of the FP32 steps (region I:
  *     offset, u, u^2 + 2y^2, the shared reciprocal, FP32 partial sums at most 32
- *     deep, 76 * 2^-24; far wings summed by cells: less; regions II-IV: the FP32 x and y
- *     through the profile's sensitivity, at most 2 x^2 = 60.5, the FP32 W4
- *     forms and, for several conditions at once, the region-I value that
- *     step two adds there and the core pass takes back, at most 1.21 W4 --
- *     about 690 * 2^-24).
+ *     deep, 76 * 2^-24; far wings by cells of N lines: moments summed N / 32
+ *     deep in FP32, a line's terms adding up in magnitude to at most
+ *     ((1 + r) / (1 - r))^2 = 3.24 of its value at r = 1 / 3.5, the recurrence,
+ *     its inputs and the series' rest within 60, (0.11 N + 60) * 2^-24 = 286 *
+ *     2^-24 at N = 2048 -- 8192 only beyond 4e8 lines in a call, 961 * 2^-24;
+ *     regions II-IV: the FP32 x and y through the profile's sensitivity, at most
+ *     2 x^2 = 60.5, the FP32 W4 forms and, for several conditions at once, the
+ *     region-I value that step two adds there and the core pass takes back, at
+ *     most 1.21 W4 -- about 690 * 2^-24).  Relative as long as a line's intensity
+ *     over its Doppler width is a normal FP32 number (above 1e-38); each weaker
+ *     line adds up to 2^-148 to the error instead.
  *     FP64 (every FP64 result, Doppler and Gaussian included): 1e-12
  *     (summation order, reciprocals, and the far wings' series, which leaves off
  *     at most 3e-15 of a line's value).

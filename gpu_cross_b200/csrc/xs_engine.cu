@@ -617,11 +617,13 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
             // mixed with cells: on 8-point rows (a coarse grid over a dense
             // list) as many conditions per warp as the batch allows (24.2 ms at
             // 8, 26.4 at 4 for the sweep of 40), else one (8 conditions on a
-            // 0.01 cm-1 grid, 1e6 lines: 2.55 ms at 1, 2.65 at 2 and 4)
+            // 0.01 cm-1 grid, 1e6 lines: 2.55 ms at 1, 2.65 at 2 and 4) -- not
+            // where the caller asks for wide tiles, which one condition at a
+            // time takes line by line
             if (mixed && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid)) {
                 for (int cg : {4, 8})
                     if (groups_ok(cg)) C = cg;
-            } else if (mixed && cells) {
+            } else if (mixed && cells && narrow_tiles) {
                 C = 1;
             }
         } else if (C > 1 && !groups_ok(C)) {

@@ -1354,6 +1354,11 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                 }
             }
         };
+        // Whole lines: Pc / u to FP32 rounding from u = 1e12 on; u^2 overflows from
+        // 1.8e19 and Pc u may, and infinity times 0 is NaN.
+        auto whole_far = [](bool whole, float u, float Pc, float& num, float& den) {
+            if (whole && u > 1.0e12f) num = Pc, den = u;
+        };
         // `full`: the line's window covers the whole tile.
         auto slow_line = [&](const unsigned char* r, bool full) {
             if (MIXED) {
@@ -1374,8 +1379,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     const float xs = whole ? float((reinterpret_cast<const RecV32*>(r)->nu - F[jj[p] < t1 ? jj[p] : tl]) / reinterpret_cast<const RecV32*>(r)->nu) * a.kx[w.c]
                                            : fmaf(m - jf[p], dfa, ra);
                     const float u = fmaf(xs, xs, Cy);
-                    const float num = fmaf(u, Pc, Pc);
-                    const float rr = rcp_approx_f32(fmaf(u, u, D2));
+                    float num = fmaf(u, Pc, Pc), den = fmaf(u, u, D2);
+                    whole_far(whole, u, Pc, num, den);
+                    const float rr = rcp_approx_f32(den);
                     if (row_in && !row_core) {
                         accf[p] = fmaf(num, rr, accf[p]);
                         continue;
@@ -1475,8 +1481,9 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
                     const float xs = whole ? float((reinterpret_cast<const RecV32*>(r)->nu - F[jj[p] < t1 ? jj[p] : tl]) / reinterpret_cast<const RecV32*>(r)->nu) * a.kx[w.c]
                                            : fmaf(v0.x - jf[p], v0.z, v0.y);
                     const float u = fmaf(xs, xs, v0.w);
-                    const float num = fmaf(u, v1.y, v1.y);
-                    const float rr = rcp_approx_f32(fmaf(u, u, v1.x));
+                    float num = fmaf(u, v1.y, v1.y), den = fmaf(u, u, v1.x);
+                    whole_far(whole, u, v1.y, num, den);
+                    const float rr = rcp_approx_f32(den);
                     if (!whole && (r1 < clo || r0 > chi)) {
                         accf[p] = fmaf(num, rr, accf[p]);
                         continue;

@@ -75,3 +75,24 @@ def test_batches_of_distinct_temperatures(engine, cuda, temperatures):
     got = run_engine(engine, capi.VOIGT, lines, *args, conds=conds, C=2, precision=capi.MIXED)
     for k in range(len(conds)):
         assert_mixed_parity(got[k], ref[k])
+
+
+@pytest.mark.parametrize("convention", [capi.CONV_GPU, capi.CONV_CPU])
+@pytest.mark.parametrize("C, P", [(1, 0), (1, 1), (1, 2), (1, 4), (1, 8), (2, 0)])
+def test_strong_lines_far_beyond_their_doppler_width(engine, cuda, convention, C, P):
+    """Strong lines at 1e-6 cm-1, where the Doppler width is some 1e-12: x reaches 1e13
+    inside the window, u = x^2 + y^2 - 1/2 is 1e26 and u times the amplitude beyond the
+    FP32 range."""
+    lines = synth.random_lines(500, 1.0, 60.0, 2500.0, 1e-6, 1e2, seed=77)
+    lines.nu[:9] = np.linspace(1e-6, 2e-6, 9)
+    lines.aif[:9] = 1e8
+    lines.gns[:9] = 100
+    grid = synth.Grid(18.0, 58.0, 4000)
+    conds = [dict(c, cut=100.0) for c in conditions(2)]
+    args = (grid.freq(), conds[0], grid.dfreq, cuda)
+    run = dict(conds=conds, convention=convention)
+    ref = run_engine(engine, capi.VOIGT, lines, *args, **run)
+    got = run_engine(engine, capi.VOIGT, lines, *args, C=C, P=P, precision=capi.MIXED, **run)
+    assert np.isfinite(got).all()
+    for k in range(2):
+        assert_mixed_parity(got[k], ref[k])

@@ -106,27 +106,23 @@ namespace xs {
 int set_error(int code, const char* msg) { return fail(code, msg); }
 
 // Default launch shapes, from measurements on a B200 (the autotuner's table
-// takes precedence).  Voigt tiles of 32 P points: two per lane where a line's
-// window spans many tiles (fewer partial lines per tile, record loads shared by
-// more points; 12000 lines on 700000 points: 109 us per call at P = 2 and 4, 131
-// at 1; 30000 on 200000: 103 at 2, 110 at 4), one on coarse grids, where a wider
-// tile would hold mostly partial and core lines.  4 warps per block.
+// takes precedence).  Voigt tiles of 32 P points, P = 1 meaning a lane per line on
+// 16- or 8-point tiles for single conditions (k_steptwo_near, k_steptwo_near64).
 // With the far wings taken by cells, what is left line by line is the lines
 // near the tile and those whose windows end in it, so narrow tiles win (FP64
 // single point, 1e7 lines, 7.5e5 points, one kernel at three shapes: 10.3 ms of
-// step two at P = 4, 7.6 at 2, 7.1 at 1): P = 1, which single conditions take with
-// a lane per line (k_steptwo_near, k_steptwo_near64).
-void default_shape(int kind, bool cells, double window_points, int* P, int* warps) {
-    if (kind == kVoigt && cells) {
-        *P = 1;
-        *warps = 4;
-    } else if (kind == kVoigt) {
-        *P = window_points >= 512.0 ? 2 : 1;
-        *warps = 4;
-    } else {
-        *P = 1;
-        *warps = 4;
-    }
+// step two at P = 4, 7.6 at 2, 7.1 at 1).
+// Without cells a tile has few lines, and what counts is the search for them:
+// FP64 two points per lane (24 conditions, 300 lines, 1e5 points, windows of 500
+// points: 100 us, 267 with a lane per line; 1 condition, 3000 lines: 35 and 44), as
+// mixed from windows of 512 points on (on coarser grids a lane per line, which has
+// W4 regions II-IV in the same launch: 30000 lines, windows of 500 points, 55 us and
+// 62); four where windows span 2048 points and there are tiles enough (24
+// conditions, 300 lines, windows of 5000 points, FP64: 103 us, 118 at 2; 30000
+// lines on 300000 points, mixed: 177 us, 195 at 2).  4 warps per block.
+void default_shape(int kind, bool mixed, bool cells, double window_points, int* P, int* warps) {
+    *P = kind != kVoigt || cells ? 1 : window_points >= 2048.0 ? 4 : !mixed || window_points >= 512.0 ? 2 : 1;
+    *warps = 4;
 }
 
 // Launch shapes chosen by xs_engine_autotune, per call signature: profile,
@@ -557,13 +553,15 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         int dP, dW;
         double cutmax = 0.0;
         for (int c = 0; c < ncond; ++c) cutmax = std::fmax(cutmax, make_cond(*opt, conds[c]).cut);
-        default_shape(kind, cells, 2.0 * cutmax / opt->dfreq, &dP, &dW);
+        default_shape(kind, mixed, cells, 2.0 * cutmax / opt->dfreq, &dP, &dW);
         // Calls with fewer tiles than the GPU holds warps take narrower tiles:
         // a line split needs a buffer and a reduction, a narrow tile neither.
         // (3000 lines, 12000 points, 5000-point windows: step two 71 us with
-        // 94 tiles of 128 points in 3 parts, 39 us with 375 of 32 in 7.)
+        // 94 tiles of 128 points in 3 parts, 39 us with 375 of 32 in 7.  128-point
+        // tiles from 12 per SM on: 30000 lines on 200000 points, 1562 tiles, 110 us
+        // and 103 at half the width; on 300000, 2344 tiles, 177 and 195.)
         while (P == 0 && dP > 1 && kind == XS_VOIGT &&
-               double(grid->points) / (32.0 * dP) * ncond < 8.0 * e->num_sms)
+               double(grid->points) / (32.0 * dP) * ncond < (dP == 4 ? 12.0 : 8.0) * e->num_sms)
             dP /= 2;
         if (P == 0) P = dP;
         if (W == 0) W = dW;

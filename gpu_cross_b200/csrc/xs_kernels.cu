@@ -1208,13 +1208,32 @@ constexpr size_t kCoreTable64 = sizeof(double) * 32 * kCoreRow64;
 // x, y and the region choice are the reference's.  Returns this lane's point's
 // sum.
 //
+// Rows with at most kFewCore candidates (sparse lists) go lane = point.
 // Before, the pairs went through a shared-memory queue, 32 at a time over all
 // regions, between step two's lines.
+constexpr long kFewCore = 3;
 template <class Get>
 __device__ __forceinline__ double core_row_f64(double (*T)[kCoreRow64], const double* F, long E, long Fc, int r0,
                                                int S, int s, int lane, Get get) {
     // Few candidate lines (sparse lists, small calls): 2 or 4 lanes to a line,
     // on every second or fourth point, so that one batch's chain is shorter.
+    if (Fc - E <= kFewCore) {
+        // one to a few lines: lane = point, without the table
+        double v = 0.0;
+        for (long i = E; i < Fc && s == 0; ++i) {
+            double nu = 0.0, g = 0.0, y = 0.0, pref = 0.0;
+            int jlo = 1, jhi = 0;
+            get(i, nu, g, y, pref, jlo, jhi);
+            const int j = r0 + lane;
+            if (jlo > jhi || j < jlo || j > jhi) continue;
+            const double ax = fabs((nu - F[j]) * g), sx = ax + y;
+            if (sx >= 15.0) continue;
+            v += pref * (sx >= 5.5 ? w4_region2_re<double>(ax, y)
+                         : y >= 0.195 * ax - 0.176 ? w4_region3_re_f64(ax, y) : w4_region4_re_f64(ax, y));
+        }
+        __syncwarp();
+        return v;
+    }
     const int sh = Fc - E <= 8L * S ? 2 : (Fc - E <= 16L * S ? 1 : 0);
     const int nb = 32 >> sh, sub = lane & ((1 << sh) - 1), step = 1 << sh;
     if (E + long(nb) * s >= Fc) return 0.0;
@@ -1589,14 +1608,24 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_min_blocks<P, WARPS, MIXED>
 #pragma unroll
         for (int p = 0; p < P; ++p) v[p] = MIXED ? double(sumf[p]) - double(cmpf[p]) : accd[p];
         if constexpr (!MIXED) {
-            // W4 regions II-IV
+            // W4 regions II-IV (one search for the tile, so that a tile without
+            // candidates, the usual one of a sparse list, makes none per row)
             double (*T)[kCoreRow64] = reinterpret_cast<double (*)[kCoreRow64]>(mine);
+            const long Ta = warp_lower_bound(La, Lb, lane, [&](long i) { return mi[i] >= t0 - kc; });
+            const long Tb = warp_lower_bound(Ta, Lb, lane, [&](long i) { return mi[i] > tl + kc; });
+            const int mt = Ta + lane < Tb ? mi[Ta + lane] : INT_MAX;
 #pragma unroll 1
-            for (int p = 0; p < P; ++p) {
+            for (int p = 0; p < P && Ta < Tb; ++p) {
                 const int r0 = t0 + 32 * p, r1 = min(r0 + 32, t1) - 1;
                 if (r0 > r1) break;
-                const long E0 = warp_lower_bound(La, Lb, lane, [&](long i) { return mi[i] >= r0 - kc; });
-                const long E1 = warp_lower_bound(E0, Lb, lane, [&](long i) { return mi[i] > r1 + kc; });
+                long E0 = Ta, E1 = Tb;
+                if (P > 1 && Tb - Ta <= 32) {
+                    E0 = Ta + __popc(__ballot_sync(0xffffffffu, mt < r0 - kc));
+                    E1 = Ta + __popc(__ballot_sync(0xffffffffu, mt <= r1 + kc));
+                } else if (P > 1) {
+                    E0 = warp_lower_bound(Ta, Tb, lane, [&](long i) { return mi[i] >= r0 - kc; });
+                    E1 = warp_lower_bound(E0, Tb, lane, [&](long i) { return mi[i] > r1 + kc; });
+                }
                 const double add =
                     core_row_f64(T, F, E0, E1, r0, a.splits, w.s, lane,
                                  [&](long i, double& nu, double& g, double& y, double& pref, int& jlo, int& jhi) {

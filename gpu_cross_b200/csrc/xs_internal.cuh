@@ -126,6 +126,8 @@ struct __align__(16) LineShX {
 static_assert(sizeof(LineShX) == 32, "LineShX layout");
 constexpr int kLineWhole = 1;
 constexpr int kLineWide = 2;
+constexpr int kLineFar = 4;  // groups of conditions: wide beyond what a plain
+                             // reciprocal per pair holds (kSoloUMax)
 // Per (line, condition) of the mixed multi-condition layout, for the core
 // pass: the grid indices of W4 regions II-IV [lo15, hi15] and III-IV
 // [lo55, hi55] (empty: lo > hi) inside the line's window.  Step two adds

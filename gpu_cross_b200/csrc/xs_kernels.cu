@@ -47,6 +47,9 @@ constexpr double kWholeXMax = 1.0e8;
 // kLineWide.
 constexpr double kPairUMax = 2.5e9;
 constexpr double kPairPcMax = 1.0e8;
+// Wide lines below these take a reciprocal per pair with no test: u^2 stays below
+// 1e36 and Pc (u + 1) below 1e36.
+constexpr double kSoloUMax = 1.0e18, kSoloPcMax = 1.0e18;
 
 
 // ---------------------------------------------------------------------------
@@ -394,7 +397,7 @@ __device__ __forceinline__ int prep_line(const PrepArgs& a, long i, int c, int* 
             ls.m = float(fabs(m) < 16000000.0 ? m : 0.0);
             ls.dfn = float(df * g);
             ls.rn = float(((nu_p - f0) - m * df) * g);
-            ls.flags = (whole ? kLineWhole : 0) |
+            ls.flags = (whole || !(xw * xw + y2 < kSoloUMax) || !(fabs(Pc) < kSoloPcMax) ? kLineWhole : 0) |
                        (!(xw * xw + y2 < kPairUMax) || !(fabs(Pc) < kPairPcMax) ? kLineWide : 0);
             ls.lo = lo;
             ls.hi = hi;
@@ -596,7 +599,7 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
     double cut_prev = -1.0;
     int lo = s, hi = s;
     int slot = -1;
-    bool wide = false;
+    bool wide = false, far = false;
     auto flush_window = [&]() {
         if (!live || slot < 0) return;
         const size_t wi = size_t(slot) * size_t(a.L.n) + size_t(i);
@@ -604,7 +607,7 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
         ls.m = float(far_m ? 0.0 : m);
         ls.dfn = float(df / nu_p);
         ls.rn = float(((nu_p - f0) - m * df) / nu_p);
-        ls.flags = (far_m ? kLineWhole : 0) | (wide ? kLineWide : 0);
+        ls.flags = (far_m ? kLineWhole : 0) | (wide ? kLineWide : 0) | (far ? kLineFar : 0);
         ls.lo = lo;
         ls.hi = hi;
         ls.nu = nu_p;
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
         if (a.wslot[cg] != slot) {
             flush_window();
             slot = a.wslot[cg];
-            wide = false;
+            wide = far = false;
             const double cut = a.cond[cg * C].cut;  // a run of groups shares its cut
             cut_prev = cut;
             if (live) {
@@ -657,6 +660,7 @@ __global__ void __launch_bounds__(256, 3) k_prep_lines_x(PrepArgs a) {
                 const bool whole = far_m || !(xw < kWholeXMax);
                 // the shared reciprocals need the products in range
                 wide = wide || !(xw * xw + y2 < kPairUMax) || !(fabs(Pc) < kPairPcMax);
+                far = far || whole || !(xw * xw + y2 < kSoloUMax) || !(fabs(Pc) < kSoloPcMax);
                 CoreIv iv;
                 const double q = nu_df * Cd.dpw;
                 region_interval_q(nu_p, g, y, 15.0, lo, hi, f0, df, md, q, tb, iv.lo15, iv.hi15);
@@ -2038,7 +2042,16 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
             const float2 sn = __ffma2_rn(nB, dA, __fmul2_rn(nA, dB));
             to = __ffma2_rn(sn, f2(rcp_approx_f32(q.x), rcp_approx_f32(q.y)), to);
         };
-        // One line (wide, whole or a core candidate, or any in their company)
+        // One line (wide, or in a wide one's company) at one point, not a core
+        // candidate: a reciprocal per pair.
+        auto solo_step = [&](float X2, float2 cy, float2 pc, int p, bool in, float2& to) {
+            const float2 u = __ffma2_rn(f2s(X2), k2[p], cy);
+            const float2 den = __ffma2_rn(u, u, region1_d2(cy));
+            float2 num = __ffma2_rn(u, pc, pc);
+            if (!in) num = f2(0.0f, 0.0f);
+            to = __ffma2_rn(num, f2(rcp_approx_f32(den.x), rcp_approx_f32(den.y)), to);
+        };
+        // One line (far, whole or a core candidate, or any in their company)
         // at one point: a reciprocal per pair.  NEAR: a pair is kept only where
         // u >= 1 (core candidates: the core pass takes u < 1).  Pc / u to FP32
         // rounding from u = 1e12 on (u^2 overflows from 1.8e19); beyond x = 1e18
@@ -2145,7 +2158,8 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                     const int2 wA = SW[tA], wB = SW[tB];
                     const float XA0 = fmaf(sA.x - jf0, sA.y, sA.z), XA1 = fmaf(sA.x - jf1, sA.y, sA.z);
                     const float XB0 = fmaf(sB.x - jf0, sB.y, sB.z), XB1 = fmaf(sB.x - jf1, sB.y, sB.z);
-                    const bool wide = ((__float_as_int(sA.w) | __float_as_int(sB.w)) & kLineWide) != 0;
+                    const int flags = __float_as_int(sA.w) | __float_as_int(sB.w);
+                    const bool wide = (flags & kLineWide) != 0;
                     const bool okA = b + sub < y, okB = b + sub + LS < y;
                     const bool inA0 = okA && j0 >= wA.x && j0 < wA.y, inA1 = okA && j1 >= wA.x && j1 < wA.y;
                     const bool inB0 = okB && j0 >= wB.x && j0 < wB.y, inB1 = okB && j1 >= wB.x && j1 < wB.y;
@@ -2170,6 +2184,18 @@ __global__ void __launch_bounds__(WARPS * 32, (voigt_mcx_min_blocks<C, WARPS>())
                         } else {
                             both(*reinterpret_cast<const float2*>(&rA.Cy[0]), *reinterpret_cast<const float2*>(&rA.Pc[0]),
                                  *reinterpret_cast<const float2*>(&rB.Cy[0]), *reinterpret_cast<const float2*>(&rB.Pc[0]), 0);
+                        }
+                    } else if (!__any_sync(0xffffffffu, (flags & (kLineFar | kLineWhole)) != 0)) {
+#pragma unroll
+                        for (int p = 0; p < NP; ++p) {
+                            const float2 cyA = *reinterpret_cast<const float2*>(&rA.Cy[2 * p]);
+                            const float2 pcA = *reinterpret_cast<const float2*>(&rA.Pc[2 * p]);
+                            const float2 cyB = *reinterpret_cast<const float2*>(&rB.Cy[2 * p]);
+                            const float2 pcB = *reinterpret_cast<const float2*>(&rB.Pc[2 * p]);
+                            solo_step(XA0 * XA0, cyA, pcA, p, inA0, acc[0][p]);
+                            solo_step(XA1 * XA1, cyA, pcA, p, inA1, acc[1][p]);
+                            solo_step(XB0 * XB0, cyB, pcB, p, inB0, acc[0][p]);
+                            solo_step(XB1 * XB1, cyB, pcB, p, inB1, acc[1][p]);
                         }
                     } else {
 #pragma unroll
@@ -2444,10 +2470,12 @@ __global__ void __launch_bounds__(WARPS * 32) k_core_v32(StepArgs a) {
 // points are wider than the near zone.
 //
 // Two evaluations share one reciprocal, 1/dA = dB / (dA dB) (narrow lines,
-// kPairUMax).  Groups with lines of the core reach choose region I or II per
-// pair by the exact region intervals; the pairs of regions III and IV, and all
-// pairs of groups with wide or whole lines, are evaluated in a loop by their
-// own line's lane into a per-warp table with a column per lane.  (Few unrolled
+// kPairUMax); groups with wide lines take one each (3000 lines, 50000 points, cut
+// 100: 189 us with all their pairs in the loop below, 102 so).  Groups with lines
+// of the core reach choose region I or II per pair by the exact region intervals;
+// the pairs of regions III and IV, and all pairs of groups with whole lines, are
+// evaluated in a loop by their own line's lane into a per-warp table with a column
+// per lane.  (Few unrolled
 // bodies: with every region unrolled a third of the time went to instruction
 // fetches.)
 //
@@ -2562,6 +2590,25 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArg
                 add_pair(num, __ffma2_rn(u, u, r.d2), acc[q]);
             }
         };
+        // A group with wide lines: region I with a reciprocal per pair.
+        auto solo_group = [&](float4 s, int2 win, float2 v, const CoreIv& iv) {
+            const float mj = s.x - t0f;
+            const unsigned wlen = unsigned(win.y - win.x);
+            const int w0 = t0 - win.x, d15 = t0 - iv.lo15;
+            const unsigned n15 = iv.lo15 <= iv.hi15 ? unsigned(iv.hi15 - iv.lo15) + 1u : 0u;
+            const R1 r = constants(v);
+#pragma unroll
+            for (int q = 0; q < PT / 2; ++q) {
+                const float2 x = offsets(mj, s, q);
+                const float2 u = __ffma2_rn(x, x, r.cy);
+                const float2 den = __ffma2_rn(u, u, r.d2);
+                float2 num = __ffma2_rn(u, r.pc, r.pc);
+                const int pa = 2 * q, pb = 2 * q + 1;
+                if (!(unsigned(w0 + pa) < wlen) || unsigned(d15 + pa) < n15) num.x = 0.0f;
+                if (!(unsigned(w0 + pb) < wlen) || unsigned(d15 + pb) < n15) num.y = 0.0f;
+                acc[q] = __ffma2_rn(num, f2(rcp_approx_f32(den.x), rcp_approx_f32(den.y)), acc[q]);
+            }
+        };
         // A group of narrow lines with core candidates: region I or II chosen
         // per pair by the region intervals; the pairs of regions III and IV are
         // left to inner_pairs.
@@ -2602,12 +2649,13 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArg
                 add_pair(num, den, acc[q]);
             }
         };
-        // Pairs of regions III and IV of a core group; `all` (wide and whole
-        // lines): every pair of the window (beyond x = 1e18 region I is taken
-        // as 0); whole lines: X from the FP64 centre.
-        auto inner_pairs = [&](float4 s, int2 win, float2 v, const CoreIv& iv, int i, bool all) {
+        // The pairs jlo .. jhi of the line in the tile, a lane going over its own:
+        // regions III and IV, or (`mixed`) regions by the intervals; whole lines: X
+        // from the FP64 centre (beyond x = 1e18 region I is taken as 0).
+        auto inner_pairs = [&](float4 s, float2 v, const CoreIv& iv, int i, int jlo, int jhi, bool mixed) {
             const bool whole = (__float_as_int(s.w) & kLineWhole) != 0;
-            const int jlo = max(all ? win.x : iv.lo55, t0), jhi = min(all ? win.y - 1 : iv.hi55, tl);
+            jlo = max(jlo, t0);
+            jhi = min(jhi, tl);
             if (!__any_sync(0xffffffffu, jlo <= jhi)) return;
             cored = true;
             const double nu = whole ? lsh[i].nu : 0.0;
@@ -2620,7 +2668,7 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArg
                 // and pref: the pair is left out, not multiplied by 0)
                 if (!(ax < 1.0e18f)) continue;
                 float wf;
-                if (!all || (j >= iv.lo55 && j <= iv.hi55)) {
+                if (!mixed || (j >= iv.lo55 && j <= iv.hi55)) {
                     wf = float(1.0 / kW4C) *
                          ((y >= fmaf(0.195f, ax, -0.176f)) ? w4_region3_re_f32(ax, y) : w4_region4_re_f32(ax, y));
                 } else if (j >= iv.lo15 && j <= iv.hi15) {
@@ -2708,8 +2756,15 @@ __global__ void __launch_bounds__(WARPS * 32, 20 / WARPS) k_steptwo_near(StepArg
                 core = __any_sync(0xffffffffu, odd || (iv.lo15 <= tl && iv.hi15 >= t0 && iv.lo15 <= iv.hi15));
             }
             if (core) {
-                if (!odd) core_group(s, win, v, iv);
-                inner_pairs(s, win, v, iv, gb + lane, odd);
+                if (!odd) {
+                    core_group(s, win, v, iv);
+                    inner_pairs(s, v, iv, gb + lane, iv.lo55, iv.hi55, false);
+                } else if (__any_sync(0xffffffffu, (__float_as_int(s.w) & kLineWhole) != 0)) {
+                    inner_pairs(s, v, iv, gb + lane, win.x, win.y - 1, true);
+                } else {
+                    solo_group(s, win, v, iv);
+                    inner_pairs(s, v, iv, gb + lane, iv.lo15, iv.hi15, true);
+                }
             } else if (gb >= fs && ge <= fe && ge - gb == 32) {
                 plain_group(std::false_type(), s, win, v);
             } else {

@@ -607,23 +607,18 @@ int engine_execute(xs_engine* e, const xs_options* opt, const xs_condition* cond
         if (kind != XS_VOIGT) {
             C = 1;
         } else if (C == 0) {
-            // Measured on B200 (40-condition sweep, 0.1 cm-1 grid): two
-            // conditions per warp or more is fastest for the mixed path; the
-            // FP64 path takes one (8 conditions, 1e6 lines, cells: 1.37 ms of
-            // step two against 1.63 with two).
-            C = mixed && groups_ok(2) ? 2 : 1;
-            // mixed with cells: on 8-point rows (a coarse grid over a dense
-            // list) as many conditions per warp as the batch allows (24.2 ms at
-            // 8, 26.4 at 4 for the sweep of 40), else one (8 conditions on a
-            // 0.01 cm-1 grid, 1e6 lines: 2.55 ms at 1, 2.65 at 2 and 4) -- not
-            // where the caller asks for wide tiles, which one condition at a
-            // time takes line by line
-            if (mixed && cells_at(8) && row_is_wide(*opt, conds, ncond, n, *grid)) {
-                for (int cg : {4, 8})
+            // Mixed: as many conditions per warp as the batch allows, with cells and
+            // without (B200, us at 1, 2, 4 and 8 per warp; 24 conditions unless said:
+            // 1.3e4 lines on 1e5 points at 0.01 cm-1 834, 493, 480, 426; 2.8e5 on
+            // 112426 at 0.21 1934, 1260, 1173, 1055; 8 conditions, 1.3e6 on 1e5 at
+            // 0.01 2517, 2097, 1788, 1737; without cells, 6300 on 1e5 709, 538, 447,
+            // 391; the sweep of 40 26.4 ms at 4, 24.2 at 8).  FP64: one (8
+            // conditions, 1e6 lines, cells: 1.37 ms of step two against 1.63 with
+            // two).
+            C = 1;
+            if (mixed)
+                for (int cg : {2, 4, 8})
                     if (groups_ok(cg)) C = cg;
-            } else if (mixed && cells && narrow_tiles) {
-                C = 1;
-            }
         } else if (C > 1 && !groups_ok(C)) {
             return fail(XS_ERR_INVALID, "conditions_per_warp needs ncond <= 64 and, for every cut, a "
                                         "number of conditions that is a multiple of it");
